@@ -88,7 +88,6 @@ struct Rep {
   Grid ag, eg;
   int abase, ebase;
   double reach_budget;
-  float fmargin;      // bound on the error of FP32 separations in this box (A)
   double qscale[3];   // mixed form: fixed-point scale 2^k per dimension ...
   float qinv[3];      // ... and 2^-k
   int Lq[3];          // rint(L 2^k)
@@ -233,7 +232,7 @@ struct Ctx {
   DBuf<int> acell_start;         // [ncell+1]
   DBuf<int> acell_atoms;         // [na] atom ids sorted by cell
   DBuf<double4> acell_pos;       // [na] wrapped positions sorted by cell, w = bitcast(id)
-  DBuf<float4> acell_pos32;      // [na] the same as floats, w = bitcast(int id)
+  DBuf<int> acell_fix;           // [3][na] the same in fixed point (the atom build's screen, neigh.cu)
   DBuf<int> acell_of;            // [na] cell of each sorted atom
   DBuf<int> ecell_start, ecell_elems;
   DBuf<int> cell_key, cell_key2, idx_tmp;

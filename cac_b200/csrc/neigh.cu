@@ -284,15 +284,39 @@ __global__ void k_cell_start(const int *skey, int n, int ncell, int *start) {
   start[c] = lo;
 }
 
-__global__ void k_gather_pos(const double4 *xs, const int *sidx, const int *skey, int n, double4 *out,
-                             float4 *out32, int *atom_slot, int *slot_cell) {
+// Fixed-point copy of a wrapped atom position for the screen of the atom build: quanta of
+// 2^-20 A from the box corner, modulo 2^32 (4096 A), so that the differences
+// of near positions are exact integers whatever the size of the box.  An atom
+// that is not in or near the box (a run that has blown up) gets FAR_ATOM and
+// is nobody's neighbour.
+constexpr int FAR_ATOM = 0x80000000;
+constexpr float QUANTUM = 1.0f / 1048576.0f;
+__device__ __forceinline__ int fix20(double x) { return (int)(unsigned)(unsigned long long)__double2ll_rn(x * 1048576.0); }
+
+// The sorted atoms: positions (w = atom index), the fixed-point copies of the
+// screen (x, y, z parts n apart), slots and cells.
+template <class RP>
+__global__ void k_gather_pos(const double4 *xs, const int *sidx, const int *skey, int n, RP P, double4 *out,
+                             int *fixed, int *atom_slot, int *slot_cell) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   int i = sidx[k];
   atom_slot[i] = k;
   slot_cell[k] = skey[k];
   double4 p = xs[i];
-  out32[k] = make_float4((float)p.x, (float)p.y, (float)p.z, __int_as_float(i));
+  const BoxD b = P.site(i).b;
+  const double q[3] = {p.x, p.y, p.z};
+  int f[3];
+  bool near = true;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    near = near && q[d] >= b.lo[d] - b.L[d] && q[d] <= b.hi[d] + b.L[d];
+    f[d] = fix20(q[d] - b.lo[d]);
+  }
+  if (f[0] == FAR_ATOM) f[0]++;
+  fixed[k] = near ? f[0] : FAR_ATOM;
+  fixed[k + (size_t)n] = f[1];
+  fixed[k + 2 * (size_t)n] = f[2];
   p.w = __longlong_as_double((long long)i);
   out[k] = p;
 }
@@ -306,7 +330,7 @@ struct BuildArgs {
   const double *eframe;
   const int *acell_start;
   const double4 *acell_pos;
-  const float4 *acell_pos32;  // wrapped positions as floats, w = atom index bits
+  const int *acell_x, *acell_y, *acell_z;   // wrapped positions in fixed point (fix20)
   const int *acell_of;        // [na] cell of each sorted atom (list slot)
   const int *ecell_start;
   const unsigned char *ecell_near;   // single systems: element cell has an element in its 27-cell block (else null)
@@ -800,49 +824,93 @@ __device__ __forceinline__ void finish_counts(const BuildArgs &A, int i, int nin
   }
 }
 
-// Atoms, atom neighbours: one block (one warp) per chunk of 32 consecutive
-// sorted atoms (list slots).  Cells (>= cutneigh) are sorted x fastest, so a
-// chunk lies in one row of cells, or in two at a row's end (then the warp
-// takes the two parts in turn).  For each of the 9 rows around the part's
-// row the lanes walk together the cells from one left of the part's first
-// cell to one right of its last, as at most three runs of consecutive cells
-// under one image (the left and right wraps and the middle), so every
-// candidate is one broadcast load shared by the warp and all 32 lanes hold
-// an atom.  A lane meets the cells of its own 27-cell block in the order a
-// walk of that block alone would take (ascending x in each row) and the
-// others only beyond its reach, so its list is the same entry for entry.
-// A conservative FP32 distance test (from a float copy of the wrapped
-// positions) decides all but the candidates near the cutoff, which take the
-// exact FP64 test.  The image of a run relative to each lane's atom is fixed
-// per run.
+// Two FP32 values in one 64-bit register and the packed operations on them
+// (sm_100: one instruction for two lanes' worth of arithmetic, each half
+// rounded as the scalar operation rounds it).
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 f2_pack(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// mask << 2 with the sign bits of the halves of v below, the first half first
+__device__ __forceinline__ unsigned f2_signs(unsigned mask, F2 v) {
+  unsigned lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+  return __funnelshift_l(hi, __funnelshift_l(lo, mask, 1), 1);
+}
+
+// Atoms, atom neighbours: one block per chunk of 32 consecutive sorted atoms
+// (list slots), the atoms as lanes.  Cells (>= cutneigh) are sorted x
+// fastest, so a chunk lies in one row of cells, or in two at a row's end
+// (then the warps take the two parts in turn).  For each of the 9 rows around
+// the part's row the candidates are the cells from one left of the part's
+// first cell to one right of its last, as at most three runs of consecutive
+// cells under one image (the left and right wraps and the middle).  A lane
+// meets the cells of its own 27-cell block in the order a walk of that block
+// alone would take (ascending x in each row) and the others only beyond its
+// reach, so its list is the same entry for entry.
 //
-// Full-list entries are written in their final form (the candidate's sorted
-// position is its list slot) and staged per lane in two 32-row rings in
-// shared memory, one per segment (lane = column, so a lane only ever touches
-// its own bank); the warp writes them out row by row: the lanes' list slots
-// are consecutive, so each row is one coalesced store across the warp
-// instead of one scattered store per entry (the lists are transposed,
-// [entry][slot]).  The warp flushes whenever a lane's ring is full and once
-// at the end.
-constexpr int STAGE_ROWS = 32;
-template <class RP>
-__device__ __forceinline__ void build_atoms_chunk(BuildArgs A, RP P, const int chunk) {
-  const int lane = threadIdx.x & 31;
-  const float fcut2 = (float)A.cutforcesq;
-  __shared__ int st_in[STAGE_ROWS][32], st_out[STAGE_ROWS][32];   // front / back segment rings
+// The kernel is bound by instruction issue, so the work is cut in three.
+// Gather: the lanes take one candidate each, 32 consecutive ones of a run at a
+// time, and keep those within reach of the box around the part's atoms (about
+// 490 of 850): position relative to the part's first cell under the run's
+// image, as floats, and list entry, in shared memory.  These coordinates are
+// a few cells long, so FP32 decides all but the few candidates within 1e-4 A
+// or so of the cutoff.
+// Screen: over each word of 32 kept candidates every lane forms, without a
+// branch, three bit masks (first candidate in the top bit): within cutneigh +
+// margin, within cutneigh - margin, within the inner radius, from broadcast
+// 128-bit loads and packed FP32 arithmetic, about 8 instructions a candidate.
+// Bits between the first two masks take the exact FP64 test at once.  The
+// masks replace the word's coordinates.
+// Write-out: each lane pops its masks' bits in order, all lanes their n-th
+// entry together: the lanes' list slots are consecutive, so each row of the
+// (transposed) list is one coalesced store.
+constexpr int SMALL_CHUNKS = 8;   // chunks per SM below which a chunk takes four warps
+template <int NW, class RP>
+__device__ __forceinline__ void build_atoms_chunk(const BuildArgs &A, const RP &P, const int chunk) {
+  // words of kept candidates between two write-outs: 16 are usual; with four
+  // warps, as many as the words of candidates taken at a time
+  constexpr int MAXW = NW == 1 ? 20 : 32;
+  __shared__ float4 kx4[MAXW][8], ky4[MAXW][8], kz4[MAXW][8];   // kept candidates' coordinates, then the masks
+  __shared__ int entry[MAXW * 32];                              // (list slot << IMG_BITS) | image code
+  __shared__ unsigned kept[NW > 1 ? MAXW : 1];
+  __shared__ int self_at[32], back[32];
+  unsigned *const m_acc = reinterpret_cast<unsigned *>(kx4), *const m_in = reinterpret_cast<unsigned *>(ky4);
+  const int lane = threadIdx.x & 31, warp = NW > 1 ? (int)threadIdx.x >> 5 : 0;
+  auto sync = [] {
+    if (NW > 1) __syncthreads();
+    else __syncwarp();
+  };
   const int h = chunk * 32 + lane;
   const bool mine = h < A.na;
   const int key = mine ? A.acell_of[h] : -1;
   Query q;
-  float wx = 0.f, wy = 0.f, wz = 0.f;
+  int3 qh = make_int3(FAR_ATOM, 0, 0);
   if (mine) {
     make_query(A, P, (int)__double_as_longlong(A.acell_pos[h].w), q);
     q.slot = h;
-    float4 w = A.acell_pos32[h];
-    wx = w.x;
-    wy = w.y;
-    wz = w.z;
+    qh = make_int3(A.acell_x[h], A.acell_y[h], A.acell_z[h]);
+  } else {
+    q.ti[0] = q.ti[1] = q.ti[2] = 0;
   }
+  const bool unwrapped = (q.ti[0] | q.ti[1] | q.ti[2]) == 0;
   // the chunk's parts, one row of cells each, lowest lanes first
   unsigned todo = __ballot_sync(0xffffffffu, mine);
   while (todo) {
@@ -857,126 +925,256 @@ __device__ __forceinline__ void build_atoms_chunk(BuildArgs A, RP P, const int c
     // unwrapped x range of the candidate cells
     const int xlo = __reduce_min_sync(0xffffffffu, active ? hx : 0x7fffffff) - 1;
     const int xhi = __reduce_max_sync(0xffffffffu, active ? hx : -1) + 1;
-    // FP32 screen: beyond cutneigh + margin never a neighbour, within
-    // cutneigh - margin always one; only the band between takes the FP64 test
-    const float pre = (float)A.cutneigh + R.fmargin, sure = (float)A.cutneigh - R.fmargin;
-    const float pre2 = pre * pre, sure2 = sure * sure;
-    int nin = 0, nout = 0, nh = 0;
-    int fin = 0, fout = 0;   // this lane's entries of each segment already written
-    // entry = (neighbour's list slot << IMG_BITS) | image code
-    auto stage = [&](int val, bool incut) {
-      if (incut) st_in[nin++ & (STAGE_ROWS - 1)][lane] = val;
-      else st_out[nout++ & (STAGE_ROWS - 1)][lane] = val;
-    };
-    // every lane writes its staged entries, row by row: front segment
-    // entries [fin, nin) to rows fin.., back segment entries [fout, nout)
-    // to rows cap-1-fout down
-    auto flush = [&]() {
-      int lo = __reduce_min_sync(0xffffffffu, active ? fin : 0x7fffffff);
-      int hi = __reduce_max_sync(0xffffffffu, active ? nin : 0);
-      for (int k = lo; k < hi; k++)
-        if (active && k >= fin && k < nin && k < A.cap)
-          A.nbr_full[(size_t)k * A.nsi + q.slot] = st_in[k & (STAGE_ROWS - 1)][lane];
-      lo = __reduce_min_sync(0xffffffffu, active ? fout : 0x7fffffff);
-      hi = __reduce_max_sync(0xffffffffu, active ? nout : 0);
-      for (int k = lo; k < hi; k++)
-        if (active && k >= fout && k < nout && k < A.cap)
-          A.nbr_full[(size_t)(A.cap - 1 - k) * A.nsi + q.slot] = st_out[k & (STAGE_ROWS - 1)][lane];
-      fin = nin;
-      fout = nout;
-    };
-    for (int oz = -1; oz <= 1; oz++) {
-      int cz, Wz;
-      wrap_cell(hz + oz, nc2, cz, Wz);
-      for (int oy = -1; oy <= 1; oy++) {
-        int cy, Wy;
-        wrap_cell(hy + oy, nc1, cy, Wy);
-        const int rowbase = R.abase + (cz * nc1 + cy) * nc0;
-        // runs: unwrapped x in [xlo, -1] (the cell nc0 - 1 one image left),
-        // [0, nc0 - 1], [nc0, xhi] (the cell 0 one image right)
-        for (int run = -1; run <= 1; run++) {
-          const int u0 = run < 0 ? xlo : (run == 0 ? max(xlo, 0) : max(xlo, nc0));
-          const int u1 = run < 0 ? min(xhi, -1) : (run == 0 ? min(xhi, nc0 - 1) : xhi);
-          if (u0 > u1) continue;
-          const int Wx = run;
-          int W[3] = {Wx, Wy, Wz};
-          // the lane's position less the run's image shift (once per run)
-          const float rx = __fsub_rn(wx, (float)(Wx * R.b.L[0]));
-          const float ry = __fsub_rn(wy, (float)(Wy * R.b.L[1]));
-          const float rz = __fsub_rn(wz, (float)(Wz * R.b.L[2]));
-          // this run's image relative to the lane's atom
-          const int s0 = Wx - q.ti[0], s1 = Wy - q.ti[1], s2 = Wz - q.ti[2];
-          const bool zero = (s0 == 0 && s1 == 0 && s2 == 0);
-          const bool far = s0 < -1 || s0 > 1 || s1 < -1 || s1 > 1 || s2 < -1 || s2 > 1;
-          const int code = far ? 0 : img_code(s0, s1, s2);
-          const int beg = A.acell_start[rowbase + u0 - Wx * nc0], end = A.acell_start[rowbase + u1 - Wx * nc0 + 1];
-          // candidate pj at list slot ks
-          // the FP32 distance in explicitly rounded operations: the
-          // in-cutoff mark below decides an entry's list segment, so every
-          // kernel that builds these lists (grid and SM-local forms) must
-          // round it the same way, whatever the compiler would contract
-          auto consider = [&](const float4 &pj, int ks) {
-            const float ex = __fsub_rn(rx, pj.x);
-            const float ey = __fsub_rn(ry, pj.y);
-            const float ez = __fsub_rn(rz, pj.z);
-            const float r2 = __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex)));
-            if (r2 > pre2) return;
-            const int j = __float_as_int(pj.w);
-            if (r2 < sure2 && !A.want_half) {
-              if (zero && j == q.i) return;
-              if (far) {
-                atomicExch(&A.overflow[2], 1);
-                return;
-              }
-              stage((ks << IMG_BITS) | code, r2 < fcut2);
-            } else {
-              try_atom(A, q, j, W, nh, [&](int, int c) {
-                stage((ks << IMG_BITS) | (c & (IN_CUT - 1)), (c & IN_CUT) != 0);
-              });
-            }
-          };
-          // candidates four at a time: the four broadcast loads are in
-          // flight together instead of one load's latency per candidate
-          int k = beg;
-          for (; k + 4 <= end; k += 4) {
-            const float4 p0 = A.acell_pos32[k], p1 = A.acell_pos32[k + 1];
-            const float4 p2 = A.acell_pos32[k + 2], p3 = A.acell_pos32[k + 3];
-            // room for four more entries in every lane's rings
-            if (__any_sync(0xffffffffu, active && (nin - fin > STAGE_ROWS - 4 || nout - fout > STAGE_ROWS - 4)))
-              flush();
-            if (active) {
-              consider(p0, k);
-              consider(p1, k + 1);
-              consider(p2, k + 2);
-              consider(p3, k + 3);
-            }
-          }
-          for (; k < end; k++) {
-            const float4 pj = A.acell_pos32[k];
-            if (__any_sync(0xffffffffu, active && (nin - fin >= STAGE_ROWS || nout - fout >= STAGE_ROWS)))
-              flush();
-            if (active) consider(pj, k);
-          }
-        }
+    // positions relative to the corner of the part's first cell
+    const unsigned ox = fix20((xlo + 1) / R.ag.inv[0]), oy = fix20(hy / R.ag.inv[1]), oz = fix20(hz / R.ag.inv[2]);
+    const unsigned Lx = fix20(R.b.L[0]), Ly = fix20(R.b.L[1]), Lz = fix20(R.b.L[2]);
+    const bool near = active && qh.x != FAR_ATOM;
+    const int ix = (int)(qh.x - ox), iy = (int)(qh.y - oy), iz = (int)(qh.z - oz);
+    const float wx = near ? (float)ix * QUANTUM : 1e18f, wy = (float)iy * QUANTUM, wz = (float)iz * QUANTUM;
+    const F2 wx2 = f2_pack(wx, wx), wy2 = f2_pack(wy, wy), wz2 = f2_pack(wz, wz);
+    // the box around the part's atoms
+    auto box_lo = [&](int v) { return (float)__reduce_min_sync(0xffffffffu, near ? v : 0x7fffffff) * QUANTUM; };
+    auto box_hi = [&](int v) { return (float)__reduce_max_sync(0xffffffffu, near ? v : (int)0x80000000) * QUANTUM; };
+    const float bx0 = box_lo(ix), by0 = box_lo(iy), bz0 = box_lo(iz), bx1 = box_hi(ix), by1 = box_hi(iy), bz1 = box_hi(iz);
+    // FP32 screen: a separation carries at most 1.5 quanta of each component,
+    // the rounding of two coordinates no longer than the part's span, and its
+    // own: together under 6e-6 A + 3e-7 span; the margin is over six times that
+    const float span = (float)((xhi - xlo + 1) / R.ag.inv[0] + 3.0 / R.ag.inv[1] + 3.0 / R.ag.inv[2]);
+    const float margin = 1e-4f + 2e-6f * span;
+    const float pre = (float)A.cutneigh + margin, sure = (float)A.cutneigh - margin;
+    const float pre2 = __uint_as_float(__float_as_uint(pre * pre) + 1u);   // r2 <= pre^2 as r2 < pre2
+    const float sure2 = sure > 0.0f ? sure * sure : 0.0f, in2 = (float)A.cutforcesq;
+    const float reach2 = (pre + margin) * (pre + margin);
+    const F2 lim_pre = f2_pack(pre2, pre2), lim_sure = f2_pack(sure2, sure2), lim_in = f2_pack(in2, in2);
+
+    // the part's runs, one per lane (9 rows x 3): unwrapped x in [xlo, -1]
+    // (the cell nc0 - 1 one image left), [0, nc0 - 1], [nc0, xhi] (the cell 0
+    // one image right), each in words of 32 candidates
+    int beg = 0, end = 0, rn = 0, rcode = 0;
+    if (lane < 27) {
+      const int run = lane % 3 - 1, ry = lane / 3;
+      int cy, Wy, cz, Wz;
+      wrap_cell(hz + ry / 3 - 1, nc2, cz, Wz);
+      wrap_cell(hy + ry % 3 - 1, nc1, cy, Wy);
+      const int u0 = run < 0 ? xlo : (run == 0 ? max(xlo, 0) : max(xlo, nc0));
+      const int u1 = run < 0 ? min(xhi, -1) : (run == 0 ? min(xhi, nc0 - 1) : xhi);
+      if (u0 <= u1) {
+        const int rowbase = R.abase + (cz * nc1 + cy) * nc0 - run * nc0;
+        beg = A.acell_start[rowbase + u0];
+        end = A.acell_start[rowbase + u1 + 1];
+        rn = (end - beg + 31) >> 5;
+        rcode = img_code(run, Wy, Wz);
       }
     }
-    flush();
-    if (active) {
-      A.site_from[q.slot] = make_int2(nin, nout);
-      finish_counts(A, q.slot, nin, nout, nh);
+    int off = rn;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, off, o);
+      if (lane >= o) off += v;
+    }
+    const int nraw = __shfl_sync(0xffffffffu, off, 31);
+    // this lane's candidate of raw word r: list slot (-1 past the run's end) and image code
+    auto candidate = [&](int r, int &code) {
+      const int m = __popc(__ballot_sync(0xffffffffu, off <= r));   // the word's run
+      const int first = __shfl_sync(0xffffffffu, beg, m) + 32 * (r - __shfl_sync(0xffffffffu, off - rn, m));
+      code = __shfl_sync(0xffffffffu, rcode, m);
+      const int k = first + lane;
+      return k < __shfl_sync(0xffffffffu, end, m) ? k : -1;
+    };
+    auto fetch = [&](int k) {
+      return k >= 0 ? make_int3(A.acell_x[k], A.acell_y[k], A.acell_z[k]) : make_int3(FAR_ATOM, 0, 0);
+    };
+    // its coordinates under the run's image, and whether they are in reach
+    auto place = [&](const int3 c, int code, float &x, float &y, float &z) {
+      unsigned ux = c.x, uy = c.y, uz = c.z;
+      if (code != IMG_ZERO) {
+        int W0, W1, W2;
+        img_decode(code, W0, W1, W2);
+        ux += W0 * Lx;
+        uy += W1 * Ly;
+        uz += W2 * Lz;
+      }
+      x = (float)(int)(ux - ox) * QUANTUM;
+      y = (float)(int)(uy - oy) * QUANTUM;
+      z = (float)(int)(uz - oz) * QUANTUM;
+      const float dx = fmaxf(fmaxf(bx0 - x, x - bx1), 0.0f), dy = fmaxf(fmaxf(by0 - y, y - by1), 0.0f),
+                  dz = fmaxf(fmaxf(bz0 - z, z - bz1), 0.0f);
+      return c.x != FAR_ATOM && dx * dx + dy * dy + dz * dz <= reach2;
+    };
+    auto keep = [&](unsigned m, int at, int k, int code, float x, float y, float z) {
+      at += __popc(m & lanemask_lt());
+      reinterpret_cast<float *>(kx4)[at] = x;
+      reinterpret_cast<float *>(ky4)[at] = y;
+      reinterpret_cast<float *>(kz4)[at] = z;
+      entry[at] = (k << IMG_BITS) | code;
+      if (code == IMG_ZERO && (unsigned)(k - chunk * 32) < 32u) self_at[k - chunk * 32] = at;
+    };
+
+    int nin = 0, nout = 0, nh = 0;
+    int r = 0;
+    int code1 = 0, k1 = -1;
+    int3 c1 = make_int3(FAR_ATOM, 0, 0);
+    if (NW == 1) {
+      k1 = candidate(0, code1);
+      c1 = fetch(k1);
+    }
+    while (r < nraw) {
+      sync();
+      if (warp == 0) self_at[lane] = -1;
+      sync();
+      int n = 0;   // candidates kept
+      if (NW == 1) {
+        // the next word's candidates are on their way while one is placed
+        while (r < nraw && n + 32 <= MAXW * 32) {
+          const int k = k1, code = code1;
+          const int3 c = c1;
+          if (++r < nraw) {
+            k1 = candidate(r, code1);
+            c1 = fetch(k1);
+          }
+          float x, y, z;
+          const bool ok = place(c, code, x, y, z);
+          const unsigned m = __ballot_sync(0xffffffffu, ok);
+          if (ok) keep(m, n, k, code, x, y, z);
+          n += __popc(m);
+        }
+      } else {
+        const int r1 = min(nraw, r + MAXW);
+        for (int u = r + warp; u < r1; u += NW) {
+          int code;
+          float x, y, z;
+          const int k = candidate(u, code);
+          const unsigned m = __ballot_sync(0xffffffffu, place(fetch(k), code, x, y, z));
+          if (lane == 0) kept[u - r] = m;
+        }
+        __syncthreads();
+        int at = lane < r1 - r ? __popc(kept[lane]) : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, at, o);
+          if (lane >= o) at += v;
+        }
+        n = __shfl_sync(0xffffffffu, at, 31);
+        for (int u = r + warp; u < r1; u += NW) {
+          int code;
+          float x, y, z;
+          const int k = candidate(u, code);
+          const unsigned m = kept[u - r];
+          const int a0 = u > r ? __shfl_sync(0xffffffffu, at, (u - r - 1) & 31) : 0;
+          place(fetch(k), code, x, y, z);
+          if ((m >> lane) & 1u) keep(m, a0, k, code, x, y, z);
+        }
+        r = r1;
+      }
+      sync();
+      const int nw = (n + 31) >> 5;
+      for (int w = warp; w < nw; w += NW) {
+        // the distance in explicitly rounded operations (packed ones round as
+        // the scalar ones): the in-cutoff mark decides an entry's list segment,
+        // so every kernel that builds these lists must round it the same way
+        unsigned mp = 0, ms = 0, mi = 0;
+#pragma unroll
+        for (int g = 0; g < 8; g++) {
+          const float4 x = kx4[w][g], y = ky4[w][g], z = kz4[w][g];
+          const F2 ex = f2_sub(wx2, f2_pack(x.x, x.y)), fx = f2_sub(wx2, f2_pack(x.z, x.w));
+          const F2 ey = f2_sub(wy2, f2_pack(y.x, y.y)), fy = f2_sub(wy2, f2_pack(y.z, y.w));
+          const F2 ez = f2_sub(wz2, f2_pack(z.x, z.y)), fz = f2_sub(wz2, f2_pack(z.z, z.w));
+          const F2 r2 = f2_fma(ez, ez, f2_fma(ey, ey, f2_mul(ex, ex)));
+          const F2 s2 = f2_fma(fz, fz, f2_fma(fy, fy, f2_mul(fx, fx)));
+          mp = f2_signs(f2_signs(mp, f2_sub(r2, lim_pre)), f2_sub(s2, lim_pre));
+          ms = f2_signs(f2_signs(ms, f2_sub(r2, lim_sure)), f2_sub(s2, lim_sure));
+          mi = f2_signs(f2_signs(mi, f2_sub(r2, lim_in)), f2_sub(s2, lim_in));
+        }
+        const int nv = n - 32 * w;
+        unsigned valid = near ? (nv < 32 ? 0xffffffffu << (32 - nv) : 0xffffffffu) : 0u;
+        // its own place under its own image (an atom of the box: image zero)
+        const int self = self_at[lane];
+        if (unwrapped && self >= 0 && (self >> 5) == w) valid &= ~(0x80000000u >> (self & 31));
+        mp &= valid;
+        unsigned acc = ms & mp, in = mi & acc, band = mp & ~acc;
+        if (A.want_half || !unwrapped) {
+          // half lists, and atoms outside the box, take every candidate
+          // through the exact test, in order
+          band = mp;
+          acc = in = 0;
+        }
+        while (band) {
+          const int at = __clz(band);
+          const unsigned bit = 0x80000000u >> at;
+          band &= ~bit;
+          const int e = entry[32 * w + at];
+          int W[3];
+          img_decode(e & ((1 << IMG_BITS) - 1), W[0], W[1], W[2]);
+          try_atom(A, q, (int)__double_as_longlong(A.acell_pos[e >> IMG_BITS].w), W, nh, [&](int, int cd) {
+            acc |= bit;
+            if (cd & IN_CUT) in |= bit;
+          });
+        }
+        __syncwarp();
+        m_acc[32 * w + lane] = acc;
+        m_in[32 * w + lane] = in;
+      }
+      sync();
+      // write-out of one segment: front entries to rows n.., back ones from
+      // row cap - 1 down
+      auto write = [&](const bool front, int &n) {
+        auto mask = [&](int w) { return front ? m_in[32 * w + lane] : m_acc[32 * w + lane] & ~m_in[32 * w + lane]; };
+        unsigned some = 0;   // the lane's words with entries, first word in the top bit
+        for (int w = 0; w < nw; w++)
+          if (mask(w)) some |= 0x80000000u >> w;
+        int w = 0;
+        unsigned bits = 0;
+        while (__any_sync(0xffffffffu, (some | bits) != 0)) {
+          if (!bits && some) {
+            w = __clz(some);
+            some &= ~(0x80000000u >> w);
+            bits = mask(w);
+          }
+          if (bits) {
+            const int at = __clz(bits);
+            bits &= ~(0x80000000u >> at);
+            int e = entry[32 * w + at];
+            if (!unwrapped) {
+              int W0, W1, W2;
+              img_decode(e & ((1 << IMG_BITS) - 1), W0, W1, W2);
+              e = (e & ~((1 << IMG_BITS) - 1)) | img_code(W0 - q.ti[0], W1 - q.ti[1], W2 - q.ti[2]);
+            }
+            if (n < A.cap) A.nbr_full[(size_t)(front ? n : A.cap - 1 - n) * A.nsi + h] = e;
+            n++;
+          }
+        }
+      };
+      if (NW == 1) {
+        write(true, nin);
+        write(false, nout);
+      } else if (warp == 0) {
+        write(true, nin);
+      } else if (warp == 1) {
+        write(false, nout);
+      }
+    }
+    if (NW > 1) {
+      if (warp == 1) back[lane] = nout;
+      __syncthreads();
+      nout = back[lane];
+    }
+    if (warp == 0 && active) {
+      A.site_from[h] = make_int2(nin, nout);
+      finish_counts(A, h, nin, nout, nh);
     }
   }
 }
 
-// The single-system forms as the compiler allocates them (96 registers with
-// the candidate loads four at a time, 118 in the persistent form: a cap at 20
-// resident warps per SM, 88 registers, was 10 % slower); the batch form
-// capped at 64 registers (a few bytes spilled) so that 32 warps are resident
-// per SM: 10 % faster on a 64-replica batch, where the same cap slowed the
-// single-system form.
-__global__ void __launch_bounds__(32) k_build_atoms(BuildArgs A, OneRep P) { build_atoms_chunk(A, P, blockIdx.x); }
-__global__ void __launch_bounds__(32, 32) k_build_atoms(BuildArgs A, ManyRep P) {
-  build_atoms_chunk(A, P, blockIdx.x);
+// Large systems: one warp per chunk.  Small ones (below SMALL_CHUNKS per SM),
+// whose chunks would leave most of the chip idle: the chunk's words over four
+// warps and the two segments' write-outs over two.  Measured per build against
+// one warp walking its chunk candidate by candidate (42 instructions a
+// candidate, entries staged in shared memory): 4.18 M atoms 6.05 -> 2.02 ms,
+// 1.05 M 1.56 -> 0.54 ms, 272 k 474 -> 177 us, 4,374 atoms (four warps)
+// 183 -> 47 us, 64 replicas of 1.44 M atoms 1.37 -> 0.51 ms.
+template <int NW, class RP>
+__global__ void __launch_bounds__(32 * NW) k_build_atoms(BuildArgs A, RP P) {
+  build_atoms_chunk<NW>(A, P, blockIdx.x);
 }
 
 // Single systems: persistent warps taking the chunks in SM-local runs (one
@@ -988,7 +1186,7 @@ __global__ void __launch_bounds__(32) k_build_atoms_sm(BuildArgs A, OneRep P, in
   for (;;) {
     const int chunk = sm_run(cnt, nsm, nchunk, v);
     if (chunk < 0) return;
-    build_atoms_chunk(A, P, chunk);
+    build_atoms_chunk<1>(A, P, chunk);
   }
 }
 
@@ -1293,15 +1491,6 @@ void neigh_plan(Ctx &c, bool want_half) {
       R.reach_budget = std::max(ereach, std::min(std::max(1.2 * ereach, ereach + 2.0), room));
     }
     setup_grids(c, R, c.rep_ne[r] > 0);
-    // FP32 separations (a wrapped position less an image shift, |.| <= 2X
-    // with X = |lo| + |hi| + L, minus a wrapped candidate) carry at most ~4
-    // ulp(X) of rounding per distance; 16 ulp of 2X bounds it with room to
-    // spare
-    {
-      double X = 1.0;
-      for (int d = 0; d < 3; d++) X = std::max(X, std::fabs(R.b.lo[d]) + std::fabs(R.b.hi[d]) + R.b.L[d]);
-      R.fmargin = (float)(16.0 * std::ldexp(1.0, std::ilogb(2.0 * X) - 23));
-    }
     // fixed-point frame of the mixed form: quantum 2^-26 A, box length in
     // quanta modulo 2^32 (pair separations are taken modulo 2^32 as well)
     for (int d = 0; d < 3; d++) {
@@ -1338,7 +1527,7 @@ void neigh_plan(Ctx &c, bool want_half) {
   c.xss.reserve(std::max(c.xs.n, (size_t)1));
   c.acell_start.reserve(c.agrid.ncell + 1);
   c.acell_pos.reserve(std::max(c.na, 1));
-  c.acell_pos32.reserve(std::max(c.na, 1));
+  c.acell_fix.reserve(3 * (size_t)std::max(c.na, 1));
   c.acell_of.reserve(std::max(c.na, 1));
   c.ecell_start.reserve(c.egrid.ncell + 1);
   c.ecell_near.reserve(c.egrid.ncell + 1);
@@ -1457,8 +1646,8 @@ void neigh_build_async(Ctx &c, bool want_half) {
         if (c.nrep == 1 && c.ne)
           k_ecell_near<<<nblk(c.agrid.ncell, 256), 256, 0, c.stream>>>(c.acell_start.p, c.rep_h[0].ag,
                                                                        c.acell_near.p);
-        k_gather_pos<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.slot_atom.p, c.cell_key2.p, c.na,
-                                                            c.acell_pos.p, c.acell_pos32.p, c.atom_slot.p,
+        k_gather_pos<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.slot_atom.p, c.cell_key2.p, c.na, P,
+                                                            c.acell_pos.p, c.acell_fix.p, c.atom_slot.p,
                                                             c.acell_of.p);
       } else {
         CACB200_CUDA(cudaMemsetAsync(c.acell_start.p, 0, sizeof(int) * (c.agrid.ncell + 1), c.stream));
@@ -1485,7 +1674,9 @@ void neigh_build_async(Ctx &c, bool want_half) {
     A.eframe = c.eframe.p;
     A.acell_start = c.acell_start.p;
     A.acell_pos = c.acell_pos.p;
-    A.acell_pos32 = c.acell_pos32.p;
+    A.acell_x = c.acell_fix.p;
+    A.acell_y = A.acell_x + c.na;
+    A.acell_z = A.acell_y + c.na;
     A.acell_of = c.acell_of.p;
     A.ecell_start = c.ecell_start.p;
     A.ecell_near = (c.nrep == 1 && c.ne) ? c.ecell_near.p : nullptr;
@@ -1540,22 +1731,25 @@ void neigh_build_async(Ctx &c, bool want_half) {
     }
     if (c.na) {
       KernelTimer t(c, "build_atoms");
+      const int nchunk = (c.na + 31) / 32;
+      bool done = false;
+      if (!want_half && nchunk < SMALL_CHUNKS * c.num_sms) {   // half lists are stored in order by one warp
+        k_build_atoms<4><<<nchunk, 128, 0, c.stream>>>(A, P);
+        done = true;
+      }
       if constexpr (std::is_same_v<decltype(P), OneRep>) {
-        if (c.work_queue) {
+        if (!done && c.work_queue) {
           static const int per_sm = [] {
             int b = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_build_atoms_sm, 32, 0);
             return b > 0 ? b : 1;
           }();
           CACB200_CUDA(cudaMemsetAsync(c.sm_counter.p, 0, sizeof(int) * c.num_sms, c.stream));
-          k_build_atoms_sm<<<per_sm * c.num_sms, 32, 0, c.stream>>>(A, P, (c.na + 31) / 32, c.sm_counter.p,
-                                                                   c.num_sms);
-        } else {
-          k_build_atoms<<<(c.na + 31) / 32, 32, 0, c.stream>>>(A, P);
+          k_build_atoms_sm<<<per_sm * c.num_sms, 32, 0, c.stream>>>(A, P, nchunk, c.sm_counter.p, c.num_sms);
+          done = true;
         }
-      } else {
-        k_build_atoms<<<(c.na + 31) / 32, 32, 0, c.stream>>>(A, P);
       }
+      if (!done) k_build_atoms<1><<<nchunk, 32, 0, c.stream>>>(A, P);
     }
     if (c.na && c.ne) {
       if (split) CACB200_CUDA(cudaStreamWaitEvent(c.stream, c.items_ev, 0));
