@@ -830,7 +830,7 @@ int cacb200_work_queue(cacb200_ctx *ctx, int enable, int tiles[3]) {
   API_BEGIN
   if (enable >= 0) {
     c.work_queue = enable != 0;
-    c.work_gen = -1;
+    drop_graphs(c);   // they hold the launch shapes
   }
   if (tiles)
     for (int k = 0; k < 3; k++) tiles[k] = c.work_tile[k];

@@ -309,6 +309,9 @@ struct Ctx {
   DBuf<float4> frho_val32, frho_der32;
   DBuf<float4> rz32;              // the same r-knot records in FP32 (32 bytes)
   bool have_mixed_tables = false;
+  DBuf<float4> fast32;            // smooth part of the r-splines as cubics in r^2 (pair32.cu)
+  int fast_lo = 0, fast_cnt = 0;
+  float fast_inv_ds = 0.0f;
   DBuf<int4> pos32;              // mixed form: fixed-point site records (qx, qy, qz, F' bits)
 
   FireParams fire;
@@ -327,21 +330,14 @@ struct Ctx {
   double graph_dt = 0.0;
   int graph_every = 0;
   long graph_launches = 0;
-  // block sizes of the force-only pair passes, chosen by timing (valid for
-  // tune_gen == gen); FP64 and mixed forms
-  long tune_gen = -1, tune_gen32 = -1;
+  // block sizes of the force-only pair passes: FP64 chosen by timing (valid
+  // for tune_gen == gen), mixed by the system's size
+  long tune_gen = -1;
   int tb_rho = 128, tb_force = 128, tb_rho32 = 128, tb_force32 = 128;
-  // batches, mixed form: persistent work-queue launches of the EAM passes.
-  // Items are runs of consecutive list slots of one replica, the largest
-  // replicas first; the run length (tile) is chosen per replica size class
-  // (i-sites < 8192, < 32768, larger) by timing when the plan changes.
+  // persistent forms of the pair passes and the atom build
   bool work_queue = true;
-  DBuf<int2> work_items;
-  DBuf<int> work_counter;
   DBuf<int> sm_counter;   // single systems: run counters of the SM-local ranges (rho, force)
-  int nwork_items = 0;
-  long work_gen = -1;
-  int work_tile[3] = {0, 0, 0};
+  int work_tile[3] = {0, 0, 0};    // batches, mixed form: list slots a resident block takes at a time
   double escale_node_last = 0.0;   // node energy scale of the last evaluation
   DBuf<int> rep_meta;              // [4][nrep] aoff, na, eoff, ne (per-replica energy)
   DBuf<double> rep_energy;         // [nrep]

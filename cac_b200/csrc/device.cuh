@@ -100,6 +100,17 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Pair passes: G neighbouring lanes share an i-site.  Lane g of the group
+// walks list rows g, g + G, ...; the lanes' sums are added in a fixed tree
+// (the same for every launch form and system size, so a site's result depends
+// on its list alone).
+template <int G, class T>
+__device__ __forceinline__ T lanes_sum(T v) {
+#pragma unroll
+  for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Deterministic block reduction of NV doubles into out[blockIdx.x * NV + k].
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(double (&vals)[NV], double *out) {

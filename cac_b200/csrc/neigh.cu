@@ -1594,7 +1594,6 @@ void neigh_plan(Ctx &c, bool want_half) {
     // only the box moved (fix deform): the block sizes chosen for this
     // system stay valid
     if (c.tune_gen == gen_before) c.tune_gen = c.gen;
-    if (c.tune_gen32 == gen_before) c.tune_gen32 = c.gen;
     c.box_replan = false;
   }
   c.plan_na = c.na;

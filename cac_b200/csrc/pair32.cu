@@ -19,6 +19,7 @@
 // copies of the FP64 splines.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "ctx.cuh"
@@ -35,7 +36,6 @@ inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 struct FixGrid {
   double lo[3];
   double scale[3];
-  float inv[3];
   int Lq[3];
   const Rep *reps;          // batches (null for one system)
   const int *site_rep;      // [nsite_i]
@@ -113,6 +113,11 @@ __global__ void k_pair_table32(const double4 *xs, const int *slot_atom, const do
   }
 }
 
+// Positions are in quanta of 2^-26 A in every replica; separations stay in
+// quanta through the pair arithmetic (scaling by a power of two is exact) and
+// the sums are scaled once per site.
+constexpr float QUANTUM = 1.0f / 67108864.0f;
+
 struct Args32 {
   const int4 *pos;
   const int *nbr;          // lists and counts indexed by list slot
@@ -130,178 +135,249 @@ struct Args32 {
   double escale_node, vscale_node;
 };
 
-__device__ __forceinline__ float fix_delta(int qi, int qj, int s, int Lq, float inv) {
-  const unsigned sl = (unsigned)s * (unsigned)Lq;   // s in {-1, 0, 1}, modulo 2^32
-  unsigned d = (unsigned)qi - (unsigned)qj - sl;
-  return (float)(int)d * inv;
-}
-
-// fixed-point frame (box lengths and quanta) of i-site i's replica
-struct SiteFix {
-  int Lq[3];
-  float inv[3];
-};
-__device__ __forceinline__ SiteFix site_fix(const Args32 &A, int i) {
-  SiteFix F;
-  if (A.G.reps) {
-    const Rep *R = A.G.reps + A.G.site_rep[i];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      F.Lq[d] = R->Lq[d];
-      F.inv[d] = R->qinv[d];
-    }
-  } else {
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      F.Lq[d] = A.G.Lq[d];
-      F.inv[d] = A.G.inv[d];
-    }
-  }
-  return F;
-}
-
 __device__ __forceinline__ int site_of_slot(const Args32 &A, int t) { return t < A.na ? A.slot_atom[t] : t; }
 
-// separation of site i (record oi) from neighbour entry v; wj = F'(j)
-__device__ __forceinline__ void sep32(const Args32 &A, const SiteFix &F, const int4 &oi, int v, float &dx,
-                                      float &dy, float &dz, float &wj) {
-  int j = v >> IMG_BITS, code = v & ((1 << IMG_BITS) - 1);
-  int4 oj = __ldg(A.pos + j);
-  int s[3] = {0, 0, 0};
-  if (code != IMG_ZERO) img_decode(code, s[0], s[1], s[2]);
-  dx = fix_delta(oi.x, oj.x, s[0], F.Lq[0], F.inv[0]);
-  dy = fix_delta(oi.y, oj.y, s[1], F.Lq[1], F.inv[1]);
-  dz = fix_delta(oi.z, oj.z, s[2], F.Lq[2], F.inv[2]);
-  wj = __int_as_float(oj.w);
-}
-
-template <class F>
-__device__ __forceinline__ void walk32(const Args32 &A, const SiteFix &fx, const int4 &oi, const int *nb, int n,
-                                       F &&f) {
-  int k = 0;
-  for (; k + 4 <= n; k += 4) {
-    int v0 = __ldcs(nb + (size_t)k * A.nsi), v1 = __ldcs(nb + (size_t)(k + 1) * A.nsi);
-    int v2 = __ldcs(nb + (size_t)(k + 2) * A.nsi), v3 = __ldcs(nb + (size_t)(k + 3) * A.nsi);
-    float d[4][4];
-    sep32(A, fx, oi, v0, d[0][0], d[0][1], d[0][2], d[0][3]);
-    sep32(A, fx, oi, v1, d[1][0], d[1][1], d[1][2], d[1][3]);
-    sep32(A, fx, oi, v2, d[2][0], d[2][1], d[2][2], d[2][3]);
-    sep32(A, fx, oi, v3, d[3][0], d[3][1], d[3][2], d[3][3]);
+// A site's sums are kept in four partial sums: entry k of a walk goes to
+// partial k mod 4, and the partials are added as (0 + 1) + (2 + 3).  G lanes
+// share a site (G = 1, 2 or 4; lane g walks entries g, g + G, ...) and each
+// holds 4 / G of the partials, so a site's result is the same bit for bit
+// whatever G is: large systems take one lane per site, small ones, which
+// would leave the chip idle, more.
+template <int G>
+struct Sum4 {
+  float a[4 / G];
+  __device__ __forceinline__ Sum4() {
 #pragma unroll
-    for (int u = 0; u < 4; u++) f(d[u][0], d[u][1], d[u][2], d[u][3]);
+    for (int k = 0; k < 4 / G; k++) a[k] = 0.0f;
   }
-  for (; k < n; k++) {
-    float dx, dy, dz, wj;
-    sep32(A, fx, oi, __ldcs(nb + (size_t)k * A.nsi), dx, dy, dz, wj);
-    f(dx, dy, dz, wj);
+  // the site's sum, in every lane of its group (every lane of the warp calls it)
+  __device__ __forceinline__ float total() const {
+    float t[4 / G];
+#pragma unroll
+    for (int k = 0; k < 4 / G; k++) t[k] = lanes_sum<G>(a[k]);
+    if constexpr (G == 1) return __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
+    else if constexpr (G == 2) return __fadd_rn(t[0], t[1]);
+    else return t[0];
+  }
+};
+
+// Walks n entries of a list: each lane takes four at a time, the next four
+// entries loaded ahead and the four records issued back to back before any is
+// used.  Entries past the end are walked as pairs too far apart to count.
+// f(partial, dx, dy, dz, rsq, w): the separation from the neighbour and its
+// square, in quanta; w = F' of the neighbour.
+template <int G, class F>
+__device__ __forceinline__ void walk32(const Args32 &A, int t, int i, const int4 &oi, const int *nb, int n, F &&f) {
+  const size_t step = (size_t)G * A.nsi;
+  const int *p = nb + (size_t)(threadIdx.x % G) * A.nsi;
+  int v[4];
+  auto load = [&](int left) {   // entries this lane still has
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = u < left ? __ldcs(p + u * step) : (t << IMG_BITS) | IMG_ZERO;
+    p += 4 * step;
+  };
+  int left = (n - (int)(threadIdx.x % G) + G - 1) / G;
+  load(left);
+  for (; left > 0; left -= 4) {
+    int4 o[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) o[u] = __ldg(A.pos + (v[u] >> IMG_BITS));
+    // images: shift the neighbour by s L, s in {-1, 0, 1}, modulo 2^32
+    if (((v[0] ^ IMG_ZERO) | (v[1] ^ IMG_ZERO) | (v[2] ^ IMG_ZERO) | (v[3] ^ IMG_ZERO)) & ((1 << IMG_BITS) - 1)) {
+      const int *Lq = A.G.reps ? A.G.reps[A.G.site_rep[i]].Lq : A.G.Lq;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        int sx, sy, sz;
+        img_decode(v[u] & ((1 << IMG_BITS) - 1), sx, sy, sz);
+        o[u].x += sx * Lq[0];
+        o[u].y += sy * Lq[1];
+        o[u].z += sz * Lq[2];
+      }
+    }
+    const int now = left;
+    load(left - 4);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const float dx = (float)(int)((unsigned)oi.x - (unsigned)o[u].x), dy = (float)(int)((unsigned)oi.y - (unsigned)o[u].y),
+                  dz = (float)(int)((unsigned)oi.z - (unsigned)o[u].z);
+      float rsq = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+      if (u && u >= now) rsq = 1e30f;
+      f(u % (4 / G), dx, dy, dz, rsq, __int_as_float(o[u].w));
+    }
   }
 }
 
 // A site's list: the inner prefix on its own, then the rest unless the
 // prefix still holds every pair of the site inside the cutoff (walk_rest,
-// device.cuh; an entry's arithmetic depends on its place in a walk, so the
+// device.cuh; an entry's partial depends on its place in a walk, so the
 // prefix is always walked alone).
-template <class F>
+template <int G, class F>
 __device__ __forceinline__ void for_each32(const Args32 &A, int t, int i, const int4 &oi, F &&f) {
-  const SiteFix fx = site_fix(A, i);
   const int n_in = A.num_in[t], n = A.num[t];
   const int *nb = A.nbr + t;
   const bool rest = n > n_in && walk_rest(A.prefix, i, A.G.reps ? A.G.site_rep[i] : 0);
 #pragma unroll 1
   for (int seg = 0; seg < (rest ? 2 : 1); seg++)
-    walk32(A, fx, oi, seg ? nb + (size_t)(A.cap - (n - n_in)) * A.nsi : nb, seg ? n - n_in : n_in, f);
+    walk32<G>(A, t, i, oi, seg ? nb + (size_t)(A.cap - (n - n_in)) * A.nsi : nb, seg ? n - n_in : n_in, f);
 }
 
-__device__ __forceinline__ void finish32(const Args32 &A, int i, bool valid, const float fi[3], bool ev,
-                                         float esum, const float vsum[6], double eextra_site,
-                                         double eextra_global) {
-  double red[7] = {0, 0, 0, 0, 0, 0, 0};
-  if (valid) {
-    bool atom = i < A.na;
-    int e = 0, g = 0, node = 0;
-    double *fo;
-    if (atom) {
-      fo = A.f + 3 * (size_t)i;
-    } else {
-      e = (i - A.na) / NG;
-      g = (i - A.na) % NG;
-      node = gauss_node(g);
-      fo = A.gaussf + (size_t)e * 24 + 3 * g;
+// Writes force (and per-site energy / virial) of i-site i and adds its global
+// energy / virial to red.
+template <bool EV>
+__device__ __forceinline__ void finish32(const Args32 &A, int i, const float fi[3], float esum, const float vsum[6],
+                                         double eextra_site, double eextra_global, double red[7]) {
+  const bool atom = i < A.na;
+  int e = 0, g = 0, node = 0;
+  double *fo;
+  if (atom) {
+    fo = A.f + 3 * (size_t)i;
+  } else {
+    e = (i - A.na) / NG;
+    g = (i - A.na) % NG;
+    node = gauss_node(g);
+    fo = A.gaussf + (size_t)e * 24 + 3 * g;
+  }
+  fo[0] = fi[0];
+  fo[1] = fi[1];
+  fo[2] = fi[2];
+  if (EV) {
+    const double es = atom ? 0.5 : A.escale_node, vs = atom ? 0.5 : A.vscale_node;
+    if (A.eflag & CACB200_ENERGY_GLOBAL) red[0] += es * (double)esum + eextra_global;
+    if (A.vflag & CACB200_VIRIAL_GLOBAL)
+#pragma unroll
+      for (int k = 0; k < 6; k++) red[1 + k] += vs * (double)vsum[k];
+    if (A.eflag & CACB200_ENERGY_ATOM) {
+      const double v = 0.5 * (double)esum + eextra_site;
+      if (atom) A.eatom[i] = v;
+      else A.enode[(size_t)e * 8 + node] = v;
     }
-    fo[0] = fi[0];
-    fo[1] = fi[1];
-    fo[2] = fi[2];
-    if (ev) {
-      double es = atom ? 0.5 : A.escale_node, vs = atom ? 0.5 : A.vscale_node;
-      if (A.eflag & CACB200_ENERGY_GLOBAL) red[0] = es * (double)esum + eextra_global;
-      if (A.vflag & CACB200_VIRIAL_GLOBAL)
+    if (A.vflag & CACB200_VIRIAL_ATOM) {
+      double *vo = atom ? A.vatom + 6 * (size_t)i : A.vnode + 48 * (size_t)e + 6 * node;
 #pragma unroll
-        for (int k = 0; k < 6; k++) red[1 + k] = vs * (double)vsum[k];
-      if (A.eflag & CACB200_ENERGY_ATOM) {
-        double v = 0.5 * (double)esum + eextra_site;
-        if (atom) A.eatom[i] = v;
-        else A.enode[(size_t)e * 8 + node] = v;
-      }
-      if (A.vflag & CACB200_VIRIAL_ATOM) {
-        double *vo = atom ? A.vatom + 6 * (size_t)i : A.vnode + 48 * (size_t)e + 6 * node;
-#pragma unroll
-        for (int k = 0; k < 6; k++) vo[k] = 0.5 * (double)vsum[k];
-      }
+      for (int k = 0; k < 6; k++) vo[k] = 0.5 * (double)vsum[k];
     }
   }
-  if (ev) block_reduce_store<7>(red, A.partial);
 }
 
-__device__ __forceinline__ void site_frame(const Args32 &A, int i, int4 &oi) { oi = __ldg(A.pos + i); }
+// The pair passes' threads: runs of 32 / G consecutive list slots, one per
+// warp, consecutive warps taking consecutive runs, grid-stride.  body(slot,
+// valid) is called by whole warps.
+template <int G, class F>
+__device__ __forceinline__ void for_each_slot(const Args32 &A, F &&body) {
+  constexpr int S = 32 / G;
+  const int warps = blockDim.x >> 5, nrun = (A.nsi + S - 1) / S;
+  for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < nrun; r += gridDim.x * warps) {
+    const int t = r * S + (threadIdx.x & 31) / G;
+    body(t, t < A.nsi);
+  }
+}
+
+// Per-site sums of a force pass.
+template <int G, bool EV>
+struct ForceSums {
+  Sum4<G> f[3], e[1], v[EV ? 6 : 1];
+  __device__ __forceinline__ void add(int part, float dx, float dy, float dz, float fpair) {
+    f[0].a[part] = __fmaf_rn(dx, fpair, f[0].a[part]);
+    f[1].a[part] = __fmaf_rn(dy, fpair, f[1].a[part]);
+    f[2].a[part] = __fmaf_rn(dz, fpair, f[2].a[part]);
+  }
+  __device__ __forceinline__ void add_ev(int part, float dx, float dy, float dz, float fpair, float phi) {
+    e[0].a[part] = __fadd_rn(e[0].a[part], phi);
+    const float a[6] = {dx * dx, dy * dy, dz * dz, dx * dy, dx * dz, dy * dz};
+#pragma unroll
+    for (int k = 0; k < 6; k++) v[k].a[part] = __fmaf_rn(a[k], fpair, v[k].a[part]);
+  }
+  // totals in A, eV; fscale: of separation times fpair, the force's unit
+  __device__ __forceinline__ void totals(float fscale, float fi[3], float &esum, float vsum[6]) const {
+#pragma unroll
+    for (int d = 0; d < 3; d++) fi[d] = f[d].total() * fscale;
+    if constexpr (EV) {
+      esum = e[0].total();
+#pragma unroll
+      for (int k = 0; k < 6; k++) vsum[k] = v[k].total() * (fscale * QUANTUM);
+    }
+  }
+};
 
 // ---------------------------------------------------------------------- LJ
 
 struct Lj32 {
-  float cutsq, lj1, lj2, lj3, lj4, offset;
+  float cutsq, lj1, lj2, lj3, lj4, offset;   // cutsq in square quanta
 };
 
-template <bool EV>
+template <int G, bool EV>
 __global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj32(Args32 A, Lj32 P) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;   // list slot
-  const bool valid = t < A.nsi;
-  const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
-  float fi[3] = {0, 0, 0}, esum = 0.f, vsum[6] = {0, 0, 0, 0, 0, 0};
-  if (valid) {
-    int4 oi;
-    site_frame(A, t, oi);
-    for_each32(A, t, i, oi, [&](float dx, float dy, float dz, float) {
-      float rsq = dx * dx + dy * dy + dz * dz;
-      if (rsq < P.cutsq) {
-        float r2inv = 1.0f / rsq;
-        float r6inv = r2inv * r2inv * r2inv;
-        float fpair = r6inv * (P.lj1 * r6inv - P.lj2) * r2inv;
-        fi[0] += dx * fpair;
-        fi[1] += dy * fpair;
-        fi[2] += dz * fpair;
-        if (EV) {
-          esum += r6inv * (P.lj3 * r6inv - P.lj4) - P.offset;
-          vsum[0] += dx * dx * fpair;
-          vsum[1] += dy * dy * fpair;
-          vsum[2] += dz * dz * fpair;
-          vsum[3] += dx * dy * fpair;
-          vsum[4] += dx * dz * fpair;
-          vsum[5] += dy * dz * fpair;
+  double red[7] = {0, 0, 0, 0, 0, 0, 0};
+  for_each_slot<G>(A, [&](int t, bool valid) {
+    const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
+    ForceSums<G, EV> S;
+    if (valid) {
+      const int4 oi = __ldg(A.pos + t);
+      for_each32<G>(A, t, i, oi, [&](int part, float dx, float dy, float dz, float rsq, float) {
+        if (rsq < P.cutsq) {
+          const float r2inv = 1.0f / (rsq * (QUANTUM * QUANTUM));
+          const float r6inv = r2inv * r2inv * r2inv;
+          const float fpair = r6inv * __fmaf_rn(P.lj1, r6inv, -P.lj2) * r2inv;
+          S.add(part, dx, dy, dz, fpair);
+          if (EV) S.add_ev(part, dx, dy, dz, fpair, __fmaf_rn(r6inv, __fmaf_rn(P.lj3, r6inv, -P.lj4), -P.offset));
         }
-      }
-    });
-  }
-  finish32(A, i, valid, fi, EV, esum, vsum, 0.0, 0.0);
+      });
+    }
+    float fi[3], esum = 0.0f, vsum[6];
+    S.totals(QUANTUM, fi, esum, vsum);
+    if (valid && threadIdx.x % G == 0) finish32<EV>(A, i, fi, esum, vsum, 0.0, 0.0, red);
+  });
+  if (EV) block_reduce_store<7>(red, A.partial);
 }
 
 // --------------------------------------------------------------------- EAM
 
 // rz: per r-knot m the rhor value coefficients at [2m] and the z2r ones at
 // [2m+1], one 32-byte record; derivatives as in the FP64 kernels.
+//
+// Beside them the smooth part of the same splines as functions of s = r^2,
+// which a pair needs no square root for: the density rho, and the two terms
+// of the force over r, rho'/r and phi'/r, each a cubic in s on intervals of
+// equal width (eam_fast_tables: fitted to the splines to 2e-8 of their local
+// size, a third of an FP32 rounding, or not used).  Their records, 16 bytes
+// per function, cover the intervals [lo, lo + cnt) and are few enough to be
+// held in shared memory `copies` times over, lane l reading copy l % copies:
+// with eight copies a warp's gather has no bank conflict, and L1 keeps the
+// site records.  Pairs beyond the cutoff read a record of zeros, so no branch
+// parts them from the others; pairs inside it but outside the intervals (too
+// close, or within the last knots of the splines) take the splines themselves.
+// The passes are bound by the L1 data pipe (ncu: 80 and 86 % of its peak while
+// active; a gather of 32 site records takes about 13 of its cycles, a 16-byte
+// spline record from global memory as many, from eight copies in shared memory
+// four; with four copies the force pass is 17 % slower).  4.98 M sites: density
+// 1.047 -> 0.73 ms, force 1.170 -> 0.88 ms; 313 k: 91 -> 60 and 96 -> 70 us.
 struct Eam32 {
   const float4 *rz, *frho_val, *frho_der;
-  float rdr, rdrho, rhomax, cutforcesq;
+  float rdr, rdrho, rhomax, cutforcesq;      // cutforcesq in square quanta
   int nr, nrho;
+  const float4 *fast;                        // [3][cnt + 1]: rho, rho'/r, phi'/r
+  float inv_ds;                              // intervals per square quantum
+  int base, cnt, copies;                     // base: bits of 2^23 + the first interval
 };
+
+// The record of s = rsq among the fast ones and the place p in its interval;
+// the last record, T.cnt, holds zeros: any s outside the intervals.
+// floor(rsq * inv_ds) + 2^23 is formed in one rounded operation, exactly.
+__device__ __forceinline__ unsigned fast_interval(const Eam32 &T, float rsq, float &p) {
+  const float x = __fmaf_rd(rsq, T.inv_ds, 8388608.0f);
+  p = __fmaf_rn(rsq, T.inv_ds, 8388608.0f - x);
+  return min((unsigned)(__float_as_int(x) - T.base), (unsigned)T.cnt);
+}
+
+// n functions' records into the block's shared memory, `copies` times.
+__device__ __forceinline__ void load_fast(const Eam32 &T, const float4 *from, int n, float4 *tab) {
+  for (int k = threadIdx.x; k < n * (T.cnt + 1) * T.copies; k += blockDim.x) tab[k] = __ldg(from + k / T.copies);
+  __syncthreads();
+}
+
+__device__ __forceinline__ float cubic(const float4 &c, float p) {
+  return __fmaf_rn(__fmaf_rn(__fmaf_rn(c.x, p, c.y), p, c.z), p, c.w);
+}
 
 __device__ __forceinline__ float fp32_of(const Eam32 &T, float rho, float *phi) {
   float p = rho * T.rdrho + 1.0f;
@@ -320,77 +396,71 @@ __device__ __forceinline__ float fp32_of(const Eam32 &T, float rho, float *phi) 
   return fp;
 }
 
-// A pair's density term (one functor for every walk, so the arithmetic is
-// the same code wherever the neighbour comes from).
-struct RhoPair {
-  const Eam32 &T;
-  float &rho;
-  __device__ __forceinline__ void operator()(float dx, float dy, float dz, float) const {
-    float rsq = dx * dx + dy * dy + dz * dz;
-    if (rsq < T.cutforcesq) {
-      float p = sqrtf(rsq) * T.rdr + 1.0f;
-      int m = (int)p;
-      m = max(1, min(m, T.nr - 1));
-      p -= (float)m;
-      p = fminf(p, 1.0f);
-      float4 c = __ldg(T.rz + 2 * m);
-      rho += ((c.x * p + c.y) * p + c.z) * p + c.w;
-    }
-  }
-};
-
-// One list slot of the density pass: rho at the site, then F' into its
-// record (and F into phi_site for energies).
-__device__ __forceinline__ void rho32_slot(const Args32 &A, const Eam32 &T, int t, double *rho_out,
-                                           double *phi_site, int4 *pos_w) {
-  const int i = site_of_slot(A, t);                       // site-table index
-  int4 oi;
-  site_frame(A, t, oi);
-  float rho = 0.f;
-  for_each32(A, t, i, oi, RhoPair{T, rho});
-  int slot = i;
-  if (i >= A.na) {
-    int e = (i - A.na) / NG, g = (i - A.na) % NG;
-    slot = A.na + 8 * e + gauss_node(g);
-  }
-  rho_out[slot] = rho;
-  float phi = 0.f;
-  float fp = fp32_of(T, rho, A.eflag ? &phi : nullptr);
-  pos_w[t].w = __float_as_int(fp);
-  if (A.eflag) phi_site[i] = phi;
+// The knot of distance r and the place in its interval.
+__device__ __forceinline__ int r_knot(const Eam32 &T, float r, float &p) {
+  p = __fmaf_rn(r, T.rdr, 1.0f);
+  int m = (int)p;
+  m = max(1, min(m, T.nr - 1));
+  p = fminf(__fadd_rn(p, -(float)m), 1.0f);
+  return m;
 }
 
-template <int TB>
-__global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho32(Args32 A, Eam32 T, double *rho_out, double *phi_site,
+// rho'/r and phi'/r from the splines, and phi itself.
+__device__ __forceinline__ void spline_force(const Eam32 &T, float rsq, float &g, float &h, float &phi) {
+  const float s = __fmul_rn(rsq, QUANTUM * QUANTUM);
+  const float recip = rsqrtf(s), r = __fmul_rn(s, recip);
+  float p;
+  const int m = r_knot(T, r, p);
+  float4 rv, zv;
+  ldg256(T.rz + 2 * m, rv, zv);
+  const float rhop = __fmul_rn(__fmaf_rn(__fmaf_rn(3.0f * rv.x, p, 2.0f * rv.y), p, rv.z), T.rdr);
+  const float z2p = __fmul_rn(__fmaf_rn(__fmaf_rn(3.0f * zv.x, p, 2.0f * zv.y), p, zv.z), T.rdr);
+  phi = __fmul_rn(cubic(zv, p), recip);
+  g = __fmul_rn(rhop, recip);
+  h = __fmul_rn(__fmaf_rn(z2p, recip, -__fmul_rn(phi, recip)), recip);
+}
+
+// Density pass: rho at each i-site, then F' into its record (and F into
+// phi_site for energies).
+template <int G, bool FAST>
+__global__ void __launch_bounds__(512, 2) k_eam_rho32(Args32 A, Eam32 T, double *rho_out, double *phi_site,
                                                       int4 *pos_w) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;   // list slot
-  if (t >= A.nsi) return;
-  rho32_slot(A, T, t, rho_out, phi_site, pos_w);
-}
-
-// Persistent work-queue launches for batches: blocks stay resident and take
-// work items one after another from a counter (cleared before the launch);
-// an item is a run of consecutive list slots of one replica (x: first slot,
-// y: count), the largest replicas' items first.  Each slot is computed by
-// the same function as in the grid launch, so results do not change.
-__device__ __forceinline__ int next_item(int *counter) {
-  __shared__ int it;
-  __syncthreads();
-  if (threadIdx.x == 0) it = atomicAdd(counter, 1);
-  __syncthreads();
-  return it;
-}
-
-template <int TB>
-__global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho32_queue(Args32 A, Eam32 T, double *rho_out,
-                                                            double *phi_site, int4 *pos_w, const int2 *items,
-                                                            int nitems, int *counter) {
-  for (;;) {
-    const int k = next_item(counter);
-    if (k >= nitems) return;
-    const int2 w = items[k];
-    for (int t = w.x + threadIdx.x; t < w.x + w.y; t += TB) rho32_slot(A, T, t, rho_out, phi_site, pos_w);
-  }
+  extern __shared__ float4 tab[];
+  if (FAST) load_fast(T, T.fast, 1, tab);
+  const float4 *mine = tab + threadIdx.x % T.copies;
+  for_each_slot<G>(A, [&](int t, bool valid) {
+    const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
+    Sum4<G> sum;
+    if (valid) {
+      const int4 oi = __ldg(A.pos + t);
+      for_each32<G>(A, t, i, oi, [&](int part, float, float, float, float rsq, float) {
+        float p, v = 0.0f;
+        bool spline = rsq < T.cutforcesq;
+        if (FAST) {
+          const unsigned m = fast_interval(T, rsq, p);
+          v = cubic(mine[m * T.copies], p);
+          spline = spline && m == T.cnt;
+        }
+        if (spline) {
+          const int k = r_knot(T, __fsqrt_rn(__fmul_rn(rsq, QUANTUM * QUANTUM)), p);
+          v = cubic(__ldg(T.rz + 2 * k), p);
+        }
+        sum.a[part] = __fadd_rn(sum.a[part], v);
+      });
+    }
+    const float rho = sum.total();
+    if (!valid || threadIdx.x % G) return;
+    int slot = i;
+    if (i >= A.na) {
+      int e = (i - A.na) / NG, g = (i - A.na) % NG;
+      slot = A.na + 8 * e + gauss_node(g);
+    }
+    rho_out[slot] = rho;
+    float phi = 0.f;
+    const float fp = fp32_of(T, rho, A.eflag ? &phi : nullptr);
+    pos_w[t].w = __float_as_int(fp);
+    if (A.eflag) phi_site[i] = phi;
+  });
 }
 
 __global__ void k_eam_site_fp32(int4 *pos, const int *act_gid, const int *nact_dev, int base, int na,
@@ -407,93 +477,52 @@ __global__ void k_eam_site_fp32(int4 *pos, const int *act_gid, const int *nact_d
   }
 }
 
-// A pair's force term (and energy and virial with EV).
-template <bool EV>
-struct ForcePair {
-  const Eam32 &T;
-  float fpi;
-  float *fi;
-  float &esum;
-  float *vsum;
-  __device__ __forceinline__ void operator()(float dx, float dy, float dz, float fpj) const {
-    float rsq = dx * dx + dy * dy + dz * dz;
-    if (rsq < T.cutforcesq) {
-      float recip = rsqrtf(rsq);
-      float r = rsq * recip;
-      float p = r * T.rdr + 1.0f;
-      int m = (int)p;
-      m = max(1, min(m, T.nr - 1));
-      p -= (float)m;
-      p = fminf(p, 1.0f);
-      float4 rv, zv;
-      ldg256(T.rz + 2 * m, rv, zv);
-      float rhop = ((3.0f * rv.x * p + 2.0f * rv.y) * p + rv.z) * T.rdr;
-      float z2p = ((3.0f * zv.x * p + 2.0f * zv.y) * p + zv.z) * T.rdr;
-      float z2 = ((zv.x * p + zv.y) * p + zv.z) * p + zv.w;
-      float phi = z2 * recip;
-      float phip = z2p * recip - phi * recip;
-      float psip = (fpi + fpj) * rhop + phip;
-      float fpair = -psip * recip;
-      fi[0] += dx * fpair;
-      fi[1] += dy * fpair;
-      fi[2] += dz * fpair;
-      if (EV) {
-        esum += phi;
-        vsum[0] += dx * dx * fpair;
-        vsum[1] += dy * dy * fpair;
-        vsum[2] += dz * dz * fpair;
-        vsum[3] += dx * dy * fpair;
-        vsum[4] += dx * dz * fpair;
-        vsum[5] += dy * dz * fpair;
-      }
+// Force pass.  A pair's force is -((F'_i + F'_j) rho'/r + phi'/r) d.
+template <int G, bool FAST, bool EV>
+__global__ void __launch_bounds__(512, EV ? 1 : 2) k_eam_force32(Args32 A, Eam32 T, const double *phi_site) {
+  extern __shared__ float4 tab[];
+  if (FAST) load_fast(T, T.fast + T.cnt + 1, 2, tab);
+  const float4 *mine = tab + threadIdx.x % T.copies;
+  const int second = (T.cnt + 1) * T.copies;
+  double red[7] = {0, 0, 0, 0, 0, 0, 0};
+  for_each_slot<G>(A, [&](int t, bool valid) {
+    const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
+    ForceSums<G, EV> S;
+    if (valid) {
+      const int4 oi = __ldg(A.pos + t);
+      const float fpi = __int_as_float(oi.w);
+      for_each32<G>(A, t, i, oi, [&](int part, float dx, float dy, float dz, float rsq, float fpj) {
+        float p, g = 0.0f, h = 0.0f, phi = 0.0f;
+        const bool inside = rsq < T.cutforcesq;
+        bool spline = inside;
+        if (FAST) {
+          const unsigned m = fast_interval(T, rsq, p);
+          g = cubic(mine[m * T.copies], p);
+          h = cubic(mine[m * T.copies + second], p);
+          spline = inside && m == T.cnt;
+        }
+        if (spline) {
+          spline_force(T, rsq, g, h, phi);
+        } else if (EV && inside) {
+          float g2, h2;
+          spline_force(T, rsq, g2, h2, phi);
+        }
+        const float pull = __fmaf_rn(__fadd_rn(fpi, fpj), g, h);
+        S.add(part, dx, dy, dz, pull);
+        if (EV) S.add_ev(part, dx, dy, dz, pull, phi);
+      });
     }
-  }
-};
-
-// One list slot of the force pass: the pair sums of a valid slot (force;
-// energy and virial with EV) and its embedding energy.
-template <bool EV>
-__device__ __forceinline__ void force32_slot(const Args32 &A, const Eam32 &T, int t, int i,
-                                             const double *phi_site, float fi[3], float &esum, float vsum[6],
-                                             double &eemb_site, double &eemb_global) {
-  int4 oi;
-  site_frame(A, t, oi);
-  const float fpi = __int_as_float(oi.w);
-  for_each32(A, t, i, oi, ForcePair<EV>{T, fpi, fi, esum, vsum});
-  if (EV && A.eflag) {
-    double phi = phi_site[i];
-    eemb_site = phi;
-    eemb_global = (i < A.na) ? phi : phi * A.escale_node * 2.0;
-  }
-}
-
-template <int TB, bool EV>
-__global__ void __launch_bounds__(TB, (EV ? 512 : 1024) / TB) k_eam_force32(Args32 A, Eam32 T,
-                                                                          const double *phi_site) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;   // list slot
-  const bool valid = t < A.nsi;
-  const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
-  float fi[3] = {0, 0, 0}, esum = 0.f, vsum[6] = {0, 0, 0, 0, 0, 0};
-  double eemb_site = 0.0, eemb_global = 0.0;
-  if (valid) force32_slot<EV>(A, T, t, i, phi_site, fi, esum, vsum, eemb_site, eemb_global);
-  finish32(A, i, valid, fi, EV, esum, vsum, eemb_site, eemb_global);
-}
-
-template <int TB>
-__global__ void __launch_bounds__(TB, 1024 / TB) k_eam_force32_queue(Args32 A, Eam32 T, const double *phi_site,
-                                                              const int2 *items, int nitems, int *counter) {
-  for (;;) {
-    const int k = next_item(counter);
-    if (k >= nitems) return;
-    const int2 w = items[k];
-    for (int t = w.x + threadIdx.x; t < w.x + w.y; t += TB) {
-      const int i = site_of_slot(A, t);
-      float fi[3] = {0, 0, 0}, esum = 0.f, vsum[6] = {0, 0, 0, 0, 0, 0};
-      double eemb_site = 0.0, eemb_global = 0.0;
-      force32_slot<false>(A, T, t, i, phi_site, fi, esum, vsum, eemb_site, eemb_global);
-      finish32(A, i, true, fi, false, esum, vsum, eemb_site, eemb_global);
+    float fi[3], esum = 0.0f, vsum[6];
+    S.totals(-QUANTUM, fi, esum, vsum);
+    if (!valid || threadIdx.x % G) return;
+    double eemb_site = 0.0, eemb_global = 0.0;
+    if (EV && A.eflag) {
+      eemb_site = phi_site[i];
+      eemb_global = i < A.na ? eemb_site : eemb_site * A.escale_node * 2.0;
     }
-  }
+    finish32<EV>(A, i, fi, esum, vsum, eemb_site, eemb_global, red);
+  });
+  if (EV) block_reduce_store<7>(red, A.partial);
 }
 
 __global__ void k_reduce_partials32(const double *partial, int nblocks, double *out) {
@@ -511,7 +540,6 @@ FixGrid make_fix_grid(const Ctx &c) {
   for (int d = 0; d < 3; d++) {
     G.lo[d] = r0.b.lo[d];
     G.scale[d] = r0.qscale[d];
-    G.inv[d] = r0.qinv[d];
     G.Lq[d] = r0.Lq[d];
   }
   G.reps = c.nrep > 1 ? c.rep_d.p : nullptr;
@@ -522,6 +550,132 @@ FixGrid make_fix_grid(const Ctx &c) {
   G.na = c.na;
   G.nsi = c.nsite_i();
   return G;
+}
+
+// The splines as the host evaluates them: value and derivative at r.
+struct HostSpline {
+  const std::vector<double4> &rz;
+  int which, nr;
+  double rdr;
+  void at(double r, double &v, double &d) const {
+    double p = r * rdr + 1.0;
+    const int m = std::max(1, std::min((int)p, nr - 1));
+    p = std::min(p - m, 1.0);
+    const double4 c = rz[2 * (size_t)m + which];
+    v = ((c.x * p + c.y) * p + c.z) * p + c.w;
+    d = ((3.0 * c.x * p + 2.0 * c.y) * p + c.z) * rdr;
+  }
+};
+
+// i-sites from which a site takes one lane, and two: below, one lane per site
+// leaves too few warps to hide the gathers' latency; above, more lanes per
+// site read more list rows per load.  Density pass in us with 1 / 2 / 4 lanes
+// (measured before the fast records, which shifted all alike): 6 k sites
+// 29 / 19 / 15, 84 k 33 / 33 / 31, 313 k 91 / 83 / 88, 1.21 M 268 / 275 / 311.
+constexpr int ONE_LANE_SITES = 600000, TWO_LANE_SITES = 100000;
+
+// The three functions of s = r^2 that the passes need, as cubics on n equal
+// intervals of [0, top^2], each the interpolant at the interval's four
+// Chebyshev nodes.  An interval is good when every function's cubic stays
+// within 2e-8 of the spline, relative to its largest value within 0.5 A.
+// Returns the first interval from which all are good (n: none).
+int fit_fast(const HostSpline &rho, const HostSpline &z, double top, int n, float &inv_ds, std::vector<float4> rec[3]) {
+  // pairs at the top or beyond fall past the last interval
+  inv_ds = (float)((double)n / (double)(float)(top * top));
+  while ((double)inv_ds * (double)(float)(top * top) < n) inv_ds = std::nextafter(inv_ds, 1e30f);
+  const double ds = 1.0 / (double)inv_ds;
+  auto eval = [&](double s, double out[3]) {
+    const double r = std::sqrt(s);
+    double dr, zv, dz;
+    rho.at(r, out[0], dr);
+    z.at(r, zv, dz);
+    out[1] = dr / r;
+    out[2] = (dz - zv / r) / s;
+  };
+  double node[4], inv[4][4];
+  for (int k = 0; k < 4; k++) node[k] = 0.5 - 0.5 * std::cos((2 * k + 1) * 3.14159265358979323846 / 8.0);
+  // Lagrange basis polynomials' coefficients
+  for (int k = 0; k < 4; k++) {
+    double c[4] = {1, 0, 0, 0};
+    int deg = 0;
+    for (int j = 0; j < 4; j++) {
+      if (j == k) continue;
+      const double q = 1.0 / (node[k] - node[j]);
+      double e[4] = {0, 0, 0, 0};
+      for (int d = 0; d <= deg; d++) {
+        e[d + 1] += c[d] * q;
+        e[d] -= c[d] * node[j] * q;
+      }
+      deg++;
+      std::copy(e, e + 4, c);
+    }
+    std::copy(c, c + 4, inv[k]);
+  }
+  constexpr int TEST = 12;
+  std::vector<double> err[3], val[3], mid(n);
+  for (int q = 0; q < 3; q++) {
+    rec[q].resize(n);
+    err[q].assign(n, 0.0);
+    val[q].assign(n, 0.0);
+  }
+  for (int m = 0; m < n; m++) {
+    mid[m] = std::sqrt((m + 0.5) * ds);
+    double c[3][4] = {};
+    for (int k = 0; k < 4; k++) {
+      double v[3];
+      eval((m + node[k]) * ds, v);
+      for (int q = 0; q < 3; q++)
+        for (int d = 0; d < 4; d++) c[q][d] += v[q] * inv[k][d];
+    }
+    for (int u = 0; u <= TEST; u++) {
+      const double p = (double)u / TEST;
+      double v[3];
+      eval(std::max((m + p) * ds, 1e-6 * ds), v);
+      for (int q = 0; q < 3; q++) {
+        const double a = ((c[q][3] * p + c[q][2]) * p + c[q][1]) * p + c[q][0];
+        err[q][m] = std::max(err[q][m], std::fabs(a - v[q]));
+        val[q][m] = std::max(val[q][m], std::fabs(v[q]));
+      }
+    }
+    for (int q = 0; q < 3; q++)
+      rec[q][m] = make_float4((float)c[q][3], (float)c[q][2], (float)c[q][1], (float)c[q][0]);
+  }
+  for (int m = n - 1; m >= 0; m--)
+    for (int q = 0; q < 3; q++) {
+      double size = 0.0;
+      for (int j = m; j >= 0 && mid[m] - mid[j] <= 0.5; j--) size = std::max(size, val[q][j]);
+      for (int j = m; j < n && mid[j] - mid[m] <= 0.5; j++) size = std::max(size, val[q][j]);
+      if (!(err[q][m] <= 2e-8 * size)) return m + 1;
+    }
+  return 0;
+}
+
+// Fast records of the context's splines: the fewest intervals that are good
+// from 0.4 of the cutoff on (closer pairs are rare), up to the cutoff or, as
+// the splines' slopes at the last knots are cruder, up to four knots before
+// it.  Tables that no fit follows (noisy ones) have none.
+void eam_fast_tables(Ctx &c, const std::vector<double4> &rz) {
+  c.fast_cnt = 0;
+  const HostSpline rho{rz, 0, c.pp.nr, c.pp.rdr}, z{rz, 1, c.pp.nr, c.pp.rdr};
+  std::vector<float4> rec[3];
+  for (int n : {192, 256, 384, 512})
+    for (double top : {c.pp.cut, c.pp.cut - 4.0 * c.pp.dr}) {
+      if (!(top > 0.5 * c.pp.cut)) continue;
+      float inv_ds;
+      const int lo = fit_fast(rho, z, top, n, inv_ds, rec);
+      if (!(std::sqrt(lo / (double)inv_ds) <= 0.4 * c.pp.cut)) continue;
+      c.fast_lo = lo;
+      c.fast_cnt = n - lo;
+      c.fast_inv_ds = inv_ds;
+      std::vector<float4> out;
+      for (int q = 0; q < 3; q++) {
+        out.insert(out.end(), rec[q].begin() + lo, rec[q].end());
+        out.push_back(make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+      }
+      c.fast32.reserve(out.size());
+      stream_copy(c, c.fast32.p, out.data(), sizeof(float4) * out.size(), cudaMemcpyHostToDevice);
+      return;
+    }
 }
 
 }  // namespace
@@ -546,63 +700,16 @@ void mixed_tables(Ctx &c) {
     for (int m = 0; m <= n; m++) g[m] = make_float4((float)h[m].x, (float)h[m].y, (float)h[m].z, (float)h[m].w);
     dst.reserve(n + 1);
     stream_copy(c, dst.p, g.data(), sizeof(float4) * (n + 1), cudaMemcpyHostToDevice);
+    return h;
   };
-  conv(c.rz, c.rz32, 2 * c.pp.nr + 1);
+  eam_fast_tables(c, conv(c.rz, c.rz32, 2 * c.pp.nr + 1));
   conv(c.frho_val, c.frho_val32, c.pp.nrho);
   conv(c.frho_der, c.frho_der32, c.pp.nrho);
 }
 
-namespace {
-
-// size class of a replica by its i-sites
-int size_class(long sites) { return sites < 8192 ? 0 : sites < 32768 ? 1 : 2; }
-
-// Work items of a batch: replicas by i-sites, largest first; each replica's
-// atom slots, then its Gauss-point slots, in runs of its class's tile.
-// only_class >= 0 keeps the items of that class alone (tuning).
-std::vector<int2> make_items(const Ctx &c, const int tile[3], int only_class) {
-  std::vector<int> order(c.nrep);
-  for (int r = 0; r < c.nrep; r++) order[r] = r;
-  auto sites = [&](int r) { return (long)c.rep_na[r] + 8L * c.rep_ne[r]; };
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sites(a) > sites(b); });
-  std::vector<int2> items;
-  for (int r : order) {
-    const int cl = size_class(sites(r));
-    if (only_class >= 0 && cl != only_class) continue;
-    const int T = tile[cl];
-    const int a0 = c.rep_aoff[r], na = c.rep_na[r];
-    for (int o = 0; o < na; o += T) items.push_back(make_int2(a0 + o, std::min(T, na - o)));
-    const int g0 = c.na + 8 * c.rep_eoff[r], ng = 8 * c.rep_ne[r];
-    for (int o = 0; o < ng; o += T) items.push_back(make_int2(g0 + o, std::min(T, ng - o)));
-  }
-  return items;
-}
-
-int queue_grid(const Ctx &c) {
-  static const int per_sm = [] {
-    int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_eam_force32_queue<128>, 128, 0);
-    return b > 0 ? b : 1;
-  }();
-  return per_sm * c.num_sms;
-}
-
-void upload_items(Ctx &c, const std::vector<int2> &items) {
-  c.work_items.reserve(std::max<size_t>(items.size(), 1));
-  if (!items.empty())
-    stream_copy(c, c.work_items.p, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice);
-  c.nwork_items = (int)items.size();
-}
-
-}  // namespace
-
 void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
   const int nsi = c.nsite_i();
-  const long ns = (long)nsi + (long)c.ne * NU;   // capacity: every lattice site active
-  const int T = 128;
-  const int nb = std::max(nblk(nsi, T), 1);
   FixGrid G = make_fix_grid(c);
-  (void)ns;   // the fixed-point records were written by pair_table_mixed
   Args32 A;
   A.pos = c.pos32.p;
   A.nbr = c.nbr_full.p;
@@ -629,7 +736,7 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
   A.enode = c.enode.p;
   A.vatom = c.vatom.p;
   A.vnode = c.vnode.p;
-  c.partial.reserve((size_t)nb * 7);
+  c.partial.reserve((size_t)c.num_sms * 8 * 7);
   c.ev_out.reserve(7);
   A.partial = c.partial.p;
   A.eflag = eflag;
@@ -639,13 +746,27 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
   A.escale_node = nodal_weight / 2.0;
   if (c.pp.style == CACB200_PAIR_EAM && c.nodal_energy_weight >= 0.0) A.escale_node = c.nodal_energy_weight / 2.0;
   c.escale_node_last = A.escale_node;
-  bool ev = eflag || vflag;
+  const bool ev = eflag || vflag;
+  // lanes per site by the size (results do not depend on it)
+  const int lanes = nsi >= ONE_LANE_SITES ? 1 : nsi >= TWO_LANE_SITES ? 2 : 4;
+  auto by_lanes = [&](auto &&launch) {
+    if (lanes == 1) launch(std::integral_constant<int, 1>());
+    else if (lanes == 2) launch(std::integral_constant<int, 2>());
+    else launch(std::integral_constant<int, 4>());
+  };
+  int grid_ev = 1;
   if (c.pp.style == CACB200_PAIR_LJ) {
-    Lj32 P{(float)(c.pp.cut * c.pp.cut), (float)c.pp.lj1, (float)c.pp.lj2, (float)c.pp.lj3, (float)c.pp.lj4,
+    const double q2 = std::ldexp(1.0, 52);
+    Lj32 P{(float)(c.pp.cut * c.pp.cut * q2), (float)c.pp.lj1, (float)c.pp.lj2, (float)c.pp.lj3, (float)c.pp.lj4,
            (float)c.pp.offset};
     KernelTimer t(c, "pair_lj32");
-    if (ev) k_lj32<true><<<nb, T, 0, c.stream>>>(A, P);
-    else k_lj32<false><<<nb, T, 0, c.stream>>>(A, P);
+    const int need = std::max(nblk((long)nsi * lanes, 128), 1);
+    grid_ev = std::min(need, c.num_sms * 8);
+    by_lanes([&](auto g) {
+      constexpr int GL = decltype(g)::value;
+      if (ev) k_lj32<GL, true><<<grid_ev, 128, 0, c.stream>>>(A, P);
+      else k_lj32<GL, false><<<need, 128, 0, c.stream>>>(A, P);
+    });
   } else {
     if (!c.have_mixed_tables) {
       mixed_tables(c);
@@ -658,135 +779,60 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
     Tb.rdr = (float)c.pp.rdr;
     Tb.rdrho = (float)c.pp.rdrho;
     Tb.rhomax = (float)c.pp.rhomax;
-    Tb.cutforcesq = (float)(c.pp.cut * c.pp.cut);
+    Tb.cutforcesq = (float)(c.pp.cut * c.pp.cut * std::ldexp(1.0, 52));
     Tb.nr = c.pp.nr;
     Tb.nrho = c.pp.nrho;
+    Tb.fast = c.fast32.p;
+    Tb.inv_ds = std::ldexp(c.fast_inv_ds, -52);
+    Tb.base = 0x4b000000 + c.fast_lo;
+    Tb.cnt = c.fast_cnt;
     c.rho.reserve(std::max(c.na + 8 * c.ne, 1));
     c.phi_site.reserve(std::max(nsi, 1));
-    auto rho = [&](int tb) {
-      if (tb == 64) k_eam_rho32<64><<<std::max(nblk(nsi, 64), 1), 64, 0, c.stream>>>(A, Tb, c.rho.p, c.phi_site.p, c.pos32.p);
-      else if (tb == 256) k_eam_rho32<256><<<std::max(nblk(nsi, 256), 1), 256, 0, c.stream>>>(A, Tb, c.rho.p, c.phi_site.p, c.pos32.p);
-      else k_eam_rho32<128><<<nb, 128, 0, c.stream>>>(A, Tb, c.rho.p, c.phi_site.p, c.pos32.p);
+    // resident blocks stride over the list slots, so the records are loaded
+    // once per block; small systems take small blocks and one copy
+    const long threads = (long)nsi * lanes;
+    const bool small = threads < (long)c.num_sms * 512;
+    const int tb = small ? 128 : 512;
+    Tb.copies = small ? 1 : 8;
+    const int need = std::max(nblk(threads, tb), 1);
+    const int grid = c.work_queue && !small ? std::min(need, 2 * c.num_sms) : need;
+    grid_ev = std::min(need, small ? c.num_sms * 8 : c.num_sms);
+    c.tb_rho32 = c.tb_force32 = tb;
+    if (c.nrep > 1 && c.work_queue)
+      for (int &k : c.work_tile) k = 512;
+    const bool fast = c.fast_cnt > 0;
+    const size_t rec = fast ? sizeof(float4) * (size_t)(c.fast_cnt + 1) * Tb.copies : 0;
+    auto go = [&](auto kernel, int blocks, size_t bytes, auto... args) {
+      if (bytes > 48 * 1024)
+        CACB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+      kernel<<<blocks, tb, bytes, c.stream>>>(A, Tb, args...);
     };
-    auto site_fp = [&] {
-      if (c.ne)
-        k_eam_site_fp32<<<stride_grid((long)c.ne * NU, 256), 256, 0, c.stream>>>(
-            c.pos32.p, c.act_gid.p, c.dev_nact.p, c.na + NG * c.ne, c.na, c.rho.p, Tb);
-    };
-    auto force = [&](int tb) {
-      if (tb == 64) k_eam_force32<64, false><<<std::max(nblk(nsi, 64), 1), 64, 0, c.stream>>>(A, Tb, c.phi_site.p);
-      else if (tb == 256) k_eam_force32<256, false><<<std::max(nblk(nsi, 256), 1), 256, 0, c.stream>>>(A, Tb, c.phi_site.p);
-      else k_eam_force32<128, false><<<nb, 128, 0, c.stream>>>(A, Tb, c.phi_site.p);
-    };
-    // batches: the persistent work-queue launches, their tiles tuned per
-    // replica size class when the plan changes (idempotent trial launches)
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CACB200_CUDA(cudaStreamIsCapturing(c.stream, &cs));
-    bool queue = c.nrep > 1 && c.work_queue;
-    c.work_counter.reserve(2);
-    auto rho_q = [&] {
-      CACB200_CUDA(cudaMemsetAsync(c.work_counter.p, 0, sizeof(int), c.stream));
-      k_eam_rho32_queue<128><<<queue_grid(c), 128, 0, c.stream>>>(A, Tb, c.rho.p, c.phi_site.p, c.pos32.p,
-                                                                 c.work_items.p, c.nwork_items, c.work_counter.p);
-    };
-    auto force_q = [&] {
-      CACB200_CUDA(cudaMemsetAsync(c.work_counter.p + 1, 0, sizeof(int), c.stream));
-      k_eam_force32_queue<128><<<queue_grid(c), 128, 0, c.stream>>>(A, Tb, c.phi_site.p, c.work_items.p,
-                                                                   c.nwork_items, c.work_counter.p + 1);
-    };
-    if (queue && c.work_gen != c.gen && cs == cudaStreamCaptureStatusNone) {
-      const int cand[3] = {512, 128, 2048};   // another tile replaces 512 only when >= 3 % faster
-      int tile[3] = {512, 512, 512};
-      {
-        // phase: densities and F' first, so the trial force passes read the step's F'
-        upload_items(c, make_items(c, tile, -1));
-        rho_q();
-        site_fp();
-        cudaEvent_t e0, e1;
-        CACB200_CUDA(cudaEventCreate(&e0));
-        CACB200_CUDA(cudaEventCreate(&e1));
-        for (int cl = 0; cl < 3; cl++) {
-          float best = 1e30f;
-          for (int T : cand) {
-            int trial[3] = {T, T, T};
-            upload_items(c, make_items(c, trial, cl));
-            if (c.nwork_items == 0) break;
-            float ms = 1e30f;
-            for (int rep = 0; rep < 3; rep++) {
-              CACB200_CUDA(cudaEventRecord(e0, c.stream));
-              force_q();
-              CACB200_CUDA(cudaEventRecord(e1, c.stream));
-              CACB200_CUDA(cudaEventSynchronize(e1));
-              float m = 0.f;
-              CACB200_CUDA(cudaEventElapsedTime(&m, e0, e1));
-              ms = std::min(ms, m);
-            }
-            if (T == 512 || ms < 0.97f * best) best = ms, tile[cl] = T;
-          }
-        }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-      }
-      for (int cl = 0; cl < 3; cl++) c.work_tile[cl] = tile[cl];
-      upload_items(c, make_items(c, tile, -1));
-      c.work_gen = c.gen;
-    }
-    // items are made outside stream capture; until then the grid launches
-    if (queue && c.work_gen != c.gen) queue = false;
-    // block sizes of the force-only passes chosen by timing on first use (as
-    // in the FP64 form; results do not depend on them)
-    if (!queue && c.tune_gen32 != c.gen && !ev && cs == cudaStreamCaptureStatusNone) {
-      const int cand[3] = {128, 64, 256};   // another size replaces 128 only when >= 3 % faster
-      cudaEvent_t e0, e1;
-      CACB200_CUDA(cudaEventCreate(&e0));
-      CACB200_CUDA(cudaEventCreate(&e1));
-      auto timed = [&](auto &&launch) {
-        float best = 1e30f;
-        for (int rep = 0; rep < 3; rep++) {
-          CACB200_CUDA(cudaEventRecord(e0, c.stream));
-          launch();
-          CACB200_CUDA(cudaEventRecord(e1, c.stream));
-          CACB200_CUDA(cudaEventSynchronize(e1));
-          float ms = 0.f;
-          CACB200_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-          best = std::min(best, ms);
-        }
-        return best;
-      };
-      float best = 1e30f;
-      for (int tb : cand) {
-        float ms = timed([&] { rho(tb); });
-        if (tb == 128 || ms < 0.97f * best) best = ms, c.tb_rho32 = tb;
-      }
-      rho(c.tb_rho32);
-      site_fp();
-      best = 1e30f;
-      for (int tb : cand) {
-        float ms = timed([&] { force(tb); });
-        if (tb == 128 || ms < 0.97f * best) best = ms, c.tb_force32 = tb;
-      }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      c.tune_gen32 = c.gen;
-    }
     {
       KernelTimer t(c, "eam_rho32");
-      if (queue) rho_q();
-      else rho(c.tb_rho32);
+      by_lanes([&](auto g) {
+        constexpr int GL = decltype(g)::value;
+        if (fast) go(k_eam_rho32<GL, true>, grid, rec, c.rho.p, c.phi_site.p, c.pos32.p);
+        else go(k_eam_rho32<GL, false>, grid, 0, c.rho.p, c.phi_site.p, c.pos32.p);
+      });
     }
     if (c.ne) {
       KernelTimer t(c, "eam_site_fp32");
-      site_fp();
+      k_eam_site_fp32<<<stride_grid((long)c.ne * NU, 256), 256, 0, c.stream>>>(
+          c.pos32.p, c.act_gid.p, c.dev_nact.p, c.na + NG * c.ne, c.na, c.rho.p, Tb);
     }
     {
       KernelTimer t(c, "eam_force32");
-      if (ev) k_eam_force32<128, true><<<nb, T, 0, c.stream>>>(A, Tb, c.phi_site.p);
-      else if (queue) force_q();
-      else force(c.tb_force32);
+      by_lanes([&](auto g) {
+        constexpr int GL = decltype(g)::value;
+        if (ev && fast) go(k_eam_force32<GL, true, true>, grid_ev, 2 * rec, c.phi_site.p);
+        else if (ev) go(k_eam_force32<GL, false, true>, grid_ev, 0, c.phi_site.p);
+        else if (fast) go(k_eam_force32<GL, true, false>, grid, 2 * rec, c.phi_site.p);
+        else go(k_eam_force32<GL, false, false>, grid, 0, c.phi_site.p);
+      });
     }
   }
   if (ev) {
-    k_reduce_partials32<<<1, 256, 0, c.stream>>>(c.partial.p, nb, c.ev_out.p);
+    k_reduce_partials32<<<1, 256, 0, c.stream>>>(c.partial.p, grid_ev, c.ev_out.p);
     c.have_peratom_e = (eflag & CACB200_ENERGY_ATOM) != 0;
     c.have_peratom_v = (vflag & CACB200_VIRIAL_ATOM) != 0;
     c.ev_pending = true;
