@@ -100,15 +100,45 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Pair passes: G neighbouring lanes share an i-site.  Lane g of the group
-// walks list rows g, g + G, ...; the lanes' sums are added in a fixed tree
-// (the same for every launch form and system size, so a site's result depends
-// on its list alone).
-template <int G, class T>
-__device__ __forceinline__ T lanes_sum(T v) {
+// Pair passes.  A site's sums are kept in four partial sums: entry k of a
+// walk goes to partial k mod 4, and the partials are added as (0 + 1) + (2 +
+// 3).  G lanes share a site (G = 1, 2 or 4; lane g walks entries g, g + G,
+// ...) and each holds 4 / G of the partials, so a site's result is the same
+// bit for bit whatever G is: large systems take few lanes per site, small
+// ones, which would leave the chip idle, more.
+template <class T, int G>
+struct Sum4 {
+  T a[4 / G];
+  __device__ __forceinline__ Sum4() {
 #pragma unroll
-  for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+    for (int k = 0; k < 4 / G; k++) a[k] = T(0);
+  }
+  // the site's sum, in every lane of its group (every lane of the warp calls it)
+  __device__ __forceinline__ T total() const {
+    T t[4 / G];
+#pragma unroll
+    for (int k = 0; k < 4 / G; k++) {
+      t[k] = a[k];
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+    }
+    if constexpr (G == 1) return (t[0] + t[1]) + (t[2] + t[3]);
+    else if constexpr (G == 2) return t[0] + t[1];
+    else return t[0];
+  }
+};
+
+// The pair passes' threads: runs of 32 / G consecutive list slots, one per
+// warp, consecutive warps taking consecutive runs, grid-stride.  body(slot,
+// valid) is called by whole warps.
+template <int G, class F>
+__device__ __forceinline__ void for_each_slot(int nsi, F &&body) {
+  constexpr int S = 32 / G;
+  const int warps = blockDim.x >> 5, nrun = (nsi + S - 1) / S;
+  for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < nrun; r += gridDim.x * warps) {
+    const int t = r * S + (threadIdx.x & 31) / G;
+    body(t, t < nsi);
+  }
 }
 
 // Deterministic block reduction of NV doubles into out[blockIdx.x * NV + k].

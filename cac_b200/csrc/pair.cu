@@ -18,6 +18,7 @@
 // one 32-byte load brings a neighbour's position and F'.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "ctx.cuh"
@@ -50,113 +51,103 @@ struct PairArgs {
 
 __device__ __forceinline__ int site_of_slot(const PairArgs &A, int t) { return t < A.na ? A.slot_atom[t] : t; }
 
-// The FP64 EAM arithmetic in explicitly rounded operations, with no fused
-// multiply-add: the operation order of the reference's source (compiled
-// there without contraction), and the same rounding in every kernel that
-// inlines it (grid and SM-local launches, grouped and remainder walks), where
-// the compiler would otherwise contract each copy its own way.
+// The FP64 pair arithmetic in explicitly rounded and explicitly fused
+// operations: every kernel that inlines it (grid and SM-local launches, with
+// and without tallies) rounds alike, where the compiler would contract each
+// copy its own way.
 __device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
 
-__device__ __forceinline__ void neighbour_pos(const PairArgs &A, double Lx, double Ly, double Lz, int v,
-                                              double4 &xj) {
-  int j = v >> IMG_BITS, code = v & ((1 << IMG_BITS) - 1);
-  xj = ldg256(A.xs + j);
-  if (code != IMG_ZERO) {
-    int sx, sy, sz;
-    img_decode(code, sx, sy, sz);
-    xj.x = radd(xj.x, rmul((double)sx, Lx));
-    xj.y = radd(xj.y, rmul((double)sy, Ly));
-    xj.z = radd(xj.z, rmul((double)sz, Lz));
-  }
-}
-
-// Walks a site's list four entries at a time: the four entry loads, then the
-// four position loads, are issued back to back before any of them is used, so
-// each thread keeps eight independent loads in flight instead of a chain of
-// dependent pairs.  List entries are read once per pass: they are loaded as
-// streaming (evict-first) so that L1 keeps the neighbour positions and spline
-// records, which are reused.  MANY: the site belongs to a batch replica with
-// its own box.
-template <bool MANY, class F>
-__device__ __forceinline__ void for_each_neighbour(const PairArgs &A, int i, const int *nb, int n, F &&f) {
-  double Lx = A.L[0], Ly = A.L[1], Lz = A.L[2];
-  if (MANY) {
-    const Rep *r = A.reps + A.site_rep[i];
-    Lx = r->b.L[0];
-    Ly = r->b.L[1];
-    Lz = r->b.L[2];
-  }
-  int k = 0;
-  for (; k + 4 <= n; k += 4) {
-    int v0 = __ldcs(nb + (size_t)k * A.nsi), v1 = __ldcs(nb + (size_t)(k + 1) * A.nsi);
-    int v2 = __ldcs(nb + (size_t)(k + 2) * A.nsi), v3 = __ldcs(nb + (size_t)(k + 3) * A.nsi);
-    double4 p0, p1, p2, p3;
-    neighbour_pos(A, Lx, Ly, Lz, v0, p0);
-    neighbour_pos(A, Lx, Ly, Lz, v1, p1);
-    neighbour_pos(A, Lx, Ly, Lz, v2, p2);
-    neighbour_pos(A, Lx, Ly, Lz, v3, p3);
-    f(p0);
-    f(p1);
-    f(p2);
-    f(p3);
-  }
-  for (; k < n; k++) {
-    double4 p;
-    neighbour_pos(A, Lx, Ly, Lz, __ldcs(nb + (size_t)k * A.nsi), p);
-    f(p);
+// Walks n entries of a list: each lane takes four at a time, the next four
+// entries loaded ahead and the four records issued back to back before any is
+// used.  Entries past the end are walked as pairs too far apart to count.
+// List entries are read once per pass: they are loaded as streaming
+// (evict-first) so that L1 keeps the neighbour positions and spline records,
+// which are reused.  f(partial, record, apart): the neighbour's record under
+// its image; apart: past the end.
+template <int G, class F>
+__device__ __forceinline__ void walk(const PairArgs &A, int t, int i, const int *nb, int n, F &&f) {
+  const size_t step = (size_t)G * A.nsi;
+  const int *p = nb + (size_t)(threadIdx.x % G) * A.nsi;
+  int v[4];
+  auto load = [&](int left) {   // entries this lane still has
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = u < left ? __ldcs(p + u * step) : (t << IMG_BITS) | IMG_ZERO;
+    p += 4 * step;
+  };
+  int left = (n - (int)(threadIdx.x % G) + G - 1) / G;
+  load(left);
+  for (; left > 0; left -= 4) {
+    double4 o[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) o[u] = ldg256(A.xs + (v[u] >> IMG_BITS));
+    if (((v[0] ^ IMG_ZERO) | (v[1] ^ IMG_ZERO) | (v[2] ^ IMG_ZERO) | (v[3] ^ IMG_ZERO)) & ((1 << IMG_BITS) - 1)) {
+      // images: an entry's image (0, 0, 0) leaves its position as it is
+      const double *L = A.site_rep ? A.reps[A.site_rep[i]].b.L : A.L;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        int sx, sy, sz;
+        img_decode(v[u] & ((1 << IMG_BITS) - 1), sx, sy, sz);
+        if (sx) o[u].x = radd(o[u].x, rmul((double)sx, L[0]));
+        if (sy) o[u].y = radd(o[u].y, rmul((double)sy, L[1]));
+        if (sz) o[u].z = radd(o[u].z, rmul((double)sz, L[2]));
+      }
+    }
+    const int now = left;
+    load(left - 4);
+#pragma unroll
+    for (int u = 0; u < 4; u++) f(u % (4 / G), o[u], u && u >= now);
   }
 }
 
 // A site's list in two walks: the inner prefix (entries within the cutoff
 // plus a margin at the build, the list's first rows), then, unless the
 // site's displacement since the build and the largest one cannot close the
-// margin (walk_rest, device.cuh), the rest (the list's last rows).  Each entry's arithmetic depends on its place in the walk (the
-// compiler may fuse multiply-adds differently in the grouped and the
-// remainder loop), so the prefix is always walked on its own: the sums are
-// the same whether the rest is walked or not.
-// The rule's flag and largest displacement belong to the site's replica (one
-// hot replica of a batch does not end the shortcut for the others); one copy
-// of the walk serves both segments, which keeps the register count of the
-// unrolled body.
-template <bool MANY, class F>
-__device__ __forceinline__ void walk_list(const PairArgs &A, int i, const int *nb, int n_in, int n, F &&f) {
-  const bool rest = n > n_in && walk_rest(A.prefix, i, MANY ? A.site_rep[i] : 0);
+// margin (walk_rest, device.cuh), the rest (the list's last rows).  An entry's
+// partial sum depends on its place in the walk, so the prefix is always walked
+// on its own: the sums are the same whether the rest is walked or not.  The
+// rule's flag and largest displacement belong to the site's replica (one hot
+// replica of a batch does not end the shortcut for the others); one copy of
+// the walk serves both segments.
+template <int G, class F>
+__device__ __forceinline__ void walk_list(const PairArgs &A, int t, int i, F &&f) {
+  const int n_in = A.num_in[t], n = A.num[t];
+  const int *nb = A.nbr + t;
+  const bool rest = n > n_in && walk_rest(A.prefix, i, A.site_rep ? A.site_rep[i] : 0);
 #pragma unroll 1
   for (int seg = 0; seg < (rest ? 2 : 1); seg++)
-    for_each_neighbour<MANY>(A, i, seg ? nb + (size_t)(A.cap - (n - n_in)) * A.nsi : nb, seg ? n - n_in : n_in,
-                             f);
+    walk<G>(A, t, i, seg ? nb + (size_t)(A.cap - (n - n_in)) * A.nsi : nb, seg ? n - n_in : n_in, f);
 }
 
-// Writes force and per-site energy/virial of i-site i and accumulates the
-// global sums (reduced per block in fixed order).
-__device__ __forceinline__ void finish_site(const PairArgs &A, int i, bool valid, const double fi[3],
-                                            double esum, const double vsum[6], double eextra_site,
-                                            double eextra_global) {
-  double red[7] = {0, 0, 0, 0, 0, 0, 0};
-  if (valid) {
-    bool atom = i < A.na;
-    int e = 0, g = 0, node = 0;
-    double *fo;
-    if (atom) {
-      fo = A.f + 3 * (size_t)i;
-    } else {
-      e = (i - A.na) / NG;
-      g = (i - A.na) % NG;
-      node = gauss_node(g);
-      fo = A.gaussf + (size_t)e * 24 + 3 * g;
-    }
-    fo[0] = fi[0];
-    fo[1] = fi[1];
-    fo[2] = fi[2];
-    double es = atom ? 0.5 : A.escale_node, vs = atom ? 0.5 : A.vscale_node;
-    if (A.eflag & CACB200_ENERGY_GLOBAL) red[0] = es * esum + eextra_global;
+// Writes force (and per-site energy / virial) of i-site i and adds its global
+// energy / virial to red.
+template <bool EV>
+__device__ __forceinline__ void finish_site(const PairArgs &A, int i, const double fi[3], double esum,
+                                            const double vsum[6], double eextra_site, double eextra_global,
+                                            double red[7]) {
+  const bool atom = i < A.na;
+  int e = 0, g = 0, node = 0;
+  double *fo;
+  if (atom) {
+    fo = A.f + 3 * (size_t)i;
+  } else {
+    e = (i - A.na) / NG;
+    g = (i - A.na) % NG;
+    node = gauss_node(g);
+    fo = A.gaussf + (size_t)e * 24 + 3 * g;
+  }
+  fo[0] = fi[0];
+  fo[1] = fi[1];
+  fo[2] = fi[2];
+  if (EV) {
+    const double es = atom ? 0.5 : A.escale_node, vs = atom ? 0.5 : A.vscale_node;
+    if (A.eflag & CACB200_ENERGY_GLOBAL) red[0] += es * esum + eextra_global;
     if (A.vflag & CACB200_VIRIAL_GLOBAL)
 #pragma unroll
-      for (int k = 0; k < 6; k++) red[1 + k] = vs * vsum[k];
+      for (int k = 0; k < 6; k++) red[1 + k] += vs * vsum[k];
     if (A.eflag & CACB200_ENERGY_ATOM) {
-      double ev = 0.5 * esum + eextra_site;
+      const double ev = 0.5 * esum + eextra_site;
       if (atom) A.eatom[i] = ev;
       else A.enode[(size_t)e * 8 + node] = ev;
     }
@@ -166,23 +157,39 @@ __device__ __forceinline__ void finish_site(const PairArgs &A, int i, bool valid
       for (int k = 0; k < 6; k++) vo[k] = 0.5 * vsum[k];
     }
   }
-  if (A.eflag || A.vflag) block_reduce_store<7>(red, A.partial);
 }
 
-// Force only (no energy or virial requested): one write per site.
-__device__ __forceinline__ void finish_force(const PairArgs &A, int i, bool valid, const double fi[3]) {
-  if (!valid) return;
-  double *fo;
-  if (i < A.na) {
-    fo = A.f + 3 * (size_t)i;
-  } else {
-    int e = (i - A.na) / NG, g = (i - A.na) % NG;
-    fo = A.gaussf + (size_t)e * 24 + 3 * g;
+// Per-site sums of a force pass; fpair and the separation as in the pair terms.
+template <int G, bool EV>
+struct ForceSums {
+  Sum4<double, G> f[3], e[1], v[EV ? 6 : 1];
+  __device__ __forceinline__ void add(int part, double dx, double dy, double dz, double fpair) {
+    f[0].a[part] = fma(dx, fpair, f[0].a[part]);
+    f[1].a[part] = fma(dy, fpair, f[1].a[part]);
+    f[2].a[part] = fma(dz, fpair, f[2].a[part]);
   }
-  fo[0] = fi[0];
-  fo[1] = fi[1];
-  fo[2] = fi[2];
-}
+  __device__ __forceinline__ void add_ev(int part, double dx, double dy, double dz, double fpair, double phi,
+                                         int eflag, int vflag) {
+    if (eflag) e[0].a[part] = radd(e[0].a[part], phi);
+    if (vflag) {
+      v[0].a[part] = fma(rmul(dx, dx), fpair, v[0].a[part]);
+      v[1].a[part] = fma(rmul(dy, dy), fpair, v[1].a[part]);
+      v[2].a[part] = fma(rmul(dz, dz), fpair, v[2].a[part]);
+      v[3].a[part] = fma(rmul(dx, dy), fpair, v[3].a[part]);
+      v[4].a[part] = fma(rmul(dx, dz), fpair, v[4].a[part]);
+      v[5].a[part] = fma(rmul(dy, dz), fpair, v[5].a[part]);
+    }
+  }
+  __device__ __forceinline__ void totals(double fi[3], double &esum, double vsum[6]) const {
+#pragma unroll
+    for (int d = 0; d < 3; d++) fi[d] = f[d].total();
+    if constexpr (EV) {
+      esum = e[0].total();
+#pragma unroll
+      for (int k = 0; k < 6; k++) vsum[k] = v[k].total();
+    }
+  }
+};
 
 // ------------------------------------------------------------------- LJ
 
@@ -190,42 +197,31 @@ struct LjParams {
   double cutsq, lj1, lj2, lj3, lj4, offset;
 };
 
-template <bool EV, bool MANY>
-__global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj(PairArgs A, LjParams P) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;   // list slot
-  const bool valid = t < A.nsi;
-  const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
-  double fi[3] = {0, 0, 0}, esum = 0.0, vsum[6] = {0, 0, 0, 0, 0, 0};
-  if (valid) {
-    double4 xi = A.xs[t];
-    const int n_in = A.num_in[t], n = A.num[t];
-    const int *nb = A.nbr + t;
-    auto pair = [&](const double4 &xj) {
-      double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      double rsq = dx * dx + dy * dy + dz * dz;
-      if (rsq < P.cutsq) {
-        double r2inv = 1.0 / rsq;
-        double r6inv = r2inv * r2inv * r2inv;
-        double forcelj = r6inv * (P.lj1 * r6inv - P.lj2);
-        double fpair = forcelj * r2inv;
-        fi[0] += dx * fpair;
-        fi[1] += dy * fpair;
-        fi[2] += dz * fpair;
-        if (EV && A.eflag) esum += r6inv * (P.lj3 * r6inv - P.lj4) - P.offset;
-        if (EV && A.vflag) {
-          vsum[0] += dx * dx * fpair;
-          vsum[1] += dy * dy * fpair;
-          vsum[2] += dz * dz * fpair;
-          vsum[3] += dx * dy * fpair;
-          vsum[4] += dx * dz * fpair;
-          vsum[5] += dy * dz * fpair;
+template <int G, bool EV>
+__global__ void __launch_bounds__(128, EV ? 4 : 6) k_lj(PairArgs A, LjParams P) {
+  double red[7] = {0, 0, 0, 0, 0, 0, 0};
+  for_each_slot<G>(A.nsi, [&](int t, bool valid) {
+    const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
+    ForceSums<G, EV> S;
+    if (valid) {
+      const double4 xi = A.xs[t];
+      walk_list<G>(A, t, i, [&](int part, const double4 &xj, bool apart) {
+        const double dx = rsub(xi.x, xj.x), dy = rsub(xi.y, xj.y), dz = rsub(xi.z, xj.z);
+        const double rsq = fma(dz, dz, fma(dy, dy, rmul(dx, dx)));
+        if (rsq < P.cutsq && !apart) {
+          const double r2inv = 1.0 / rsq;
+          const double r6inv = rmul(rmul(r2inv, r2inv), r2inv);
+          const double fpair = rmul(rmul(r6inv, fma(P.lj1, r6inv, -P.lj2)), r2inv);
+          S.add(part, dx, dy, dz, fpair);
+          if (EV) S.add_ev(part, dx, dy, dz, fpair, fma(r6inv, fma(P.lj3, r6inv, -P.lj4), -P.offset), A.eflag, A.vflag);
         }
-      }
-    };
-    walk_list<MANY>(A, i, nb, n_in, n, pair);
-  }
-  if (EV) finish_site(A, i, valid, fi, esum, vsum, 0.0, 0.0);
-  else finish_force(A, i, valid, fi);
+      });
+    }
+    double fi[3], esum = 0.0, vsum[6];
+    S.totals(fi, esum, vsum);
+    if (valid && threadIdx.x % G == 0) finish_site<EV>(A, i, fi, esum, vsum, 0.0, 0.0, red);
+  });
+  if (EV) block_reduce_store<7>(red, A.partial);
 }
 
 // ------------------------------------------------------------------ EAM
@@ -240,6 +236,36 @@ struct EamTables {
   double rdr, rdrho, rhomax, cutforcesq;
   int nr, nrho;
 };
+
+// Distance and its reciprocal from the square: rsqrt carries at most one ulp,
+// as the reciprocal of a rounded square root does, and one step of Newton's
+// method takes r = rsq / sqrt(rsq) to within rounding of the square root.
+__device__ __forceinline__ double distance(double rsq, double &recip) {
+  recip = rsqrt(rsq);
+  const double r = rmul(rsq, recip);
+  return fma(fma(-r, r, rsq), rmul(0.5, recip), r);
+}
+
+// The knot of distance r and the place p in its interval, as the reference's
+// m = int(r / dr + 1), limited to nr - 1, and p = min(r / dr + 1 - m, 1): the
+// truncation is a fused operation rounded down at 2^52.
+__device__ __forceinline__ int r_knot(const EamTables &T, double r, double &p) {
+  const double x = __fma_rd(r, T.rdr, 4503599627370497.0);   // 2^52 + 1
+  int m = __double2loint(x);
+  p = fma(r, T.rdr, rsub(4503599627370497.0, x));
+  if (m >= T.nr) {
+    m = T.nr - 1;
+    p = 1.0;
+  }
+  return m;
+}
+
+// A cubic's value and derivative (Horner's scheme and its derivative's).
+__device__ __forceinline__ double cubic(const double4 &c, double p) { return fma(fma(fma(c.x, p, c.y), p, c.z), p, c.w); }
+__device__ __forceinline__ double cubic_slope(const double4 &c, double p) {
+  const double b = fma(c.x, p, c.y);
+  return fma(fma(c.x, p, b), p, fma(b, p, c.z));
+}
 
 // F'(rho) and F(rho) on the frho spline row (PairEAM::compute_fp,
 // pair_eam.cpp:1160-1169; the energy read on the same row, i.e. the
@@ -264,28 +290,25 @@ __device__ __forceinline__ double eam_fp(const EamTables &T, double rho, double 
 // pass 1: density at atoms and node Gauss points (pair_eam.cpp:707-812), then
 // F' at the site itself into xs[i].w (pair_eam.cpp:819-833 for atoms; for a
 // node the reference's rhoi = noderho at :901-903).
-template <bool MANY>
-__device__ __forceinline__ void rho_slot(const PairArgs &A, const EamTables &T, int t, double *rho_out,
+template <int G>
+__device__ __forceinline__ void rho_slot(const PairArgs &A, const EamTables &T, int t, bool valid, double *rho_out,
                                          double *phi_site) {
-  const int i = site_of_slot(A, t);                       // site-table index
-  double4 xi = A.xs[t];
-  const int n_in = A.num_in[t], n = A.num[t];
-  const int *nb = A.nbr + t;
-  double rho = 0.0;
-  auto pair = [&](const double4 &xj) {
-    const double dx = rsub(xi.x, xj.x), dy = rsub(xi.y, xj.y), dz = rsub(xi.z, xj.z);
-    const double rsq = radd(radd(rmul(dx, dx), rmul(dy, dy)), rmul(dz, dz));
-    if (rsq < T.cutforcesq) {
-      double p = radd(rmul(sqrt(rsq), T.rdr), 1.0);
-      int m = (int)p;
-      m = max(1, min(m, T.nr - 1));
-      p = rsub(p, (double)m);
-      p = fmin(p, 1.0);
-      double4 c = ldg256(T.rz + 2 * m);
-      rho = radd(rho, radd(rmul(radd(rmul(radd(rmul(c.x, p), c.y), p), c.z), p), c.w));
-    }
-  };
-  walk_list<MANY>(A, i, nb, n_in, n, pair);
+  const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
+  Sum4<double, G> sum;
+  if (valid) {
+    const double4 xi = A.xs[t];
+    walk_list<G>(A, t, i, [&](int part, const double4 &xj, bool apart) {
+      const double dx = rsub(xi.x, xj.x), dy = rsub(xi.y, xj.y), dz = rsub(xi.z, xj.z);
+      const double rsq = fma(dz, dz, fma(dy, dy, rmul(dx, dx)));
+      if (rsq < T.cutforcesq && !apart) {
+        double recip, p;
+        const int m = r_knot(T, distance(rsq, recip), p);
+        sum.a[part] = radd(sum.a[part], cubic(ldg256(T.rz + 2 * m), p));
+      }
+    });
+  }
+  const double rho = sum.total();
+  if (!valid || threadIdx.x % G) return;
   int slot = i;
   if (i >= A.na) {
     int e = (i - A.na) / NG, g = (i - A.na) % NG;
@@ -298,28 +321,35 @@ __device__ __forceinline__ void rho_slot(const PairArgs &A, const EamTables &T, 
   if (A.eflag) phi_site[i] = phi;
 }
 
-template <int TB, bool MANY>
+template <int TB, int G>
 __global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho(PairArgs A, EamTables T, double *rho_out,
                                                        double *phi_site) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;   // list slot
-  if (t >= A.nsi) return;
-  rho_slot<MANY>(A, T, t, rho_out, phi_site);
+  for_each_slot<G>(A.nsi, [&](int t, bool valid) { rho_slot<G>(A, T, t, valid, rho_out, phi_site); });
 }
 
+// Both passes are bound by the L1 data pipe (ncu, 313 k sites: force pass 84 %
+// of its peak while active, FP64 pipe 24 %, density pass 77 % and 20 %): each
+// neighbour's 32-byte record and each in-cutoff pair's 64-byte spline record is
+// a scattered read.  Fused operations and one rsqrt in place of a root and a
+// division halve the FP64 work (1.21 M sites: density 410 -> 397 us, force 581
+// -> 570; with tallies 747 -> 658; 6 k sites, four lanes a site, 43 -> 15 and
+// 45 -> 17).  Sharing a spline record's two halves between neighbouring lanes
+// was slower (641 us: the exchanges cost more than the reads).
+//
 // Single systems: the force-only passes over SM-local runs of list slots
 // (sm_run, device.cuh); each slot is computed by the same function as in the
 // grid launch, so the results are the grid launch's bit for bit.
-template <int TB>
+template <int TB, int G>
 __global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho_sm(PairArgs A, EamTables T, double *rho_out,
                                                           double *phi_site, int *cnt, int nsm) {
   __shared__ int v;
   if (threadIdx.x == 0) v = sm_id() % nsm;
-  const int nrun = (A.nsi + TB - 1) / TB;
+  const int nrun = (A.nsi + TB / G - 1) / (TB / G);
   for (;;) {
     const int r = sm_run(cnt, nsm, nrun, v);
     if (r < 0) return;
-    const int t = r * TB + threadIdx.x;
-    if (t < A.nsi) rho_slot<false>(A, T, t, rho_out, phi_site);
+    const int t = r * (TB / G) + (int)threadIdx.x / G;
+    rho_slot<G>(A, T, t, t < A.nsi, rho_out, phi_site);
   }
 }
 
@@ -340,88 +370,60 @@ __global__ void k_eam_site_fp(double4 *xs, const int *act_gid, const int *nact_d
 }
 
 // pass 2: forces (pair_eam.cpp:845-1028)
-template <bool EV, bool MANY>
-__device__ __forceinline__ void force_slot(const PairArgs &A, const EamTables &T, int t, int i,
-                                           const double *phi_site, double fi[3], double &esum, double vsum[6],
-                                           double &eemb_site, double &eemb_global) {
-  {
-    double4 xi = A.xs[t];
-    double fpi = xi.w;
-    const int n_in = A.num_in[t], n = A.num[t];
-    const int *nb = A.nbr + t;
-    auto pair = [&](const double4 &xj) {
+template <int G, bool EV>
+__device__ __forceinline__ void force_slot(const PairArgs &A, const EamTables &T, int t, bool valid,
+                                           const double *phi_site, double red[7]) {
+  const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
+  ForceSums<G, EV> S;
+  if (valid) {
+    const double4 xi = A.xs[t];
+    const double fpi = xi.w;
+    walk_list<G>(A, t, i, [&](int part, const double4 &xj, bool apart) {
       const double dx = rsub(xi.x, xj.x), dy = rsub(xi.y, xj.y), dz = rsub(xi.z, xj.z);
-      const double rsq = radd(radd(rmul(dx, dx), rmul(dy, dy)), rmul(dz, dz));
-      if (rsq < T.cutforcesq) {
-        const double r = sqrt(rsq);
-        double p = radd(rmul(r, T.rdr), 1.0);
-        int m = (int)p;
-        m = max(1, min(m, T.nr - 1));
-        p = rsub(p, (double)m);
-        p = fmin(p, 1.0);
-        double4 rv = ldg256(T.rz + 2 * m);
-        double4 zv = ldg256(T.rz + 2 * m + 1);
-        const double rhop = rmul(radd(rmul(radd(rmul(rmul(3.0, rv.x), p), rmul(2.0, rv.y)), p), rv.z), T.rdr);
-        const double z2p = rmul(radd(rmul(radd(rmul(rmul(3.0, zv.x), p), rmul(2.0, zv.y)), p), zv.z), T.rdr);
-        const double z2 = radd(rmul(radd(rmul(radd(rmul(zv.x, p), zv.y), p), zv.z), p), zv.w);
-        const double recip = 1.0 / r;
-        const double phi = rmul(z2, recip);
-        const double phip = rsub(rmul(z2p, recip), rmul(phi, recip));
-        const double psip = radd(radd(rmul(fpi, rhop), rmul(xj.w, rhop)), phip);
-        const double fpair = -rmul(psip, recip);
-        fi[0] = radd(fi[0], rmul(dx, fpair));
-        fi[1] = radd(fi[1], rmul(dy, fpair));
-        fi[2] = radd(fi[2], rmul(dz, fpair));
-        if (EV && A.eflag) esum = radd(esum, phi);
-        if (EV && A.vflag) {
-          vsum[0] = radd(vsum[0], rmul(rmul(dx, dx), fpair));
-          vsum[1] = radd(vsum[1], rmul(rmul(dy, dy), fpair));
-          vsum[2] = radd(vsum[2], rmul(rmul(dz, dz), fpair));
-          vsum[3] = radd(vsum[3], rmul(rmul(dx, dy), fpair));
-          vsum[4] = radd(vsum[4], rmul(rmul(dx, dz), fpair));
-          vsum[5] = radd(vsum[5], rmul(rmul(dy, dz), fpair));
-        }
+      const double rsq = fma(dz, dz, fma(dy, dy, rmul(dx, dx)));
+      if (rsq < T.cutforcesq && !apart) {
+        double recip, p;
+        const int m = r_knot(T, distance(rsq, recip), p);
+        const double4 rv = ldg256(T.rz + 2 * m), zv = ldg256(T.rz + 2 * m + 1);
+        const double rhop = rmul(cubic_slope(rv, p), T.rdr);
+        const double phi = rmul(cubic(zv, p), recip);
+        const double phip = rmul(fma(cubic_slope(zv, p), T.rdr, -phi), recip);
+        const double fpair = -rmul(fma(radd(fpi, xj.w), rhop, phip), recip);
+        S.add(part, dx, dy, dz, fpair);
+        if (EV) S.add_ev(part, dx, dy, dz, fpair, phi, A.eflag, A.vflag);
       }
-    };
-    walk_list<MANY>(A, i, nb, n_in, n, pair);
-    if (EV && A.eflag) {
-      double phi = phi_site[i];
-      eemb_site = phi;
-      eemb_global = (i < A.na) ? phi : phi * A.escale_node * 2.0;
-    }
+    });
   }
+  double fi[3], esum = 0.0, vsum[6];
+  S.totals(fi, esum, vsum);
+  if (!valid || threadIdx.x % G) return;
+  double eemb_site = 0.0, eemb_global = 0.0;
+  if (EV && A.eflag) {
+    eemb_site = phi_site[i];
+    eemb_global = i < A.na ? eemb_site : eemb_site * A.escale_node * 2.0;
+  }
+  finish_site<EV>(A, i, fi, esum, vsum, eemb_site, eemb_global, red);
 }
 
-template <int TB, bool EV, bool MANY>
+template <int TB, int G, bool EV>
 __global__ void __launch_bounds__(TB, (EV ? 512 : 768) / TB) k_eam_force(PairArgs A, EamTables T,
                                                                        const double *phi_site) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;   // list slot
-  const bool valid = t < A.nsi;
-  const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
-  double fi[3] = {0, 0, 0}, esum = 0.0, vsum[6] = {0, 0, 0, 0, 0, 0};
-  double eemb_site = 0.0, eemb_global = 0.0;
-  if (valid) force_slot<EV, MANY>(A, T, t, i, phi_site, fi, esum, vsum, eemb_site, eemb_global);
-  if (EV) finish_site(A, i, valid, fi, esum, vsum, eemb_site, eemb_global);
-  else finish_force(A, i, valid, fi);
+  double red[7] = {0, 0, 0, 0, 0, 0, 0};
+  for_each_slot<G>(A.nsi, [&](int t, bool valid) { force_slot<G, EV>(A, T, t, valid, phi_site, red); });
+  if (EV) block_reduce_store<7>(red, A.partial);
 }
 
-template <int TB>
-__global__ void __launch_bounds__(TB, 768 / TB) k_eam_force_sm(PairArgs A, EamTables T, const double *phi_site,
+template <int TB, int G>
+__global__ void __launch_bounds__(TB, 640 / TB) k_eam_force_sm(PairArgs A, EamTables T, const double *phi_site,
                                                            int *cnt, int nsm) {
   __shared__ int v;
   if (threadIdx.x == 0) v = sm_id() % nsm;
-  const int nrun = (A.nsi + TB - 1) / TB;
+  const int nrun = (A.nsi + TB / G - 1) / (TB / G);
   for (;;) {
     const int r = sm_run(cnt, nsm, nrun, v);
     if (r < 0) return;
-    const int t = r * TB + threadIdx.x;
-    if (t < A.nsi) {
-      const int i = site_of_slot(A, t);
-      double fi[3] = {0, 0, 0}, esum = 0.0, vsum[6] = {0, 0, 0, 0, 0, 0};
-      double eemb_site = 0.0, eemb_global = 0.0;
-      force_slot<false, false>(A, T, t, i, phi_site, fi, esum, vsum, eemb_site, eemb_global);
-      finish_force(A, i, true, fi);
-    }
+    const int t = r * (TB / G) + (int)threadIdx.x / G;
+    force_slot<G, false>(A, T, t, t < A.nsi, phi_site, nullptr);
   }
 }
 
@@ -504,23 +506,32 @@ void eam_tables(Ctx &c, const double *frho, const double *rhor, const double *z2
   stream_copy(c, c.rz.p, rz.data(), sizeof(double4) * rz.size(), cudaMemcpyHostToDevice);
 }
 
-// Block size of the force-only pair passes, chosen per context by timing 64,
-// 128 and 256 threads (best of three launches each; 128 unless another is at
-// least 3 % faster) on the context's own lists the first time they run
-// (every thread owns one list slot, so results do not depend on the choice;
-// the passes are idempotent, so the trial launches change nothing).  Not
-// during stream capture: there the default stays.
-template <bool MANY>
+// i-sites from which a site takes two lanes, and below which four (the sums
+// do not depend on it).  us with 1 / 2 / 4 lanes a site before the walk loaded
+// ahead: LJ pass 6 k sites 34 / 21 / 17, 84 k 42 / 40 / 39, 313 k 119 / 105 /
+// 118, 1.21 M 356 / 354 / 423; EAM force pass 45 / 31 / 22, 68 / 63 / 61,
+// 178 / 174 / 182, 578 / 574 / 616.
+constexpr int TWO_LANE_SITES = 100000;
+
+// Block size of the force-only pair passes of batches, chosen per context by
+// timing 64, 128 and 256 threads (best of three launches each; 128 unless
+// another is at least 3 % faster) on the context's own lists the first time
+// they run (results do not depend on the choice; the passes are idempotent, so
+// the trial launches change nothing).  Not during stream capture: there the
+// default stays.
+template <int G>
 void launch_rho(int tb, int nsi, cudaStream_t st, const PairArgs &A, const EamTables &T, double *rho, double *phi) {
-  if (tb == 64) k_eam_rho<64, MANY><<<std::max(nblk(nsi, 64), 1), 64, 0, st>>>(A, T, rho, phi);
-  else if (tb == 256) k_eam_rho<256, MANY><<<std::max(nblk(nsi, 256), 1), 256, 0, st>>>(A, T, rho, phi);
-  else k_eam_rho<128, MANY><<<std::max(nblk(nsi, 128), 1), 128, 0, st>>>(A, T, rho, phi);
+  const int nb = std::max(nblk((long)nsi * G, tb), 1);
+  if (tb == 64) k_eam_rho<64, G><<<nb, 64, 0, st>>>(A, T, rho, phi);
+  else if (tb == 256) k_eam_rho<256, G><<<nb, 256, 0, st>>>(A, T, rho, phi);
+  else k_eam_rho<128, G><<<nb, 128, 0, st>>>(A, T, rho, phi);
 }
-template <bool MANY>
+template <int G>
 void launch_force(int tb, int nsi, cudaStream_t st, const PairArgs &A, const EamTables &T, const double *phi) {
-  if (tb == 64) k_eam_force<64, false, MANY><<<std::max(nblk(nsi, 64), 1), 64, 0, st>>>(A, T, phi);
-  else if (tb == 256) k_eam_force<256, false, MANY><<<std::max(nblk(nsi, 256), 1), 256, 0, st>>>(A, T, phi);
-  else k_eam_force<128, false, MANY><<<std::max(nblk(nsi, 128), 1), 128, 0, st>>>(A, T, phi);
+  const int nb = std::max(nblk((long)nsi * G, tb), 1);
+  if (tb == 64) k_eam_force<64, G, false><<<nb, 64, 0, st>>>(A, T, phi);
+  else if (tb == 256) k_eam_force<256, G, false><<<nb, 256, 0, st>>>(A, T, phi);
+  else k_eam_force<128, G, false><<<nb, 128, 0, st>>>(A, T, phi);
 }
 
 template <class F>
@@ -558,7 +569,13 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
   }
   const int nsi = c.nsite_i();
   const int T = 128;
-  const int nb = std::max(nblk(nsi, T), 1);
+  const int lanes = nsi >= TWO_LANE_SITES ? 2 : 4;
+  auto by_lanes = [&](auto &&launch) {
+    if (lanes == 2) launch(std::integral_constant<int, 2>());
+    else launch(std::integral_constant<int, 4>());
+  };
+  const int nb = std::max(nblk((long)nsi * lanes, T), 1);
+  const int nb_ev = std::min(nb, 4 * c.num_sms);   // with tallies: resident blocks, one partial each
   PairArgs A;
   A.xs = c.xss.p;
   A.nbr = c.nbr_full.p;
@@ -587,7 +604,7 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
   A.enode = c.enode.p;
   A.vatom = c.vatom.p;
   A.vnode = c.vnode.p;
-  c.partial.reserve((size_t)nb * 7);
+  c.partial.reserve((size_t)nb_ev * 7);
   c.ev_out.reserve(7);
   A.partial = c.partial.p;
   A.eflag = eflag;
@@ -602,13 +619,11 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
   if (c.pp.style == CACB200_PAIR_LJ) {
     LjParams P{c.pp.cut * c.pp.cut, c.pp.lj1, c.pp.lj2, c.pp.lj3, c.pp.lj4, c.pp.offset};
     KernelTimer t(c, "pair_lj");
-    if (c.nrep > 1) {
-      if (eflag || vflag) k_lj<true, true><<<nb, T, 0, c.stream>>>(A, P);
-      else k_lj<false, true><<<nb, T, 0, c.stream>>>(A, P);
-    } else {
-      if (eflag || vflag) k_lj<true, false><<<nb, T, 0, c.stream>>>(A, P);
-      else k_lj<false, false><<<nb, T, 0, c.stream>>>(A, P);
-    }
+    by_lanes([&](auto g) {
+      constexpr int G = decltype(g)::value;
+      if (eflag || vflag) k_lj<G, true><<<nb_ev, T, 0, c.stream>>>(A, P);
+      else k_lj<G, false><<<nb, T, 0, c.stream>>>(A, P);
+    });
   } else if (c.pp.style == CACB200_PAIR_EAM) {
     EamTables Tb;
     Tb.rz = c.rz.p;
@@ -629,15 +644,14 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
             c.xss.p, c.act_gid.p, c.dev_nact.p, c.na + NG * c.ne, c.na, c.rho.p, Tb);
     };
     auto rho = [&](int tb) {
-      if (many) launch_rho<true>(tb, nsi, c.stream, A, Tb, c.rho.p, c.phi_site.p);
-      else launch_rho<false>(tb, nsi, c.stream, A, Tb, c.rho.p, c.phi_site.p);
+      by_lanes([&](auto g) { launch_rho<decltype(g)::value>(tb, nsi, c.stream, A, Tb, c.rho.p, c.phi_site.p); });
     };
     auto force = [&](int tb) {
-      if (many) launch_force<true>(tb, nsi, c.stream, A, Tb, c.phi_site.p);
-      else launch_force<false>(tb, nsi, c.stream, A, Tb, c.phi_site.p);
+      by_lanes([&](auto g) { launch_force<decltype(g)::value>(tb, nsi, c.stream, A, Tb, c.phi_site.p); });
     };
-    // single systems: the force-only passes over SM-local runs
-    const bool smq = !many && c.work_queue;
+    // single systems of more than a wave of blocks: the force-only passes
+    // over SM-local runs
+    const bool smq = !many && c.work_queue && lanes == 2;
     c.sm_counter.reserve(2 * c.num_sms);
     auto sm_grid = [&](auto kernel, int &cache) {
       if (!cache) {
@@ -650,15 +664,15 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
     static int grid_rho_sm = 0, grid_force_sm = 0;
     auto rho_s = [&] {
       CACB200_CUDA(cudaMemsetAsync(c.sm_counter.p, 0, sizeof(int) * c.num_sms, c.stream));
-      k_eam_rho_sm<128><<<sm_grid(k_eam_rho_sm<128>, grid_rho_sm), 128, 0, c.stream>>>(
+      k_eam_rho_sm<128, 2><<<sm_grid(k_eam_rho_sm<128, 2>, grid_rho_sm), 128, 0, c.stream>>>(
           A, Tb, c.rho.p, c.phi_site.p, c.sm_counter.p, c.num_sms);
     };
     auto force_s = [&] {
       CACB200_CUDA(cudaMemsetAsync(c.sm_counter.p + c.num_sms, 0, sizeof(int) * c.num_sms, c.stream));
-      k_eam_force_sm<128><<<sm_grid(k_eam_force_sm<128>, grid_force_sm), 128, 0, c.stream>>>(
+      k_eam_force_sm<128, 2><<<sm_grid(k_eam_force_sm<128, 2>, grid_force_sm), 128, 0, c.stream>>>(
           A, Tb, c.phi_site.p, c.sm_counter.p + c.num_sms, c.num_sms);
     };
-    if (!smq && c.tune_gen != c.gen && !eflag && !vflag && !capturing(c.stream)) {
+    if (many && c.tune_gen != c.gen && !eflag && !vflag && !capturing(c.stream)) {
       // another size replaces 128 only when it is at least 3 % faster
       const int cand[3] = {128, 64, 256};
       float best = 1e30f;
@@ -687,8 +701,9 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
     {
       KernelTimer t(c, "eam_force");
       if (eflag || vflag) {
-        if (many) k_eam_force<128, true, true><<<nb, T, 0, c.stream>>>(A, Tb, c.phi_site.p);
-        else k_eam_force<128, true, false><<<nb, T, 0, c.stream>>>(A, Tb, c.phi_site.p);
+        by_lanes([&](auto g) {
+          k_eam_force<128, decltype(g)::value, true><<<nb_ev, T, 0, c.stream>>>(A, Tb, c.phi_site.p);
+        });
       } else if (smq) {
         force_s();
       } else {
@@ -699,7 +714,7 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
     throw Error(CACB200_ESTATE, "no pair style set");
   }
   if (eflag || vflag) {
-    k_reduce_partials<<<1, 256, 0, c.stream>>>(c.partial.p, nb, c.ev_out.p);
+    k_reduce_partials<<<1, 256, 0, c.stream>>>(c.partial.p, nb_ev, c.ev_out.p);
     c.have_peratom_e = (eflag & CACB200_ENERGY_ATOM) != 0;
     c.have_peratom_v = (vflag & CACB200_VIRIAL_ATOM) != 0;
     c.ev_pending = true;

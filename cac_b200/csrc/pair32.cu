@@ -137,30 +137,6 @@ struct Args32 {
 
 __device__ __forceinline__ int site_of_slot(const Args32 &A, int t) { return t < A.na ? A.slot_atom[t] : t; }
 
-// A site's sums are kept in four partial sums: entry k of a walk goes to
-// partial k mod 4, and the partials are added as (0 + 1) + (2 + 3).  G lanes
-// share a site (G = 1, 2 or 4; lane g walks entries g, g + G, ...) and each
-// holds 4 / G of the partials, so a site's result is the same bit for bit
-// whatever G is: large systems take one lane per site, small ones, which
-// would leave the chip idle, more.
-template <int G>
-struct Sum4 {
-  float a[4 / G];
-  __device__ __forceinline__ Sum4() {
-#pragma unroll
-    for (int k = 0; k < 4 / G; k++) a[k] = 0.0f;
-  }
-  // the site's sum, in every lane of its group (every lane of the warp calls it)
-  __device__ __forceinline__ float total() const {
-    float t[4 / G];
-#pragma unroll
-    for (int k = 0; k < 4 / G; k++) t[k] = lanes_sum<G>(a[k]);
-    if constexpr (G == 1) return __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
-    else if constexpr (G == 2) return __fadd_rn(t[0], t[1]);
-    else return t[0];
-  }
-};
-
 // Walks n entries of a list: each lane takes four at a time, the next four
 // entries loaded ahead and the four records issued back to back before any is
 // used.  Entries past the end are walked as pairs too far apart to count.
@@ -259,23 +235,10 @@ __device__ __forceinline__ void finish32(const Args32 &A, int i, const float fi[
   }
 }
 
-// The pair passes' threads: runs of 32 / G consecutive list slots, one per
-// warp, consecutive warps taking consecutive runs, grid-stride.  body(slot,
-// valid) is called by whole warps.
-template <int G, class F>
-__device__ __forceinline__ void for_each_slot(const Args32 &A, F &&body) {
-  constexpr int S = 32 / G;
-  const int warps = blockDim.x >> 5, nrun = (A.nsi + S - 1) / S;
-  for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < nrun; r += gridDim.x * warps) {
-    const int t = r * S + (threadIdx.x & 31) / G;
-    body(t, t < A.nsi);
-  }
-}
-
 // Per-site sums of a force pass.
 template <int G, bool EV>
 struct ForceSums {
-  Sum4<G> f[3], e[1], v[EV ? 6 : 1];
+  Sum4<float, G> f[3], e[1], v[EV ? 6 : 1];
   __device__ __forceinline__ void add(int part, float dx, float dy, float dz, float fpair) {
     f[0].a[part] = __fmaf_rn(dx, fpair, f[0].a[part]);
     f[1].a[part] = __fmaf_rn(dy, fpair, f[1].a[part]);
@@ -308,7 +271,7 @@ struct Lj32 {
 template <int G, bool EV>
 __global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj32(Args32 A, Lj32 P) {
   double red[7] = {0, 0, 0, 0, 0, 0, 0};
-  for_each_slot<G>(A, [&](int t, bool valid) {
+  for_each_slot<G>(A.nsi, [&](int t, bool valid) {
     const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
     ForceSums<G, EV> S;
     if (valid) {
@@ -428,9 +391,9 @@ __global__ void __launch_bounds__(512, 2) k_eam_rho32(Args32 A, Eam32 T, double 
   extern __shared__ float4 tab[];
   if (FAST) load_fast(T, T.fast, 1, tab);
   const float4 *mine = tab + threadIdx.x % T.copies;
-  for_each_slot<G>(A, [&](int t, bool valid) {
+  for_each_slot<G>(A.nsi, [&](int t, bool valid) {
     const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
-    Sum4<G> sum;
+    Sum4<float, G> sum;
     if (valid) {
       const int4 oi = __ldg(A.pos + t);
       for_each32<G>(A, t, i, oi, [&](int part, float, float, float, float rsq, float) {
@@ -485,7 +448,7 @@ __global__ void __launch_bounds__(512, EV ? 1 : 2) k_eam_force32(Args32 A, Eam32
   const float4 *mine = tab + threadIdx.x % T.copies;
   const int second = (T.cnt + 1) * T.copies;
   double red[7] = {0, 0, 0, 0, 0, 0, 0};
-  for_each_slot<G>(A, [&](int t, bool valid) {
+  for_each_slot<G>(A.nsi, [&](int t, bool valid) {
     const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
     ForceSums<G, EV> S;
     if (valid) {
