@@ -195,7 +195,6 @@ struct Ctx {
   DBuf<int> dev_nact;            // device count written by each rebuild
   size_t ns_cap = 0;             // site-table capacity (every lattice site active)
   DBuf<int> act_gid;             // [nact] e*729 + u
-  DBuf<int> act_off;             // [ne+1] CSR of active sites by element (into act_gid)
   int nsite_i() const { return na + NG * ne; }
 
   DBuf<double> v, f;             // atoms [na*3]
@@ -235,6 +234,7 @@ struct Ctx {
   DBuf<int> acell_fix;           // [3][na] the same in fixed point (the atom build's screen, neigh.cu)
   DBuf<int> acell_of;            // [na] cell of each sorted atom
   DBuf<int> ecell_start, ecell_elems;
+  DBuf<double4> ecell_sphere;    // [ne] candidate spheres of the sorted elements
   DBuf<int> cell_key, cell_key2, idx_tmp;
   DBuf<int> atom_work, atom_nwork;   // atoms with element sites in reach (rebuild work list)
   DBuf<int2> items;                  // [slots][item_cap] element boxes to test, per query
@@ -295,8 +295,8 @@ struct Ctx {
   bool have_half = false, lists_valid = false;
   DBuf<int> raw_full, raw_half;  // build-time element-site entries (full) and half lists before compaction
   DBuf<unsigned char> img_full, img_half;
-  DBuf<int> site_flag;           // [ne*729 + 1] marks
-  DBuf<int> site_pref;           // [ne*729 + 1] exclusive prefix of the marks
+  DBuf<unsigned char> site_flag; // marks of the lattice sites that are neighbours (neigh.cu) ...
+  DBuf<uint2> site_words;        // ... as bits, with their ranks in act_gid
   DBuf<int> overflow;            // [16] device flags (see neigh_check)
   int build_count = 0;
 

@@ -54,6 +54,10 @@ namespace cacb200 {
 
 namespace {
 
+// Marks of an element's lattice sites: a byte each while lists are built, then
+// one bit each in words of 32 with the pair-table rank of the word's first.
+constexpr int MARK_WORDS = (NU + 31) / 32, MARKS = 32 * MARK_WORDS;
+
 constexpr int KIND_SITE = 1 << 30;  // build-time entry flag: lattice site (gid = e*729+u)
 
 // Replica lookup.  A single system uses OneRep (its descriptor is a kernel
@@ -79,10 +83,36 @@ struct ManyRep {
 
 // ------------------------------------------------------------------ pbc
 
-// Domain::pbc for owned atoms (domain.cpp:562-630)
+// What a rebuild starts from, cleared by its first kernel.
+struct BuildStart {
+  double4 *xbuild;      // the wrapped positions the lists are built from (null: only wrap)
+  float *disp;
+  int *inner_ok;        // [nrep]
+  int inner;            // the prefix is usable (its margin is not zero)
+  unsigned *dmax;       // [nrep]
+  int *overflow, *nact, *nwork, *sm_counter;
+  int nrep, nsm;
+};
+
+// Domain::pbc for owned atoms (domain.cpp:562-630), and the clearing of the
+// rebuild's flags and counters (one launch instead of a dozen small ones,
+// which a small system would wait for one by one).
 template <class RP>
-__global__ void k_pbc_atoms(double4 *xs, int na, RP P) {
+__global__ void k_pbc_atoms(double4 *xs, int na, RP P, BuildStart S) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (S.xbuild) {
+    if (i < S.nrep) {
+      S.inner_ok[i] = S.inner;
+      S.dmax[i] = 0u;
+    }
+    if (i < S.nsm) S.sm_counter[i] = 0;
+    if (i < 4) S.overflow[i] = 0;
+    if (i < 2) S.overflow[8 + i] = 0;
+    if (i == 0) {
+      *S.nact = 0;
+      *S.nwork = 0;
+    }
+  }
   if (i >= na) return;
   const BoxD b = P.site(i).b;
   double4 p = xs[i];
@@ -98,6 +128,10 @@ __global__ void k_pbc_atoms(double4 *xs, int na, RP P) {
     q[d] = x;
   }
   xs[i] = p;
+  if (S.xbuild) {
+    S.xbuild[i] = p;
+    S.disp[i] = 0.0f;
+  }
 }
 
 // Element centre (ElementVecCAC::update_center_coord, element_vec_cac.cpp:3740-3765),
@@ -116,7 +150,7 @@ constexpr int EFR = 28;
 
 template <class RP>
 __global__ void k_elem_geom(double *nodex, int ne, RP P, double4 *ecenter, double *eframe,
-                            unsigned long long *reach_bits, int *grew) {
+                            unsigned long long *reach_bits, int *grew, double *nodex_build, float *edisp) {
   int e = blockIdx.x * blockDim.x + threadIdx.x;
   double reach = 0.0;
   if (e < ne) {
@@ -206,6 +240,10 @@ __global__ void k_elem_geom(double *nodex, int ne, RP P, double4 *ecenter, doubl
 #pragma unroll
       for (int d = 0; d < 3; d++) fr[13 + 3 * q + d] = A[d][q];
     ecenter[e] = make_double4(c[0], c[1], c[2], R);
+    if (nodex_build) {   // the nodes the lists are built from
+      for (int k = 0; k < 24; k++) nodex_build[(size_t)e * 24 + k] = nx[k];
+      edisp[e] = 0.0f;
+    }
     reach = R + dmax;
     if (!(reach <= rp.reach_budget)) atomicExch(grew, 1);
     // per-replica maximum (non-negative doubles order like their bit patterns)
@@ -284,6 +322,17 @@ __global__ void k_cell_start(const int *skey, int n, int ncell, int *start) {
   start[c] = lo;
 }
 
+// The sorted elements' candidate spheres: centre, and reach of the sites
+// (radius + deviation from affine) in w.
+__global__ void k_gather_spheres(const double4 *ecenter, const double *eframe, const int *sidx, int n, double4 *out) {
+  int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int e = sidx[k];
+  double4 c = ecenter[e];
+  c.w += eframe[(size_t)e * EFR + 12];
+  out[k] = c;
+}
+
 // Fixed-point copy of a wrapped atom position for the screen of the atom build: quanta of
 // 2^-20 A from the box corner, modulo 2^32 (4096 A), so that the differences
 // of near positions are exact integers whatever the size of the box.  An atom
@@ -336,8 +385,9 @@ struct BuildArgs {
   const unsigned char *ecell_near;   // single systems: element cell has an element in its 27-cell block (else null)
   const unsigned char *acell_near;   // single systems: atom cell has an atom in its 27-cell block (else null)
   const int *ecell_elems;
+  const double4 *ecell_sphere;   // the sorted elements' candidate spheres
   const int *atom_of_slot;    // list slot (cell-sorted position) -> atom index
-  int *site_flag;             // [ne * 729] marks the lattice sites some full list references
+  unsigned char *site_flag;   // [ne * MARKS] marks the lattice sites some full list references
   int na, ne, nsi, cap;
   RefBins rb;                 // single systems only (half lists)
   double cutneigh, cutneighsq;
@@ -520,10 +570,71 @@ __device__ __forceinline__ void unpack_item(int2 it, int &e, int s[3], int lo[3]
   }
 }
 
-// Phase A for one query: the element walk (candidate sphere test, then the
-// lattice-index box of the sites whose affine position can lie within
-// cutneigh + the element's deviation from affine).  Returns the number of
-// items; at most cap are stored.
+__device__ __forceinline__ unsigned lanemask_lt() {
+  unsigned m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+
+// The cell c (0 .. 26, x fastest) around a query's element cell: its elements
+// [beg, end) of the sorted ones, and the image its elements are seen under.
+__device__ __forceinline__ void element_cell(const BuildArgs &A, const Query &q, const int ci[3], int c, int &beg,
+                                             int &end, int s[3]) {
+  const Grid &eg = q.r.eg;
+  const int o[3] = {c % 3 - 1, c / 3 % 3 - 1, c / 9 - 1};
+  int cc[3], W;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    wrap_cell(ci[d] + o[d], eg.nc[d], cc[d], W);
+    s[d] = W - q.ti[d];
+  }
+  const int cell = q.r.ebase + (cc[2] * eg.nc[1] + cc[1]) * eg.nc[0] + cc[0];
+  beg = A.ecell_start[cell];
+  end = A.ecell_start[cell + 1];
+}
+
+// The work item of the element at place kk of the sorted ones, seen under
+// image s: a candidate sphere test, then the lattice-index box of the sites
+// whose affine position can lie within cutneigh + the element's deviation from
+// affine.  False: no site in reach.
+__device__ __forceinline__ bool element_item(const BuildArgs &A, const Query &q, int kk, const int s[3], int2 &item) {
+  const double4 ce = ldg256(A.ecell_sphere + kk);
+  // sphere test in the element's raw frame: |xi - s L - centre| <= cutneigh + R
+  const double p[3] = {q.xi[0] - s[0] * q.r.b.L[0], q.xi[1] - s[1] * q.r.b.L[1], q.xi[2] - s[2] * q.r.b.L[2]};
+  const double R = ce.w + A.cutneigh + 1e-6;
+  const double dcx = p[0] - ce.x, dcy = p[1] - ce.y, dcz = p[2] - ce.z;
+  if (dcx * dcx + dcy * dcy + dcz * dcz > R * R) return false;
+  const int e = A.ecell_elems[kk];
+  const double *fr = A.eframe + (size_t)e * EFR;
+  const double dmax = fr[12];
+  const double rel[3] = {p[0] - fr[0], p[1] - fr[1], p[2] - fr[2]};
+  int lo[3], hi[3];
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const double a0 = fr[3 + 3 * r], a1 = fr[4 + 3 * r], a2 = fr[5 + 3 * r];
+    const double fidx = a0 * rel[0] + a1 * rel[1] + a2 * rel[2];
+    const double rho = (A.cutneigh + dmax + 1e-6) * fr[22 + r] + 1e-6;
+    lo[r] = max(0, (int)ceil(fidx - rho));
+    hi[r] = min(NC - 1, (int)floor(fidx + rho));
+    if (lo[r] > hi[r]) return false;
+  }
+  // a box shorter than the candidate sphere's diameter shows an element
+  // under two images; images beyond +-2 cannot be encoded (and are far
+  // beyond any cutoff in such a box)
+  if (s[0] < -3 || s[0] > 3 || s[1] < -3 || s[1] > 3 || s[2] < -3 || s[2] > 3) {
+    atomicExch(&A.overflow[2], 1);
+    return false;
+  }
+  item = pack_item(e, s, lo, hi);
+  return true;
+}
+
+// Phase A for one query, by L neighbouring lanes (L = 1 or 8; every lane of the
+// group calls it with the same query): the items of the 27 cells around, in
+// cell order.  Eight lanes walk eight cells at a time and place their items by
+// the counts of the cells before.  Returns the number of items; at most cap
+// are stored.
+template <int L>
 __device__ int element_items(const BuildArgs &A, const Query &q, int2 *out, int cap) {
   const Grid &eg = q.r.eg;
   int ci[3];
@@ -532,64 +643,53 @@ __device__ int element_items(const BuildArgs &A, const Query &q, int2 *out, int 
     ci[d] = min(max((int)((q.wi[d] - q.r.b.lo[d]) * eg.inv[d]), 0), eg.nc[d] - 1);
   // no element in the 27 cells around: nothing to walk
   if (A.ecell_near && !A.ecell_near[q.r.ebase + (ci[2] * eg.nc[1] + ci[1]) * eg.nc[0] + ci[0]]) return 0;
-  int n = 0;
-  for (int oz = -1; oz <= 1; oz++) {
-    int cz, Wz;
-    wrap_cell(ci[2] + oz, eg.nc[2], cz, Wz);
-    for (int oy = -1; oy <= 1; oy++) {
-      int cy, Wy;
-      wrap_cell(ci[1] + oy, eg.nc[1], cy, Wy);
-      for (int ox = -1; ox <= 1; ox++) {
-        int cx, Wx;
-        wrap_cell(ci[0] + ox, eg.nc[0], cx, Wx);
-        int cell = q.r.ebase + (cz * eg.nc[1] + cy) * eg.nc[0] + cx;
-        int beg = A.ecell_start[cell], end = A.ecell_start[cell + 1];
-        if (beg == end) continue;
-        int s[3] = {Wx - q.ti[0], Wy - q.ti[1], Wz - q.ti[2]};
-        double sL[3] = {s[0] * q.r.b.L[0], s[1] * q.r.b.L[1], s[2] * q.r.b.L[2]};
-        for (int kk = beg; kk < end; kk++) {
-          int e = A.ecell_elems[kk];
-          double4 ce = A.ecenter[e];
-          // sphere test in the element's raw frame: |xi - s L - centre| <= cutneigh + R
-          double p[3] = {q.xi[0] - sL[0], q.xi[1] - sL[1], q.xi[2] - sL[2]};
-          const double *fr = A.eframe + (size_t)e * EFR;
-          double dmax = fr[12];
-          double R = ce.w + dmax + A.cutneigh + 1e-6;
-          double dcx = p[0] - ce.x, dcy = p[1] - ce.y, dcz = p[2] - ce.z;
-          if (dcx * dcx + dcy * dcy + dcz * dcz > R * R) continue;
-          double rel[3] = {p[0] - fr[0], p[1] - fr[1], p[2] - fr[2]};
-          int lo[3], hi[3];
-          bool empty = false;
-#pragma unroll
-          for (int r = 0; r < 3; r++) {
-            double a0 = fr[3 + 3 * r], a1 = fr[4 + 3 * r], a2 = fr[5 + 3 * r];
-            double fidx = a0 * rel[0] + a1 * rel[1] + a2 * rel[2];
-            double rho = (A.cutneigh + dmax + 1e-6) * fr[22 + r] + 1e-6;
-            lo[r] = max(0, (int)ceil(fidx - rho));
-            hi[r] = min(NC - 1, (int)floor(fidx + rho));
-            if (lo[r] > hi[r]) empty = true;
-          }
-          if (empty) continue;
-          // a box shorter than the candidate sphere's diameter shows an element
-          // under two images; images beyond +-2 cannot be encoded (and are far
-          // beyond any cutoff in such a box)
-          if (s[0] < -3 || s[0] > 3 || s[1] < -3 || s[1] > 3 || s[2] < -3 || s[2] > 3) {
-            atomicExch(&A.overflow[2], 1);
-            continue;
-          }
-          if (n < cap) out[n] = pack_item(e, s, lo, hi);
+  int n = 0, s[3], beg, end;
+  int2 item;
+  if (L == 1) {
+    for (int c = 0; c < 27; c++) {
+      element_cell(A, q, ci, c, beg, end, s);
+      for (int kk = beg; kk < end; kk++)
+        if (element_item(A, q, kk, s, item)) {
+          if (n < cap) out[n] = item;
           n++;
         }
+    }
+    return n;
+  }
+  const int sub = threadIdx.x % L;
+  const unsigned group = ((1ull << L) - 1u) << ((threadIdx.x & 31) - sub);
+  for (int c0 = 0; c0 < 27; c0 += L) {
+    beg = end = 0;
+    if (c0 + sub < 27) element_cell(A, q, ci, c0 + sub, beg, end, s);
+    // the lane's accepted elements, 32 of its cell at a time (one round unless
+    // a cell holds more; then the cells' items must not interleave)
+    const bool crowded = __any_sync(group, end - beg > 32);
+    for (int turn = 0; turn < (crowded ? L : 1); turn++) {
+      const bool mine = !crowded || turn == sub;
+      unsigned acc = 0;
+      int count = 0;
+      for (int kk = beg; mine && kk < end; kk++)
+        if (element_item(A, q, kk, s, item)) {
+          if (kk - beg < 32) acc |= 1u << (kk - beg);
+          if (crowded && n + count < cap) out[n + count] = item;
+          count++;
+        }
+      int at = count;
+#pragma unroll
+      for (int o = 1; o < L; o <<= 1) {
+        const int v = __shfl_up_sync(group, at, o, L);
+        if (sub >= o) at += v;
       }
+      const int total = __shfl_sync(group, at, L - 1, L);
+      if (!crowded) {
+        at += n - count;
+        for (; acc; acc &= acc - 1, at++)
+          if (at < cap && element_item(A, q, beg + __ffs(acc) - 1, s, item)) out[at] = item;
+      }
+      n += total;
     }
   }
   return n;
-}
-
-__device__ __forceinline__ unsigned lanemask_lt() {
-  unsigned m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
 }
 
 // Warp-wide emission: the lanes' accepted candidates are stored in lane
@@ -676,7 +776,7 @@ __device__ __forceinline__ void items_exact(const BuildArgs &A, const Query &q, 
         pf = true;
         val = KIND_SITE | (e * NU + u);
         codef = code | (rsq < A.cutforcesq ? IN_CUT : 0);
-        if (site_gauss(u) < 0) A.site_flag[e * NU + u] = 1;   // to be interpolated
+        if (site_gauss(u) < 0) A.site_flag[(size_t)e * MARKS + u] = 1;   // to be interpolated
         ph = true;
         if (A.want_half && !q.iatom) {
           int jg = site_gauss(u);
@@ -1193,11 +1293,11 @@ __global__ void __launch_bounds__(32) k_build_atoms_sm(BuildArgs A, OneRep P, in
 // Phase A over every list slot: the element walk of each atom and Gauss
 // point; atoms with at least one item go on the work list of phase B (its
 // order does not matter: an atom's entries depend on that atom alone).
-template <class RP>
-__device__ __forceinline__ void elem_items_slot(BuildArgs A, RP P, int2 *items, int *nitems, int icap, int *work,
-                                                int *nwork) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= A.nsi) return;
+template <int L, class RP>
+__device__ __forceinline__ void elem_items_slot(const BuildArgs &A, const RP &P, int2 *items, int *nitems, int icap,
+                                                int *work, int *nwork) {
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+  if (t >= A.nsi) return;   // whole groups
   Query q;
   if (t < A.na) {
     make_query(A, P, A.atom_of_slot[t], q);
@@ -1205,7 +1305,8 @@ __device__ __forceinline__ void elem_items_slot(BuildArgs A, RP P, int2 *items, 
   } else {
     make_query(A, P, t, q);
   }
-  const int n = element_items(A, q, items + (size_t)t * icap, icap);
+  const int n = element_items<L>(A, q, items + (size_t)t * icap, icap);
+  if (threadIdx.x % L) return;
   nitems[t] = n;
   if (n > icap) {
     atomicExch(&A.overflow[8], 1);
@@ -1214,16 +1315,21 @@ __device__ __forceinline__ void elem_items_slot(BuildArgs A, RP P, int2 *items, 
   if (t < A.na && n > 0) work[atomicAdd(nwork, 1)] = t;
 }
 
-// The single-system form as the compiler allocates it; the batch form capped
-// at 64 registers (from 70) for 8 resident blocks per SM: 4 % faster on a
-// 64-replica batch, where the same cap slowed the single-system form.
+// One lane per query in the single-system form as the compiler allocates it;
+// the batch form capped at 64 registers (from 70) for 8 resident blocks per
+// SM: 4 % faster on a 64-replica batch, where the same cap slowed the
+// single-system form.  Below EIGHT_LANE_QUERIES a query's serial chain of cell
+// and element loads is what the kernel takes, and eight lanes share it.
+constexpr int EIGHT_LANE_QUERIES = 30000;
+template <int L>
 __global__ void __launch_bounds__(128) k_elem_items(BuildArgs A, OneRep P, int2 *items, int *nitems, int icap,
                                                     int *work, int *nwork) {
-  elem_items_slot(A, P, items, nitems, icap, work, nwork);
+  elem_items_slot<L>(A, P, items, nitems, icap, work, nwork);
 }
+template <int L>
 __global__ void __launch_bounds__(128, 8) k_elem_items(BuildArgs A, ManyRep P, int2 *items, int *nitems, int icap,
                                                        int *work, int *nwork) {
-  elem_items_slot(A, P, items, nitems, icap, work, nwork);
+  elem_items_slot<L>(A, P, items, nitems, icap, work, nwork);
 }
 
 // Phase B for atoms: one warp per listed atom, its element sites appended
@@ -1312,16 +1418,62 @@ __global__ void __launch_bounds__(128, 8) k_build_gauss(BuildArgs A, RP P, const
 
 // ------------------------------------------------------------- compaction
 
-__global__ void k_act_table(const int *flag, const int *pref, int ngid, int ne, int nsi, int *act_gid,
-                            int *act_off, int *nact, int *too_many) {
-  int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid < ngid && flag[gid]) act_gid[pref[gid]] = gid;
-  if (gid < ne) act_off[gid] = pref[gid * NU];
-  if (gid == 0) {
-    act_off[ne] = pref[ngid];
-    *nact = pref[ngid];
-    if ((long)nsi + pref[ngid] >= (1L << (31 - IMG_BITS))) *too_many = 1;
+// The table of marked sites, one warp per element: its marks become words of
+// bits, each with the rank of its first site, and its sites get consecutive
+// ranks.  Elements take their ranges from a counter, a block at a time, so
+// their order in the table may differ from one rebuild to the next; nothing
+// depends on it.
+__global__ void __launch_bounds__(256) k_act_table(const unsigned char *flag, int ne, int nsi, uint2 *words, int *act_gid,
+                                                   int *nact, int *too_many) {
+  __shared__ int total[8], base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = blockIdx.x * 8 + warp;
+  unsigned word = 0;
+  if (e < ne) {
+    const unsigned char *f = flag + (size_t)e * MARKS;
+#pragma unroll
+    for (int w = 0; w < MARK_WORDS; w++) {
+      const unsigned b = __ballot_sync(0xffffffffu, f[32 * w + lane] != 0);
+      if (lane == w) word = b;
+    }
   }
+  int incl = __popc(word);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) total[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int n = 0;
+    for (int w = 0; w < 8; w++) {
+      const int t = total[w];
+      total[w] = n;
+      n += t;
+    }
+    base = atomicAdd(nact, n);
+    if ((long)nsi + base + n >= (1L << (31 - IMG_BITS))) *too_many = 1;
+  }
+  __syncthreads();
+  if (e >= ne) return;
+  const int first = base + total[warp] + incl - __popc(word);
+  if (lane < MARK_WORDS) words[(size_t)e * MARK_WORDS + lane] = make_uint2(word, first);
+#pragma unroll 1
+  for (int w = 0; w < MARK_WORDS; w++) {
+    const unsigned b = __shfl_sync(0xffffffffu, word, w);
+    const int r = __shfl_sync(0xffffffffu, first, w);
+    if ((b >> lane) & 1u) act_gid[r + __popc(b & lanemask_lt())] = e * NU + 32 * w + lane;
+  }
+}
+
+// Pair-table index of lattice site gid (Gauss points at their fixed place, the
+// other sites by rank among the marked ones).
+__device__ __forceinline__ int site_index(int gid, const uint2 *words, int na, int ne) {
+  const int e = gid / NU, u = gid % NU, g = site_gauss(u);
+  if (g >= 0) return na + NG * e + g;
+  const uint2 w = words[(size_t)e * MARK_WORDS + (u >> 5)];
+  return na + NG * ne + (int)w.y + __popc(w.x & ((1u << (u & 31)) - 1u));
 }
 
 // Packs each entry as (pair-table index << 5 | image code): atoms by their
@@ -1332,7 +1484,7 @@ __global__ void k_act_table(const int *flag, const int *pref, int ngid, int ne, 
 // margin since the build, every pair inside the cutoff lies in that prefix,
 // in the same order, so the pair loops may stop there with identical sums.
 __global__ void k_remap(const int *raw, const unsigned char *img, const int *num, int nsi, int cap,
-                        const int *pref, const int *atom_slot, int na, int ne, int *out, int *num_in) {
+                        const uint2 *words, const int *atom_slot, int na, int ne, int *out, int *num_in) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nsi) return;
   int n = min(num[i], cap);
@@ -1346,10 +1498,7 @@ __global__ void k_remap(const int *raw, const unsigned char *img, const int *num
     int v = raw[o];
     int sidx;
     if (v & KIND_SITE) {
-      int gid = v & ~KIND_SITE;
-      int e = gid / NU, u = gid % NU;
-      int g = site_gauss(u);
-      sidx = (g >= 0) ? na + NG * e + g : na + NG * ne + pref[gid];
+      sidx = site_index(v & ~KIND_SITE, words, na, ne);
     } else {
       sidx = atom_slot[v];
     }
@@ -1360,25 +1509,26 @@ __global__ void k_remap(const int *raw, const unsigned char *img, const int *num
 
 // Converts the element-site entries of the full lists (rows site_from.x ..
 // num_in - 1 of the front segment, cap - back .. cap - 1 - site_from.y of the
-// back one) from lattice-site ids to pair-table indices: Gauss points at
-// their fixed place, the other sites by their rank among the marked ones.
-__global__ void k_remap_sites(const int *raw, const unsigned char *img, const int *num, const int *num_in,
-                              const int2 *site_from, int nsi, int cap, const int *pref, int na, int ne, int *out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsi) return;
-  const int nin = num_in[i], nback = num[i] - nin;
-  if (nin + nback > cap) return;   // overflow: the build is repeated
-  const int2 from = site_from[i];
-  auto one = [&](int row) {
-    const size_t o = (size_t)row * nsi + i;
-    const int gid = raw[o] & ~KIND_SITE;
-    const int e = gid / NU, u = gid % NU;
-    const int g = site_gauss(u);
-    const int sidx = (g >= 0) ? na + NG * e + g : na + NG * ne + pref[gid];
-    out[o] = (sidx << IMG_BITS) | img[o];
-  };
-  for (int k = from.x; k < nin; k++) one(k);
-  for (int k = from.y; k < nback; k++) one(cap - 1 - k);
+// back one) from lattice-site ids to pair-table indices.  Only Gauss points and
+// the atoms of the work list have any; a site's rows are shared by the 8
+// threads of a column (x: sites, y: rows).
+__global__ void __launch_bounds__(256) k_remap_sites(const int *raw, const unsigned char *img, const int *num,
+                                                     const int *num_in, const int2 *site_from, int nsi, int cap,
+                                                     const uint2 *words, int na, int ne, const int *work,
+                                                     const int *nwork, int *out) {
+  const int n = NG * ne + *nwork;
+  for (int d = blockIdx.x * 32 + threadIdx.x; d < n; d += gridDim.x * 32) {
+    const int i = d < NG * ne ? na + d : work[d - NG * ne];
+    const int nin = num_in[i], nback = num[i] - nin;
+    if (nin + nback > cap) continue;   // overflow: the build is repeated
+    const int2 from = site_from[i];
+    auto one = [&](int row) {
+      const size_t o = (size_t)row * nsi + i;
+      out[o] = (site_index(raw[o] & ~KIND_SITE, words, na, ne) << IMG_BITS) | img[o];
+    };
+    for (int k = from.x + threadIdx.y; k < nin; k += 8) one(k);
+    for (int k = from.y + threadIdx.y; k < nback; k += 8) one(cap - 1 - k);
+  }
 }
 
 inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
@@ -1471,9 +1621,10 @@ void neigh_plan(Ctx &c, bool want_half) {
   std::vector<unsigned long long> bits(c.nrep, 0);
   if (c.ne) {
     with_reps(c, [&](auto P) {
-      if (c.na) k_pbc_atoms<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P);
-      k_elem_geom<<<nblk(c.ne, 128), 128, 0, c.stream>>>(c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
-                                                         c.reach_bits.p, c.overflow.p + 3);
+      if (c.na) k_pbc_atoms<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P, BuildStart{});
+      k_elem_geom<<<nblk(c.ne, 64), 64, 0, c.stream>>>(c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
+                                                       c.reach_bits.p, c.overflow.p + 3, (double *)nullptr,
+                                                       (float *)nullptr);
     });
     stream_copy(c, bits.data(), c.reach_bits.p, sizeof(unsigned long long) * c.nrep, cudaMemcpyDeviceToHost);
   }
@@ -1533,6 +1684,7 @@ void neigh_plan(Ctx &c, bool want_half) {
   c.ecell_near.reserve(c.egrid.ncell + 1);
   c.acell_near.reserve(c.agrid.ncell + 1);
   c.ecell_elems.reserve(std::max(c.ne, 1));
+  c.ecell_sphere.reserve(std::max(c.ne, 1));
   size_t slots = (size_t)c.cap * std::max(nsi, 1);
   c.raw_full.reserve(slots);
   c.img_full.reserve(slots);
@@ -1549,10 +1701,9 @@ void neigh_plan(Ctx &c, bool want_half) {
   c.nitems.reserve(std::max(nsi, 1));
   c.atom_work.reserve(std::max(c.na, 1));
   c.atom_nwork.reserve(1);
-  c.site_flag.reserve(ngid + 1);
-  c.site_pref.reserve(ngid + 1);
+  c.site_flag.reserve((size_t)std::max(c.ne, 1) * MARKS);
+  c.site_words.reserve((size_t)std::max(c.ne, 1) * MARK_WORDS);
   c.act_gid.reserve(std::max<size_t>(ngid, 1));
-  c.act_off.reserve(c.ne + 1);
   // site table for every lattice site active, keeping the atom positions
   size_t ns_cap = (size_t)nsi + ngid;
   if (ns_cap > c.xs.n) {
@@ -1579,8 +1730,6 @@ void neigh_plan(Ctx &c, bool want_half) {
   need = std::max(need, bytes);
   cub::DeviceRadixSort::SortPairs(nullptr, bytes, c.cell_key.p, c.cell_key2.p, c.idx_tmp.p, c.ecell_elems.p,
                                   std::max(c.ne, 1), 0, bits_e, c.stream);
-  need = std::max(need, bytes);
-  cub::DeviceScan::ExclusiveSum(nullptr, bytes, c.site_flag.p, c.site_pref.p, (int)(ngid + 1), c.stream);
   need = std::max(need, bytes);
   c.cub_tmp.reserve(need);
   c.cub_bytes = need;
@@ -1609,29 +1758,21 @@ void neigh_build_async(Ctx &c, bool want_half) {
   if (!c.planned || c.plan_na != c.na || c.plan_ne != c.ne || (want_half && !c.plan_half))
     throw Error(CACB200_ESTATE, "rebuild without a capacity plan");
   const int nsi = c.nsite_i();
-  const size_t ngid = (size_t)c.ne * NU;
-  CACB200_CUDA(cudaMemsetAsync(c.overflow.p, 0, 4 * sizeof(int), c.stream));
-  CACB200_CUDA(cudaMemsetAsync(c.overflow.p + 8, 0, 2 * sizeof(int), c.stream));
   with_reps(c, [&](auto P) {
     {
       KernelTimer t(c, "pbc_geom");
-      if (c.na) k_pbc_atoms<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P);
+      // the positions these lists are built from are kept for the displacement
+      // test of the inner prefix, which is usable until a site has moved far
+      const BuildStart S{c.xbuild.p, c.disp.p,       c.inner_ok.p, inner_limit(c) > 0.0 ? 1 : 0, c.dmax.p,
+                         c.overflow.p, c.dev_nact.p, c.atom_nwork.p, c.sm_counter.p,
+                         c.nrep,       c.num_sms};
+      const int n = std::max(std::max(c.na, c.nrep), c.num_sms);
+      k_pbc_atoms<<<nblk(n, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P, S);
       if (c.ne)
-        k_elem_geom<<<nblk(c.ne, 128), 128, 0, c.stream>>>(c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
-                                                           c.reach_bits.p, c.overflow.p + 3);
+        k_elem_geom<<<nblk(c.ne, 64), 64, 0, c.stream>>>(c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
+                                                         c.reach_bits.p, c.overflow.p + 3, c.nodex_build.p,
+                                                         c.edisp.p);
     }
-    // the positions these lists are built from, for the displacement test of
-    // the inner prefix; the prefix is usable until a site moves half the margin
-    if (c.na)
-      CACB200_CUDA(cudaMemcpyAsync(c.xbuild.p, c.xs.p, sizeof(double4) * c.na, cudaMemcpyDeviceToDevice, c.stream));
-    if (c.ne)
-      CACB200_CUDA(cudaMemcpyAsync(c.nodex_build.p, c.nodex.p, sizeof(double) * 24 * c.ne,
-                                   cudaMemcpyDeviceToDevice, c.stream));
-    CACB200_CUDA(cudaMemsetAsync(c.inner_ok.p, inner_limit(c) > 0.0 ? 1 : 0, sizeof(int) * c.nrep, c.stream));
-    // every site is where the lists are built from
-    if (c.na) CACB200_CUDA(cudaMemsetAsync(c.disp.p, 0, sizeof(float) * c.na, c.stream));
-    if (c.ne) CACB200_CUDA(cudaMemsetAsync(c.edisp.p, 0, sizeof(float) * c.ne, c.stream));
-    CACB200_CUDA(cudaMemsetAsync(c.dmax.p, 0, sizeof(unsigned) * c.nrep, c.stream));
     {
       KernelTimer t(c, "bin");
       size_t bytes = c.cub_bytes;
@@ -1659,6 +1800,8 @@ void neigh_build_async(Ctx &c, bool want_half) {
                                                      c.stream));
         k_cell_start<<<nblk(c.egrid.ncell + 1, 256), 256, 0, c.stream>>>(c.cell_key2.p, c.ne, c.egrid.ncell,
                                                                         c.ecell_start.p);
+        k_gather_spheres<<<nblk(c.ne, 256), 256, 0, c.stream>>>(c.ecenter.p, c.eframe.p, c.ecell_elems.p, c.ne,
+                                                                c.ecell_sphere.p);
         if (c.nrep == 1)
           k_ecell_near<<<nblk(c.egrid.ncell, 256), 256, 0, c.stream>>>(c.ecell_start.p, c.rep_h[0].eg,
                                                                        c.ecell_near.p);
@@ -1681,9 +1824,10 @@ void neigh_build_async(Ctx &c, bool want_half) {
     A.ecell_near = (c.nrep == 1 && c.ne) ? c.ecell_near.p : nullptr;
     A.acell_near = (c.nrep == 1 && c.na && c.ne) ? c.acell_near.p : nullptr;
     A.ecell_elems = c.ecell_elems.p;
+    A.ecell_sphere = c.ecell_sphere.p;
     A.atom_of_slot = c.slot_atom.p;
     A.site_flag = c.site_flag.p;
-    if (ngid) CACB200_CUDA(cudaMemsetAsync(c.site_flag.p, 0, sizeof(int) * (ngid + 1), c.stream));
+    if (c.ne) CACB200_CUDA(cudaMemsetAsync(c.site_flag.p, 0, (size_t)c.ne * MARKS, c.stream));
     A.na = c.na;
     A.ne = c.ne;
     A.nsi = nsi;
@@ -1717,9 +1861,12 @@ void neigh_build_async(Ctx &c, bool want_half) {
     if (c.ne) {
       {
         KernelTimer t(c, "build_items");
-        CACB200_CUDA(cudaMemsetAsync(c.atom_nwork.p, 0, sizeof(int), es));
-        k_elem_items<<<nblk(nsi, 128), 128, 0, es>>>(A, P, c.items.p, c.nitems.p, c.item_cap, c.atom_work.p,
-                                                    c.atom_nwork.p);
+        if (nsi < EIGHT_LANE_QUERIES)
+          k_elem_items<8><<<nblk(8L * nsi, 128), 128, 0, es>>>(A, P, c.items.p, c.nitems.p, c.item_cap,
+                                                               c.atom_work.p, c.atom_nwork.p);
+        else
+          k_elem_items<1><<<nblk(nsi, 128), 128, 0, es>>>(A, P, c.items.p, c.nitems.p, c.item_cap, c.atom_work.p,
+                                                          c.atom_nwork.p);
       }
       if (split) CACB200_CUDA(cudaEventRecord(c.items_ev, c.side));
       {
@@ -1743,7 +1890,6 @@ void neigh_build_async(Ctx &c, bool want_half) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_build_atoms_sm, 32, 0);
             return b > 0 ? b : 1;
           }();
-          CACB200_CUDA(cudaMemsetAsync(c.sm_counter.p, 0, sizeof(int) * c.num_sms, c.stream));
           k_build_atoms_sm<<<per_sm * c.num_sms, 32, 0, c.stream>>>(A, P, nchunk, c.sm_counter.p, c.num_sms);
           done = true;
         }
@@ -1767,21 +1913,17 @@ void neigh_build_async(Ctx &c, bool want_half) {
   });
   {
     KernelTimer t(c, "compact");
-    int *flag = c.site_flag.p;
-    int *pref = c.site_pref.p;
-    if (ngid) {
-      size_t bytes = c.cub_bytes;
-      CACB200_CUDA(cub::DeviceScan::ExclusiveSum(c.cub_tmp.p, bytes, flag, pref, (int)(ngid + 1), c.stream));
-      k_act_table<<<nblk((long)ngid, 256), 256, 0, c.stream>>>(flag, pref, (int)ngid, c.ne, nsi, c.act_gid.p,
-                                                              c.act_off.p, c.dev_nact.p, c.overflow.p + 7);
+    if (c.ne) {
+      k_act_table<<<nblk(c.ne, 8), 256, 0, c.stream>>>(c.site_flag.p, c.ne, nsi, c.site_words.p, c.act_gid.p,
+                                                       c.dev_nact.p, c.overflow.p + 7);
+      const int grid = (int)std::min<long>(nblk((long)NG * c.ne + c.na, 32), (long)8 * c.num_sms);
+      k_remap_sites<<<grid, dim3(32, 8), 0, c.stream>>>(c.raw_full.p, c.img_full.p, c.num_full.p, c.num_in.p,
+                                                        c.site_from.p, nsi, c.cap, c.site_words.p, c.na, c.ne,
+                                                        c.atom_work.p, c.atom_nwork.p, c.nbr_full.p);
     }
-    if (c.ne)
-      k_remap_sites<<<nblk(nsi, 256), 256, 0, c.stream>>>(c.raw_full.p, c.img_full.p, c.num_full.p, c.num_in.p,
-                                                         c.site_from.p, nsi, c.cap, pref, c.na, c.ne,
-                                                         c.nbr_full.p);
     if (want_half)
-      k_remap<<<nblk(nsi, 256), 256, 0, c.stream>>>(c.raw_half.p, c.img_half.p, c.num_half.p, nsi, c.cap, pref,
-                                                     c.atom_slot.p, c.na, c.ne, c.nbr_half.p, nullptr);
+      k_remap<<<nblk(nsi, 256), 256, 0, c.stream>>>(c.raw_half.p, c.img_half.p, c.num_half.p, nsi, c.cap,
+                                                     c.site_words.p, c.atom_slot.p, c.na, c.ne, c.nbr_half.p, nullptr);
   }
   c.have_half = want_half;
   c.lists_valid = true;

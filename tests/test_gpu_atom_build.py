@@ -42,3 +42,30 @@ def test_lists_equal_the_restatement(shape, oracle_mod):
     assert np.array_equal(e.neighbor_list(), want[False])
     assert np.array_equal(e.neighbor_list(half=True), want[True])
     e.close()
+
+
+@pytest.mark.parametrize("copies,na", [(1, 1458), (6, 1458), (6, 0), (6, 40000)])
+def test_element_walk_with_crowded_cells(copies, na, oracle_mod):
+    """Elements lying over one another, so that an element cell holds more than
+    32 of them (36 with six copies), for both forms of the element walk (eight
+    lanes a query below 30,000 queries)."""
+    from cac_b200.api import Engine
+    s = gen.build_slab(3, 1, 1, 3, temperature=300.0, seed=4)
+    rng = np.random.default_rng(9)
+    s.nodex = np.concatenate([s.nodex + rng.uniform(-0.5, 0.5, (1, 1, 3)) for _ in range(copies)])
+    s.nodev = np.concatenate([s.nodev] * copies)
+    if na > s.natoms:      # more atoms, anywhere
+        s.x = np.concatenate([s.x, rng.uniform(s.boxlo, s.boxhi, (na - s.natoms, 3))])
+        s.v = np.zeros_like(s.x)
+    s.x, s.v = s.x[:na].copy(), s.v[:na].copy()
+    gen.wrap_into_box(s)
+    cut = 3.0 if na < 40000 else 0.6
+    st = oracle_mod.OracleState(s)
+    want = oracle_mod.build_list(st, cut + 0.4, False).canonical(s.natoms)
+    e = Engine(0)
+    e.upload(s)
+    e.pair_lj(0.4093, 2.338, cut)
+    e.neighbor(0.4, 10)
+    e.build_lists()
+    assert np.array_equal(e.neighbor_list(), want)
+    e.close()
