@@ -235,7 +235,7 @@ struct Ctx {
   DBuf<int> acell_of;            // [na] cell of each sorted atom
   DBuf<int> ecell_start, ecell_elems;
   DBuf<double4> ecell_sphere;    // [ne] candidate spheres of the sorted elements
-  DBuf<int> cell_key, cell_key2, idx_tmp;
+  DBuf<int> atom_key, atom_place, atom_order, elem_key, elem_place, elem_order, cell_count;   // binning
   DBuf<int> atom_work, atom_nwork;   // atoms with element sites in reach (rebuild work list)
   DBuf<int2> items;                  // [slots][item_cap] element boxes to test, per query
   DBuf<int> nitems;                  // [slots]
@@ -253,7 +253,6 @@ struct Ctx {
   DBuf<double4> xss;
   DBuf<unsigned char> cub_tmp;
   size_t cub_bytes = 0;
-  int sort_bits_a = 1, sort_bits_e = 1;
   double reach_budget = 0.0;
   bool planned = false, plan_half = false;
   int plan_na = -1, plan_ne = -1;

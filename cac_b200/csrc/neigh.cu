@@ -83,6 +83,16 @@ struct ManyRep {
 
 // ------------------------------------------------------------------ pbc
 
+__device__ __forceinline__ int grid_cell(const Grid &g, const BoxD &b, const double *w) {
+  int c[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    int v = (int)((w[d] - b.lo[d]) * g.inv[d]);
+    c[d] = min(max(v, 0), g.nc[d] - 1);
+  }
+  return (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
+}
+
 // What a rebuild starts from, cleared by its first kernel.
 struct BuildStart {
   double4 *xbuild;      // the wrapped positions the lists are built from (null: only wrap)
@@ -92,6 +102,7 @@ struct BuildStart {
   unsigned *dmax;       // [nrep]
   int *overflow, *nact, *nwork, *sm_counter;
   int nrep, nsm;
+  int *key, *place, *count;   // per atom: its cell and its place among the cell's arrivals; atoms per cell
 };
 
 // Domain::pbc for owned atoms (domain.cpp:562-630), and the clearing of the
@@ -131,6 +142,10 @@ __global__ void k_pbc_atoms(double4 *xs, int na, RP P, BuildStart S) {
   if (S.xbuild) {
     S.xbuild[i] = p;
     S.disp[i] = 0.0f;
+    const Rep r = P.site(i);
+    const int c = r.abase + grid_cell(r.ag, r.b, q);
+    S.key[i] = c;
+    S.place[i] = atomicAdd(S.count + c, 1);
   }
 }
 
@@ -150,7 +165,8 @@ constexpr int EFR = 28;
 
 template <class RP>
 __global__ void k_elem_geom(double *nodex, int ne, RP P, double4 *ecenter, double *eframe,
-                            unsigned long long *reach_bits, int *grew, double *nodex_build, float *edisp) {
+                            unsigned long long *reach_bits, int *grew, double *nodex_build, float *edisp, int *key,
+                            int *place, int *count) {
   int e = blockIdx.x * blockDim.x + threadIdx.x;
   double reach = 0.0;
   if (e < ne) {
@@ -243,6 +259,9 @@ __global__ void k_elem_geom(double *nodex, int ne, RP P, double4 *ecenter, doubl
     if (nodex_build) {   // the nodes the lists are built from
       for (int k = 0; k < 24; k++) nodex_build[(size_t)e * 24 + k] = nx[k];
       edisp[e] = 0.0f;
+      const int k = rp.ebase + grid_cell(rp.eg, b, c);
+      key[e] = k;
+      place[e] = atomicAdd(count + k, 1);
     }
     reach = R + dmax;
     if (!(reach <= rp.reach_budget)) atomicExch(grew, 1);
@@ -257,44 +276,68 @@ __global__ void k_elem_geom(double *nodex, int ne, RP P, double4 *ecenter, doubl
 
 // ---------------------------------------------------------------- binning
 
-__device__ __forceinline__ int grid_cell(const Grid &g, const BoxD &b, const double *w) {
-  int c[3];
+// Binning is a counting sort: the kernels above count the arrivals of each
+// cell, a scan turns the counts into the cells' first places, each atom (and
+// element) is put at its cell's first place plus its order of arrival, and
+// there takes the place that its index has among the cell's members, so the
+// order is that of a stable sort by cell whatever the order of arrival was.
+// Few launches (a radix sort takes about a dozen for atoms and elements, which
+// is what small systems waited for), and no keys to move.
+
+// Exclusive scan of the atom cells' counts and of the element cells', each
+// with its total behind (one block; larger grids use CUB).
+constexpr int SCAN_CELLS = 16384;
+__global__ void __launch_bounds__(1024) k_scan_cells(const int *count, int na_cell, int ne_cell, int *astart, int *estart) {
+  __shared__ int warp_sum[32];
+  __shared__ int carry, atoms;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = na_cell + ne_cell;
+  if (threadIdx.x == 0) carry = 0;
+  if (threadIdx.x == 0 && na_cell == 0) atoms = 0;
+  for (int base = 0; base < n; base += 4096) {
+    const int i0 = base + 4 * threadIdx.x;
+    int v[4], sum = 0;
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    int v = (int)((w[d] - b.lo[d]) * g.inv[d]);
-    c[d] = min(max(v, 0), g.nc[d] - 1);
+    for (int u = 0; u < 4; u++) {
+      v[u] = i0 + u < n ? count[i0 + u] : 0;
+      sum += v[u];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    __syncthreads();   // the last round's warp_sum and carry have been read
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    int before = carry;
+    for (int w = 0; w < warp; w++) before += warp_sum[w];
+    int at = before + incl - sum;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int i = i0 + u;
+      if (i < na_cell) astart[i] = at;
+      else if (i < n) estart[i - na_cell] = at;
+      at += v[u];
+      if (i == na_cell - 1) atoms = at;
+    }
+    __syncthreads();
+    if (threadIdx.x == 1023) carry = before + incl;
   }
-  return (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
-}
-
-template <class RP>
-__global__ void k_atom_keys(const double4 *xs, int na, RP P, int *key, int *idx) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= na) return;
-  const Rep r = P.site(i);
-  double4 p = xs[i];
-  double w[3] = {p.x, p.y, p.z};
-  key[i] = r.abase + grid_cell(r.ag, r.b, w);
-  idx[i] = i;
-}
-
-template <class RP>
-__global__ void k_elem_keys(const double4 *ecenter, int ne, RP P, int *key, int *idx) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const Rep r = P.elem(e);
-  double4 p = ecenter[e];
-  double w[3] = {p.x, p.y, p.z};
-  key[e] = r.ebase + grid_cell(r.eg, r.b, w);
-  idx[e] = e;
+  __syncthreads();
+  // element places count from their own zero
+  const int a = atoms;
+  for (int i = threadIdx.x; i < ne_cell; i += 1024) estart[i] -= a;
+  if (threadIdx.x == 0) {
+    astart[na_cell] = a;
+    estart[ne_cell] = carry - a;
+  }
 }
 
 // near[c]: some cell of the 27-cell block around cell c (a single system's
 // grid, periodic) holds an entry (element grid: an element; atom grid: an
 // atom)
-__global__ void k_ecell_near(const int *start, Grid g, unsigned char *near) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= g.ncell) return;
+__device__ __forceinline__ void near_cell(int c, const int *start, const Grid &g, unsigned char *near) {
   const int cx = c % g.nc[0], cy = (c / g.nc[0]) % g.nc[1], cz = c / (g.nc[0] * g.nc[1]);
   bool any = false;
   for (int oz = -1; oz <= 1 && !any; oz++)
@@ -308,29 +351,43 @@ __global__ void k_ecell_near(const int *start, Grid g, unsigned char *near) {
   near[c] = any ? 1 : 0;
 }
 
-// cell_start[c] = first sorted position with key >= c, for c in [0, ncell]
-// (lower bound by binary search, one thread per cell)
-__global__ void k_cell_start(const int *skey, int n, int ncell, int *start) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > ncell) return;
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (skey[mid] < c) lo = mid + 1;
-    else hi = mid;
+struct BinArgs {
+  const int *akey, *aplace, *astart, *ekey, *eplace, *estart;
+  int *aorder, *eorder;             // members of each cell in order of arrival
+  int na, ne;
+  unsigned char *anear, *enear;     // single systems with elements (else null)
+  Grid ag, eg;
+};
+
+// Atoms and elements to their cells; the cells' near flags.
+__global__ void k_scatter(BinArgs B) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < B.na) {
+    B.aorder[B.astart[B.akey[i]] + B.aplace[i]] = i;
+    return;
   }
-  start[c] = lo;
+  i -= B.na;
+  if (i < B.ne) {
+    B.eorder[B.estart[B.ekey[i]] + B.eplace[i]] = i;
+    return;
+  }
+  i -= B.ne;
+  if (!B.enear) return;
+  if (i < B.eg.ncell) {
+    near_cell(i, B.estart, B.eg, B.enear);
+    return;
+  }
+  i -= B.eg.ncell;
+  if (i < B.ag.ncell) near_cell(i, B.astart, B.ag, B.anear);
 }
 
-// The sorted elements' candidate spheres: centre, and reach of the sites
-// (radius + deviation from affine) in w.
-__global__ void k_gather_spheres(const double4 *ecenter, const double *eframe, const int *sidx, int n, double4 *out) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const int e = sidx[k];
-  double4 c = ecenter[e];
-  c.w += eframe[(size_t)e * EFR + 12];
-  out[k] = c;
+// The place of member i of a cell: its first place plus the members of
+// smaller index.
+__device__ __forceinline__ int cell_place(const int *start, const int *order, int cell, int i) {
+  const int beg = start[cell], end = start[cell + 1];
+  int r = 0;
+  for (int k = beg; k < end; k++) r += order[k] < i;
+  return beg + r;
 }
 
 // Fixed-point copy of a wrapped atom position for the screen of the atom build: quanta of
@@ -343,31 +400,43 @@ constexpr float QUANTUM = 1.0f / 1048576.0f;
 __device__ __forceinline__ int fix20(double x) { return (int)(unsigned)(unsigned long long)__double2ll_rn(x * 1048576.0); }
 
 // The sorted atoms: positions (w = atom index), the fixed-point copies of the
-// screen (x, y, z parts n apart), slots and cells.
+// screen (x, y, z parts na apart), slots and cells; and the sorted elements
+// with their candidate spheres (centre, and reach of the sites -- radius +
+// deviation from affine -- in w).
 template <class RP>
-__global__ void k_gather_pos(const double4 *xs, const int *sidx, const int *skey, int n, RP P, double4 *out,
-                             int *fixed, int *atom_slot, int *slot_cell) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  int i = sidx[k];
-  atom_slot[i] = k;
-  slot_cell[k] = skey[k];
-  double4 p = xs[i];
-  const BoxD b = P.site(i).b;
-  const double q[3] = {p.x, p.y, p.z};
-  int f[3];
-  bool near = true;
+__global__ void k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *fixed, int *slot_atom, int *atom_slot,
+                        int *slot_cell, const double4 *ecenter, const double *eframe, int *elems, double4 *spheres) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < B.na) {
+    const int cell = B.akey[i], k = cell_place(B.astart, B.aorder, cell, i);
+    slot_atom[k] = i;
+    atom_slot[i] = k;
+    slot_cell[k] = cell;
+    double4 p = xs[i];
+    const BoxD b = P.site(i).b;
+    const double q[3] = {p.x, p.y, p.z};
+    int f[3];
+    bool near = true;
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    near = near && q[d] >= b.lo[d] - b.L[d] && q[d] <= b.hi[d] + b.L[d];
-    f[d] = fix20(q[d] - b.lo[d]);
+    for (int d = 0; d < 3; d++) {
+      near = near && q[d] >= b.lo[d] - b.L[d] && q[d] <= b.hi[d] + b.L[d];
+      f[d] = fix20(q[d] - b.lo[d]);
+    }
+    if (f[0] == FAR_ATOM) f[0]++;
+    fixed[k] = near ? f[0] : FAR_ATOM;
+    fixed[k + (size_t)B.na] = f[1];
+    fixed[k + 2 * (size_t)B.na] = f[2];
+    p.w = __longlong_as_double((long long)i);
+    out[k] = p;
+    return;
   }
-  if (f[0] == FAR_ATOM) f[0]++;
-  fixed[k] = near ? f[0] : FAR_ATOM;
-  fixed[k + (size_t)n] = f[1];
-  fixed[k + 2 * (size_t)n] = f[2];
-  p.w = __longlong_as_double((long long)i);
-  out[k] = p;
+  i -= B.na;
+  if (i >= B.ne) return;
+  const int k = cell_place(B.estart, B.eorder, B.ekey[i], i);
+  elems[k] = i;
+  double4 c = ecenter[i];
+  c.w += eframe[(size_t)i * EFR + 12];
+  spheres[k] = c;
 }
 
 // -------------------------------------------------------------- the build
@@ -1623,8 +1692,8 @@ void neigh_plan(Ctx &c, bool want_half) {
     with_reps(c, [&](auto P) {
       if (c.na) k_pbc_atoms<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P, BuildStart{});
       k_elem_geom<<<nblk(c.ne, 64), 64, 0, c.stream>>>(c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
-                                                       c.reach_bits.p, c.overflow.p + 3, (double *)nullptr,
-                                                       (float *)nullptr);
+                                                       c.reach_bits.p, c.overflow.p + 3, nullptr, nullptr, nullptr,
+                                                       nullptr, nullptr);
     });
     stream_copy(c, bits.data(), c.reach_bits.p, sizeof(unsigned long long) * c.nrep, cudaMemcpyDeviceToHost);
   }
@@ -1670,9 +1739,13 @@ void neigh_plan(Ctx &c, bool want_half) {
   const int nsi = c.nsite_i();
   const size_t ngid = (size_t)c.ne * NU;
   int nmax = std::max(std::max(c.na, c.ne), 1);
-  c.cell_key.reserve(nmax);
-  c.cell_key2.reserve(nmax);
-  c.idx_tmp.reserve(nmax);
+  c.atom_key.reserve(std::max(c.na, 1));
+  c.atom_place.reserve(std::max(c.na, 1));
+  c.atom_order.reserve(std::max(c.na, 1));
+  c.elem_key.reserve(std::max(c.ne, 1));
+  c.elem_place.reserve(std::max(c.ne, 1));
+  c.elem_order.reserve(std::max(c.ne, 1));
+  c.cell_count.reserve((size_t)c.agrid.ncell + c.egrid.ncell + 2);
   c.slot_atom.reserve(nmax);
   c.atom_slot.reserve(std::max(c.na, 1));
   c.xss.reserve(std::max(c.xs.n, (size_t)1));
@@ -1720,21 +1793,14 @@ void neigh_plan(Ctx &c, bool want_half) {
     c.xs.n = ns_cap;
   }
   c.ns_cap = ns_cap;
-  // CUB temporary storage for the largest sort and the scan
+  // CUB temporary storage of the cell scans
   size_t need = 0, bytes = 0;
-  int bits_a = 1, bits_e = 1;
-  while ((1 << bits_a) <= c.agrid.ncell && bits_a < 31) bits_a++;
-  while ((1 << bits_e) <= c.egrid.ncell && bits_e < 31) bits_e++;
-  cub::DeviceRadixSort::SortPairs(nullptr, bytes, c.cell_key.p, c.cell_key2.p, c.idx_tmp.p, c.slot_atom.p,
-                                  std::max(c.na, 1), 0, bits_a, c.stream);
+  cub::DeviceScan::ExclusiveSum(nullptr, bytes, c.cell_count.p, c.acell_start.p, c.agrid.ncell + 1, c.stream);
+  need = bytes;
+  cub::DeviceScan::ExclusiveSum(nullptr, bytes, c.cell_count.p, c.ecell_start.p, c.egrid.ncell + 1, c.stream);
   need = std::max(need, bytes);
-  cub::DeviceRadixSort::SortPairs(nullptr, bytes, c.cell_key.p, c.cell_key2.p, c.idx_tmp.p, c.ecell_elems.p,
-                                  std::max(c.ne, 1), 0, bits_e, c.stream);
-  need = std::max(need, bytes);
-  c.cub_tmp.reserve(need);
+  c.cub_tmp.reserve(std::max<size_t>(need, 1));
   c.cub_bytes = need;
-  c.sort_bits_a = bits_a;
-  c.sort_bits_e = bits_e;
   c.plan_half = want_half;
   c.planned = true;
   const long gen_before = c.gen;
@@ -1765,49 +1831,43 @@ void neigh_build_async(Ctx &c, bool want_half) {
       // test of the inner prefix, which is usable until a site has moved far
       const BuildStart S{c.xbuild.p, c.disp.p,       c.inner_ok.p, inner_limit(c) > 0.0 ? 1 : 0, c.dmax.p,
                          c.overflow.p, c.dev_nact.p, c.atom_nwork.p, c.sm_counter.p,
-                         c.nrep,       c.num_sms};
+                         c.nrep,       c.num_sms,    c.atom_key.p,     c.atom_place.p, c.cell_count.p};
+      // counts of the atom cells, one more, then of the element cells and one
+      // more (the single-block scan needs no gap: its element counts follow)
+      const bool small = c.agrid.ncell + (c.ne ? c.egrid.ncell : 0) <= SCAN_CELLS;
+      int *const ecount = c.cell_count.p + c.agrid.ncell + (small ? 0 : 1);
+      CACB200_CUDA(cudaMemsetAsync(c.cell_count.p, 0, sizeof(int) * ((size_t)c.agrid.ncell + c.egrid.ncell + 2),
+                                   c.stream));
       const int n = std::max(std::max(c.na, c.nrep), c.num_sms);
       k_pbc_atoms<<<nblk(n, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P, S);
       if (c.ne)
         k_elem_geom<<<nblk(c.ne, 64), 64, 0, c.stream>>>(c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
                                                          c.reach_bits.p, c.overflow.p + 3, c.nodex_build.p,
-                                                         c.edisp.p);
+                                                         c.edisp.p, c.elem_key.p, c.elem_place.p, ecount);
     }
     {
       KernelTimer t(c, "bin");
-      size_t bytes = c.cub_bytes;
-      if (c.na) {
-        k_atom_keys<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P, c.cell_key.p, c.idx_tmp.p);
-        CACB200_CUDA(cub::DeviceRadixSort::SortPairs(c.cub_tmp.p, bytes, c.cell_key.p, c.cell_key2.p,
-                                                     c.idx_tmp.p, c.slot_atom.p, c.na, 0, c.sort_bits_a,
-                                                     c.stream));
-        k_cell_start<<<nblk(c.agrid.ncell + 1, 256), 256, 0, c.stream>>>(c.cell_key2.p, c.na, c.agrid.ncell,
-                                                                        c.acell_start.p);
-        if (c.nrep == 1 && c.ne)
-          k_ecell_near<<<nblk(c.agrid.ncell, 256), 256, 0, c.stream>>>(c.acell_start.p, c.rep_h[0].ag,
-                                                                       c.acell_near.p);
-        k_gather_pos<<<nblk(c.na, 256), 256, 0, c.stream>>>(c.xs.p, c.slot_atom.p, c.cell_key2.p, c.na, P,
-                                                            c.acell_pos.p, c.acell_fix.p, c.atom_slot.p,
-                                                            c.acell_of.p);
+      const int nac = c.agrid.ncell, nec = c.ne ? c.egrid.ncell : 0;
+      if (nac + nec <= SCAN_CELLS) {
+        k_scan_cells<<<1, 1024, 0, c.stream>>>(c.cell_count.p, nac, nec, c.acell_start.p, c.ecell_start.p);
       } else {
-        CACB200_CUDA(cudaMemsetAsync(c.acell_start.p, 0, sizeof(int) * (c.agrid.ncell + 1), c.stream));
+        size_t bytes = c.cub_bytes;
+        CACB200_CUDA(cub::DeviceScan::ExclusiveSum(c.cub_tmp.p, bytes, c.cell_count.p, c.acell_start.p, nac + 1, c.stream));
+        if (c.ne)
+          CACB200_CUDA(cub::DeviceScan::ExclusiveSum(c.cub_tmp.p, bytes, c.cell_count.p + nac + 1, c.ecell_start.p,
+                                                     nec + 1, c.stream));
       }
-      if (c.ne) {
-        bytes = c.cub_bytes;
-        k_elem_keys<<<nblk(c.ne, 256), 256, 0, c.stream>>>(c.ecenter.p, c.ne, P, c.cell_key.p, c.idx_tmp.p);
-        CACB200_CUDA(cub::DeviceRadixSort::SortPairs(c.cub_tmp.p, bytes, c.cell_key.p, c.cell_key2.p,
-                                                     c.idx_tmp.p, c.ecell_elems.p, c.ne, 0, c.sort_bits_e,
-                                                     c.stream));
-        k_cell_start<<<nblk(c.egrid.ncell + 1, 256), 256, 0, c.stream>>>(c.cell_key2.p, c.ne, c.egrid.ncell,
-                                                                        c.ecell_start.p);
-        k_gather_spheres<<<nblk(c.ne, 256), 256, 0, c.stream>>>(c.ecenter.p, c.eframe.p, c.ecell_elems.p, c.ne,
-                                                                c.ecell_sphere.p);
-        if (c.nrep == 1)
-          k_ecell_near<<<nblk(c.egrid.ncell, 256), 256, 0, c.stream>>>(c.ecell_start.p, c.rep_h[0].eg,
-                                                                       c.ecell_near.p);
-      } else {
-        CACB200_CUDA(cudaMemsetAsync(c.ecell_start.p, 0, sizeof(int) * (c.egrid.ncell + 1), c.stream));
-      }
+      const bool near = c.nrep == 1 && c.ne;
+      const BinArgs B{c.atom_key.p,  c.atom_place.p, c.acell_start.p, c.elem_key.p, c.elem_place.p,
+                      c.ecell_start.p, c.atom_order.p, c.elem_order.p, c.na,         c.ne,
+                      near ? c.acell_near.p : nullptr, near ? c.ecell_near.p : nullptr,
+                      c.rep_h[0].ag, c.rep_h[0].eg};
+      const long n = (long)c.na + c.ne, cells = near ? (long)c.rep_h[0].ag.ncell + c.rep_h[0].eg.ncell : 0;
+      if (n + cells) k_scatter<<<nblk(n + cells, 256), 256, 0, c.stream>>>(B);
+      if (n)
+        k_place<<<nblk(n, 256), 256, 0, c.stream>>>(B, P, c.xs.p, c.acell_pos.p, c.acell_fix.p, c.slot_atom.p,
+                                                    c.atom_slot.p, c.acell_of.p, c.ecenter.p, c.eframe.p,
+                                                    c.ecell_elems.p, c.ecell_sphere.p);
     }
     BuildArgs A;
     A.xs = c.xs.p;
