@@ -379,10 +379,10 @@ bool rebuild_due(Ctx &c) {
   return !c.dist_check || moved_past_trigger(c);
 }
 
-void forces(Ctx &c, int eflag, int vflag) {
+void forces(Ctx &c, int eflag, int vflag, bool assemble = true) {
   interpolate_sites(c);
   pair_compute(c, eflag, vflag);
-  assemble_nodef(c);
+  if (assemble) assemble_nodef(c);
   c.forces_current = true;
 }
 
@@ -453,13 +453,15 @@ void nve_cycle(Ctx &c, double dt) {
       neigh_build_async(c, false);
     });
     // between two steps of the cycle nothing reads the velocities, so each
-    // step's second half-kick runs inside the next step's drift kernel
+    // step's second half-kick runs inside the next step's drift kernel, and
+    // so does the assembly of the node forces (a thermostat adds to them)
+    const bool assemble = c.lgv.on;
     c.g_steps = capture(c, [&] {
-      forces(c, 0, 0);
+      forces(c, 0, 0, assemble || every == 1);
       langevin_post_force(c, dt);
       for (int k = 1; k < every; k++) {
-        nve_initial(c, dt, true);
-        forces(c, 0, 0);
+        nve_initial(c, dt, true, !assemble);
+        forces(c, 0, 0, assemble || k + 1 == every);
         langevin_post_force(c, dt);
       }
       nve_final(c, dt);

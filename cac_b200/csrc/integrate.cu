@@ -52,15 +52,10 @@ __global__ void k_pair_table(const double4 *xs, double4 *xss, const int *slot_at
 // nodef[a] += sum_b Minv[a][b] fc[b] with the Hex inverse mass matrix
 // (element.cpp:1784-1850, the tensor product of [[4,-2],[-2,4]]).  With the
 // Gauss points on the nodes, wsa[g][n] = 1/8 when g sits on n, else 0; the
-// loops keep the reference's order of terms.  One thread per (element,
-// node): the element's 8 threads read its 24 Gauss-point components
-// together and each writes its node's force.
-__global__ void k_assemble(const double *gaussf, double *nodef, int ne) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const int e = (int)(t >> 3), a = (int)(t & 7);
-  if (e >= ne) return;
+// loops keep the reference's order of terms.  Node a of the element whose 24
+// Gauss-point components are gf.
+__device__ __forceinline__ void node_force(const double *gf, int a, double acc[3]) {
   const double weight = (double)NU / (1.0 * 8) * 1.0;   // UNIFORM node weight
-  const double *gf = gaussf + (size_t)e * 24;
   double fc[8][3];
 #pragma unroll
   for (int n = 0; n < 8; n++) fc[n][0] = fc[n][1] = fc[n][2] = 0.0;
@@ -74,8 +69,7 @@ __global__ void k_assemble(const double *gaussf, double *nodef, int ne) {
       for (int d = 0; d < 3; d++) fc[n][d] += w * gf[3 * g + d];
     }
   }
-  double *nf = nodef + (size_t)e * 24;
-  double acc[3] = {0.0, 0.0, 0.0};
+  acc[0] = acc[1] = acc[2] = 0.0;
 #pragma unroll
   for (int b = 0; b < NPE; b++) {
     double m = (node_xi(a) == node_xi(b) ? 4.0 : -2.0) * (node_eta(a) == node_eta(b) ? 4.0 : -2.0) *
@@ -83,6 +77,17 @@ __global__ void k_assemble(const double *gaussf, double *nodef, int ne) {
 #pragma unroll
     for (int d = 0; d < 3; d++) acc[d] += m * fc[b][d];
   }
+}
+
+// One thread per (element, node): the element's 8 threads read its 24
+// Gauss-point components together and each writes its node's force.
+__global__ void k_assemble(const double *gaussf, double *nodef, int ne) {
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const int e = (int)(t >> 3), a = (int)(t & 7);
+  if (e >= ne) return;
+  double acc[3];
+  node_force(gaussf + (size_t)e * 24, a, acc);
+  double *nf = nodef + (size_t)e * 24;
   nf[3 * a] = acc[0];
   nf[3 * a + 1] = acc[1];
   nf[3 * a + 2] = acc[2];
@@ -94,12 +99,14 @@ __global__ void k_assemble(const double *gaussf, double *nodef, int ne) {
 // whole elements).  With xb, the drift also records each site's distance
 // from where the lists were built, rounded up, for the prefix rule
 // (PrefixRule, ctx.cuh): disp per atom, edisp per element (its largest node
-// displacement), and the largest of all per replica into dmax (cleared
-// before the launch; non-negative floats as bits, whose integer order is
-// theirs).
+// displacement), and the largest of all since the build per replica into dmax
+// (cleared by the build; non-negative floats as bits, whose integer order is
+// theirs).  With gaussf the node forces are formed here from the Gauss points'
+// (node_force), as k_assemble would have left them in nodef: between two steps
+// of a run nothing else reads them, and a launch per step is saved.
 __global__ void k_nve_initial(double4 *xs, double *v, const double *f, int na, int napad, double *nodex,
-                              double *nodev, const double *nodef, int nnode, double dtfm, double dtv, int prekick,
-                              const double4 *xb, const double *nxb, float *disp, float *edisp, unsigned *dmax,
+                              double *nodev, const double *nodef, const double *gaussf, int nnode, double dtfm,
+                              double dtv, int prekick, const double4 *xb, const double *nxb, float *disp, float *edisp, unsigned *dmax,
                               const int *site_rep, const int *elem_rep) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   float d = 0.0f;
@@ -137,13 +144,19 @@ __global__ void k_nve_initial(double4 *xs, double *v, const double *f, int na, i
   } else if (t >= napad) {
     const int k = t - napad;   // node 8 e + n of element e
     if (k < nnode) {
-      double dd = 0.0;
+      double dd = 0.0, nf[3];
+      if (gaussf) {
+        node_force(gaussf + (size_t)(k / 8) * 24, k & 7, nf);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; c++) nf[c] = nodef[3 * (size_t)k + c];
+      }
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const size_t m = 3 * (size_t)k + c;
         double vn = nodev[m];
-        if (prekick) vn = __dadd_rn(vn, __dmul_rn(dtfm, nodef[m]));
-        vn = __dadd_rn(vn, __dmul_rn(dtfm, nodef[m]));
+        if (prekick) vn = __dadd_rn(vn, __dmul_rn(dtfm, nf[c]));
+        vn = __dadd_rn(vn, __dmul_rn(dtfm, nf[c]));
         nodev[m] = vn;
         const double xn = __dadd_rn(nodex[m], __dmul_rn(dtv, vn));
         nodex[m] = xn;
@@ -224,19 +237,19 @@ void assemble_nodef(Ctx &c) {
   k_assemble<<<nblk(8L * c.ne, 128), 128, 0, c.stream>>>(c.gaussf.p, c.nodef.p, c.ne);
 }
 
-void nve_initial(Ctx &c, double dt, bool prekick) {
+void nve_initial(Ctx &c, double dt, bool prekick, bool assembling) {
   c.forces_current = false;   // the drift moves every site
   double dtf = 0.5 * dt * (1.0 / 1.0364269e-4);   // metal units, update.cpp:161-164
   double dtfm = dtf / c.mass;
   if (c.na + c.ne == 0) return;
   KernelTimer t(c, "nve_initial");
   const bool check = c.lists_valid && c.inner_ok.p && c.xbuild.p && c.disp.p && inner_limit(c) > 0.0;
-  if (check) CACB200_CUDA(cudaMemsetAsync(c.dmax.p, 0, sizeof(unsigned) * c.nrep, c.stream));
   const int napad = (c.na + 31) & ~31;
   const long n = (long)napad + 8L * c.ne;
   const bool many = c.nrep > 1;
   k_nve_initial<<<nblk(n, 256), 256, 0, c.stream>>>(
-      c.xs.p, c.v.p, c.f.p, c.na, napad, c.nodex.p, c.nodev.p, c.nodef.p, 8 * c.ne, dtfm, dt, prekick ? 1 : 0,
+      c.xs.p, c.v.p, c.f.p, c.na, napad, c.nodex.p, c.nodev.p, c.nodef.p,
+      assembling ? c.gaussf.p : nullptr, 8 * c.ne, dtfm, dt, prekick ? 1 : 0,
       check ? c.xbuild.p : nullptr, check ? c.nodex_build.p : nullptr, c.disp.p, c.edisp.p,
       check ? c.dmax.p : nullptr, many ? c.site_rep.p : nullptr, many ? c.elem_rep.p : nullptr);
 }
