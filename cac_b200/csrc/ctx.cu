@@ -1,4 +1,5 @@
 // Context lifetime, host<->device transfer and the extern "C" entry points.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -637,7 +638,10 @@ void minimize_fire(Ctx &c, double etol, double ftol, int maxiter, double dt, int
     int done = 0;
     const int chunk = 25;
     while (true) {
-      for (int k = 0; k < chunk; k++) {
+      // iteration maxiter + 1 only ends the minimisation: none is queued
+      // behind it
+      const int queued = std::min(chunk, std::max(maxiter + 1 - done, 1));
+      for (int k = 0; k < queued; k++) {
         fire_step(c);
         done++;
         c.step++;
@@ -645,7 +649,23 @@ void minimize_fire(Ctx &c, double etol, double ftol, int maxiter, double dt, int
         forces(c, CACB200_ENERGY_GLOBAL, 0);
       }
       s = fire_read(c);
-      if (s.status >= 0 || done > maxiter + chunk) break;
+      if (s.status >= 0 || done > maxiter) {
+        // the steps to the end of the chunk count, and so does a list rebuild
+        // due among them, which wraps the final positions into the box
+        bool wrapped = false;
+        for (int k = queued; k < chunk; k++) {
+          c.step++;
+          if (!rebuild_due(c)) continue;
+          if (wrapped) {
+            c.last_build_step = c.step;   // nothing has moved since
+          } else {
+            build(c, false);
+            forces(c, CACB200_ENERGY_GLOBAL, 0);
+            wrapped = true;
+          }
+        }
+        break;
+      }
     }
     if (s.status < 0) s.status = 0;
     *stop_code = s.status;
