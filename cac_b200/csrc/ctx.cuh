@@ -292,8 +292,8 @@ struct Ctx {
   DBuf<double> nodex_build;
   DBuf<int> nbr_half, num_half;
   bool have_half = false, lists_valid = false;
-  DBuf<int> raw_full, raw_half;  // build-time element-site entries (full) and half lists before compaction
-  DBuf<unsigned char> img_full, img_half;
+  DBuf<int> raw_sites, raw_half; // build-time element-site entries (full) and half lists before compaction
+  DBuf<unsigned char> img_half;
   DBuf<unsigned char> site_flag; // marks of the lattice sites that are neighbours (neigh.cu) ...
   DBuf<uint2> site_words;        // ... as bits, with their ranks in act_gid
   DBuf<int> overflow;            // [16] device flags (see neigh_check)
