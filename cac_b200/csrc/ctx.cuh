@@ -234,7 +234,7 @@ struct Ctx {
   DBuf<int> acell_fix;           // [3][na] the same in fixed point (the atom build's screen, neigh.cu)
   DBuf<int> acell_of;            // [na] cell of each sorted atom
   DBuf<int> ecell_start, ecell_elems;
-  DBuf<double4> ecell_sphere;    // [ne] candidate spheres of the sorted elements
+  DBuf<char> ecell_box;          // [ne] the sorted elements as the element walk reads them (ElemBox, neigh.cu)
   DBuf<int> atom_key, atom_place, atom_order, elem_key, elem_place, elem_order, cell_count;   // binning
   DBuf<int> atom_work, atom_nwork;   // atoms with element sites in reach (rebuild work list)
   DBuf<int2> items;                  // [slots][item_cap] element boxes to test, per query

@@ -399,13 +399,22 @@ constexpr int FAR_ATOM = 0x80000000;
 constexpr float QUANTUM = 1.0f / 1048576.0f;
 __device__ __forceinline__ int fix20(double x) { return (int)(unsigned)(unsigned long long)__double2ll_rn(x * 1048576.0); }
 
+// What the element walk reads of an element, in FP32: its centre from the box
+// corner with the reach of its sites (radius + deviation from affine); the rows
+// of its inverse frame (position from the centre -> lattice indices) with the
+// centre's own indices; and the rows' norms with the deviation from affine.
+// Rounding is at most a few 2^-24 of the box, which the walk allows for
+// (it only has to find every site; the sites are tested for themselves).
+struct ElemBox {
+  float4 centre, row[3], norm;
+};
+
 // The sorted atoms: positions (w = atom index), the fixed-point copies of the
 // screen (x, y, z parts na apart), slots and cells; and the sorted elements
-// with their candidate spheres (centre, and reach of the sites -- radius +
-// deviation from affine -- in w).
+// with their boxes.
 template <class RP>
 __global__ void k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *fixed, int *slot_atom, int *atom_slot,
-                        int *slot_cell, const double4 *ecenter, const double *eframe, int *elems, double4 *spheres) {
+                        int *slot_cell, const double4 *ecenter, const double *eframe, int *elems, ElemBox *boxes) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < B.na) {
     const int cell = B.akey[i], k = cell_place(B.astart, B.aorder, cell, i);
@@ -434,9 +443,20 @@ __global__ void k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *f
   if (i >= B.ne) return;
   const int k = cell_place(B.estart, B.eorder, B.ekey[i], i);
   elems[k] = i;
-  double4 c = ecenter[i];
-  c.w += eframe[(size_t)i * EFR + 12];
-  spheres[k] = c;
+  const double4 c = ecenter[i];
+  const double *fr = eframe + (size_t)i * EFR;
+  const BoxD b = P.elem(i).b;
+  ElemBox &o = boxes[k];
+  o.centre = make_float4((float)(c.x - b.lo[0]), (float)(c.y - b.lo[1]), (float)(c.z - b.lo[2]),
+                         __double2float_ru(c.w + fr[12]));
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const double a0 = fr[3 + 3 * r], a1 = fr[4 + 3 * r], a2 = fr[5 + 3 * r];
+    o.row[r] = make_float4((float)a0, (float)a1, (float)a2,
+                           (float)(a0 * (c.x - fr[0]) + a1 * (c.y - fr[1]) + a2 * (c.z - fr[2])));
+  }
+  o.norm = make_float4(__double2float_ru(fr[22]), __double2float_ru(fr[23]), __double2float_ru(fr[24]),
+                       __double2float_ru(fr[12]));
 }
 
 // -------------------------------------------------------------- the build
@@ -454,7 +474,7 @@ struct BuildArgs {
   const unsigned char *ecell_near;   // single systems: element cell has an element in its 27-cell block (else null)
   const unsigned char *acell_near;   // single systems: atom cell has an atom in its 27-cell block (else null)
   const int *ecell_elems;
-  const double4 *ecell_sphere;   // the sorted elements' candidate spheres
+  const ElemBox *ecell_box;      // the sorted elements, as the element walk reads them
   const int *atom_of_slot;    // list slot (cell-sorted position) -> atom index
   unsigned char *site_flag;   // [ne * MARKS] marks the lattice sites some full list references
   int na, ne, nsi, cap;
@@ -645,117 +665,212 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return m;
 }
 
-// The cell c (0 .. 26, x fastest) around a query's element cell: its elements
-// [beg, end) of the sorted ones, and the image its elements are seen under.
-__device__ __forceinline__ void element_cell(const BuildArgs &A, const Query &q, const int ci[3], int c, int &beg,
-                                             int &end, int s[3]) {
+// Phase A for the Q queries of a warp (32 / Q lanes each, all with the query):
+// those of one replica within two cells of one another are taken together.
+// The lanes walk the cells around all of them, 32 at a time, and keep the
+// elements that can reach the queries' bounding box (the candidate sphere, then
+// the lattice-index box); each query tests the few that are left.  A query's
+// items are those of the 27 cells around it in the order of the cells (x
+// fastest) and of the elements in each, whatever queries it shares the walk
+// with.  Returns the number of items of the lane's query; at most cap are stored.
+// All in FP32 from the box corner, with the roundings allowed for: an item too
+// many costs a few site tests and changes no list.
+constexpr int NEAR = 64;
+struct NearStage {
+  float4 centre[NEAR];    // of the image in the box the queries are wrapped into; w: reach of the sites
+  int kk[NEAR];           // place among the sorted elements
+  int w[NEAR];            // the cell's image + 1 per dimension, 2 bits each
+  int2 item[8][32];       // accepted items until their places are known (Q = 8)
+};
+template <int Q>
+__device__ int element_items(const BuildArgs &A, const Query &q, int rep, bool live, int2 *out, int cap,
+                             NearStage &st) {
+  constexpr int S = 32 / Q;
+  static_assert(Q == 32 || Q == 8, "st.item's rows");
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   const Grid &eg = q.r.eg;
-  const int o[3] = {c % 3 - 1, c / 3 % 3 - 1, c / 9 - 1};
-  int cc[3], W;
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    wrap_cell(ci[d] + o[d], eg.nc[d], cc[d], W);
-    s[d] = W - q.ti[d];
-  }
-  const int cell = q.r.ebase + (cc[2] * eg.nc[1] + cc[1]) * eg.nc[0] + cc[0];
-  beg = A.ecell_start[cell];
-  end = A.ecell_start[cell + 1];
-}
-
-// The work item of the element at place kk of the sorted ones, seen under
-// image s: a candidate sphere test, then the lattice-index box of the sites
-// whose affine position can lie within cutneigh + the element's deviation from
-// affine.  False: no site in reach.
-__device__ __forceinline__ bool element_item(const BuildArgs &A, const Query &q, int kk, const int s[3], int2 &item) {
-  const double4 ce = ldg256(A.ecell_sphere + kk);
-  // sphere test in the element's raw frame: |xi - s L - centre| <= cutneigh + R
-  const double p[3] = {q.xi[0] - s[0] * q.r.b.L[0], q.xi[1] - s[1] * q.r.b.L[1], q.xi[2] - s[2] * q.r.b.L[2]};
-  const double R = ce.w + A.cutneigh + 1e-6;
-  const double dcx = p[0] - ce.x, dcy = p[1] - ce.y, dcz = p[2] - ce.z;
-  if (dcx * dcx + dcy * dcy + dcz * dcz > R * R) return false;
-  const int e = A.ecell_elems[kk];
-  const double *fr = A.eframe + (size_t)e * EFR;
-  const double dmax = fr[12];
-  const double rel[3] = {p[0] - fr[0], p[1] - fr[1], p[2] - fr[2]};
-  int lo[3], hi[3];
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    const double a0 = fr[3 + 3 * r], a1 = fr[4 + 3 * r], a2 = fr[5 + 3 * r];
-    const double fidx = a0 * rel[0] + a1 * rel[1] + a2 * rel[2];
-    const double rho = (A.cutneigh + dmax + 1e-6) * fr[22 + r] + 1e-6;
-    lo[r] = max(0, (int)ceil(fidx - rho));
-    hi[r] = min(NC - 1, (int)floor(fidx + rho));
-    if (lo[r] > hi[r]) return false;
-  }
-  // a box shorter than the candidate sphere's diameter shows an element
-  // under two images; images beyond +-2 cannot be encoded (and are far
-  // beyond any cutoff in such a box)
-  if (s[0] < -3 || s[0] > 3 || s[1] < -3 || s[1] > 3 || s[2] < -3 || s[2] > 3) {
-    atomicExch(&A.overflow[2], 1);
-    return false;
-  }
-  item = pack_item(e, s, lo, hi);
-  return true;
-}
-
-// Phase A for one query, by L neighbouring lanes (L = 1 or 8; every lane of the
-// group calls it with the same query): the items of the 27 cells around, in
-// cell order.  Eight lanes walk eight cells at a time and place their items by
-// the counts of the cells before.  Returns the number of items; at most cap
-// are stored.
-template <int L>
-__device__ int element_items(const BuildArgs &A, const Query &q, int2 *out, int cap) {
-  const Grid &eg = q.r.eg;
+  float lo[3], hi[3];
   int ci[3];
 #pragma unroll
-  for (int d = 0; d < 3; d++)
+  for (int d = 0; d < 3; d++) {
+    const double r = fmax(q.wi[d] - q.r.b.lo[d], 0.0);
+    lo[d] = __double2float_rd(r);
+    hi[d] = __double2float_ru(r);
     ci[d] = min(max((int)((q.wi[d] - q.r.b.lo[d]) * eg.inv[d]), 0), eg.nc[d] - 1);
-  // no element in the 27 cells around: nothing to walk
-  if (A.ecell_near && !A.ecell_near[q.r.ebase + (ci[2] * eg.nc[1] + ci[1]) * eg.nc[0] + ci[0]]) return 0;
-  int n = 0, s[3], beg, end;
-  int2 item;
-  if (L == 1) {
-    for (int c = 0; c < 27; c++) {
-      element_cell(A, q, ci, c, beg, end, s);
-      for (int kk = beg; kk < end; kk++)
-        if (element_item(A, q, kk, s, item)) {
-          if (n < cap) out[n] = item;
-          n++;
-        }
-    }
-    return n;
   }
-  const int sub = threadIdx.x % L;
-  const unsigned group = ((1ull << L) - 1u) << ((threadIdx.x & 31) - sub);
-  for (int c0 = 0; c0 < 27; c0 += L) {
-    beg = end = 0;
-    if (c0 + sub < 27) element_cell(A, q, ci, c0 + sub, beg, end, s);
-    // the lane's accepted elements, 32 of its cell at a time (one round unless
-    // a cell holds more; then the cells' items must not interleave)
-    const bool crowded = __any_sync(group, end - beg > 32);
-    for (int turn = 0; turn < (crowded ? L : 1); turn++) {
-      const bool mine = !crowded || turn == sub;
-      unsigned acc = 0;
-      int count = 0;
-      for (int kk = beg; mine && kk < end; kk++)
-        if (element_item(A, q, kk, s, item)) {
-          if (kk - beg < 32) acc |= 1u << (kk - beg);
-          if (crowded && n + count < cap) out[n + count] = item;
-          count++;
-        }
-      int at = count;
+  // no element in the 27 cells around: nothing to walk
+  if (A.ecell_near && !A.ecell_near[q.r.ebase + (ci[2] * eg.nc[1] + ci[1]) * eg.nc[0] + ci[0]]) live = false;
+  int n = 0;
+  for (unsigned todo = __ballot_sync(full, live); todo;) {
+    const int lead = __ffs(todo) - 1;
+    const int lead_rep = __shfl_sync(full, rep, lead);
+    bool in = ((todo >> lane) & 1u) && rep == lead_rep;
+    int c0[3], nc[3], nr[3], ebase = __shfl_sync(full, q.r.ebase, lead);
+    float blo[3], bhi[3], L[3];   // positions from the box corner
 #pragma unroll
-      for (int o = 1; o < L; o <<= 1) {
-        const int v = __shfl_up_sync(group, at, o, L);
-        if (sub >= o) at += v;
+    for (int d = 0; d < 3; d++) {
+      const float far = fabsf(lo[d] - __shfl_sync(full, lo[d], lead)) * (float)eg.inv[d];
+      in = in && far <= 2.0f;
+    }
+    in = in || lane / S == lead / S;
+    todo &= ~__ballot_sync(full, in);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      blo[d] = __int_as_float(__reduce_min_sync(full, in ? __float_as_int(lo[d]) : 0x7fffffff));
+      bhi[d] = __int_as_float(__reduce_max_sync(full, in ? __float_as_int(hi[d]) : 0));
+      c0[d] = __reduce_min_sync(full, in ? ci[d] : 0x7fffffff) - 1;
+      nr[d] = __reduce_max_sync(full, in ? ci[d] : 0) + 2 - c0[d];
+      nc[d] = __shfl_sync(full, eg.nc[d], lead);
+      L[d] = __shfl_sync(full, (float)q.r.b.L[d], lead);
+    }
+    // roundings of the positions (each at most 2^-23 of the box)
+    const float slack = 1e-6f * (L[0] + L[1] + L[2]) + 1e-4f;
+    int m = 0;
+    auto flush = [&] {
+      __syncwarp();
+      for (int b = 0; b < m; b += 32) {
+        const int mm = min(32, m - b);
+        unsigned acc = 0;
+        for (int j = lane % S; j < mm; j += S) {
+          const float4 ce = st.centre[b + j];
+          const float dx = lo[0] - ce.x, dy = lo[1] - ce.y, dz = lo[2] - ce.z, R = ce.w + (float)A.cutneigh + slack;
+          if (in && dx * dx + dy * dy + dz * dz <= R * R) acc |= 1u << j;
+        }
+        unsigned ok = 0;
+        for (; acc; acc &= acc - 1) {
+          // the box of the sites whose affine position can lie within cutneigh +
+          // the element's deviation from affine
+          const int j = __ffs(acc) - 1, w = st.w[b + j], kk = st.kk[b + j];
+          const float4 ce = st.centre[b + j], norm = A.ecell_box[kk].norm;
+          const float dx = lo[0] - ce.x, dy = lo[1] - ce.y, dz = lo[2] - ce.z;
+          const float n3[3] = {norm.x, norm.y, norm.z}, far = (float)A.cutneigh + norm.w + slack;
+          int blo3[3], bhi3[3];
+          bool some = true;
+#pragma unroll
+          for (int r = 0; r < 3; r++) {
+            const float4 row = A.ecell_box[kk].row[r];
+            const float idx = row.x * dx + row.y * dy + row.z * dz + row.w, rho = far * n3[r] + 1e-4f;
+            blo3[r] = max(0, (int)ceilf(idx - rho));
+            bhi3[r] = min(NC - 1, (int)floorf(idx + rho));
+            some = some && blo3[r] <= bhi3[r];
+          }
+          const int s[3] = {(w & 3) - 1 - q.ti[0], ((w >> 2) & 3) - 1 - q.ti[1], (w >> 4) - 1 - q.ti[2]};
+          // a box shorter than the candidate sphere's diameter shows an element
+          // under two images; images beyond +-2 cannot be encoded (and are far
+          // beyond any cutoff in such a box)
+          if (some && (s[0] < -3 || s[0] > 3 || s[1] < -3 || s[1] > 3 || s[2] < -3 || s[2] > 3)) {
+            atomicExch(&A.overflow[2], 1);
+            some = false;
+          }
+          if (some) {
+            const int2 item = pack_item(A.ecell_elems[kk], s, blo3, bhi3);
+            if (S > 1) {
+              st.item[lane / S][j] = item;
+              ok |= 1u << j;
+            } else {
+              if (n < cap) out[n] = item;
+              n++;
+            }
+          }
+        }
+        if (S > 1) {
+          unsigned all = ok;
+          __syncwarp();
+#pragma unroll
+          for (int o = 1; o < S; o <<= 1) all |= __shfl_xor_sync(full, all, o);
+          for (; ok; ok &= ok - 1) {
+            const int j = __ffs(ok) - 1, at = n + __popc(all & ((1u << j) - 1u));
+            if (at < cap) out[at] = st.item[lane / S][j];
+          }
+          n += __popc(all);
+        }
       }
-      const int total = __shfl_sync(group, at, L - 1, L);
-      if (!crowded) {
-        at += n - count;
-        for (; acc; acc &= acc - 1, at++)
-          if (at < cap && element_item(A, q, beg + __ffs(acc) - 1, s, item)) out[at] = item;
+      m = 0;
+      __syncwarp();
+    };
+    // elements of a cell this far from the bounding box are out of reach
+    const float reach = __shfl_sync(full, (float)q.r.reach_budget, lead) + (float)A.cutneigh + 0.01f + slack;
+    float size[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) size[d] = L[d] / (float)nc[d];
+    const int cells = nr[0] * nr[1] * nr[2];
+    for (int b = 0; b < cells; b += 32) {
+      const int c = b + lane;
+      int end = 0, incl = 0, w = 0;
+      if (c < cells) {
+        const int y = c / nr[0], z = y / nr[1];
+        const int o[3] = {c0[0] + c - y * nr[0], c0[1] + y - z * nr[1], c0[2] + z};
+        int cc[3], W[3];
+        float d2 = 0.0f;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          wrap_cell(o[d], nc[d], cc[d], W[d]);
+          const float g = fmaxf(0.0f, fmaxf((float)o[d] * size[d] - bhi[d], blo[d] - (float)(o[d] + 1) * size[d]));
+          d2 += g * g;
+        }
+        if (d2 <= reach * reach) {
+          const int cell = ebase + (cc[2] * nc[1] + cc[1]) * nc[0] + cc[0];
+          w = (W[0] + 1) | (W[1] + 1) << 2 | (W[2] + 1) << 4;
+          end = A.ecell_start[cell + 1];
+          incl = end - A.ecell_start[cell];
+        }
       }
-      n += total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int total = __shfl_sync(full, incl, 31);
+      int k0 = 0;
+      do {
+        const int k = k0 + lane;
+        int o = 0;   // the lane whose cell holds the k-th element
+#pragma unroll
+        for (int step = 16; step; step >>= 1)
+          if (__shfl_sync(full, incl, o + step - 1) <= k) o += step;
+        const int kk = __shfl_sync(full, end, o) - (__shfl_sync(full, incl, o) - k);
+        const int ow = __shfl_sync(full, w, o);
+        bool pass = false;
+        float4 ce = make_float4(0, 0, 0, 0);
+        if (k < total) {
+          ce = A.ecell_box[kk].centre;
+          ce.x += ((ow & 3) - 1) * L[0];
+          ce.y += (((ow >> 2) & 3) - 1) * L[1];
+          ce.z += ((ow >> 4) - 1) * L[2];
+          const float R = ce.w + (float)A.cutneigh + slack;
+          const float dx = fmaxf(0.0f, fmaxf(blo[0] - ce.x, ce.x - bhi[0]));
+          const float dy = fmaxf(0.0f, fmaxf(blo[1] - ce.y, ce.y - bhi[1]));
+          const float dz = fmaxf(0.0f, fmaxf(blo[2] - ce.z, ce.z - bhi[2]));
+          pass = dx * dx + dy * dy + dz * dz <= R * R;
+          if (pass) {
+            // the same in the element's own directions: the lattice indices of
+            // the bounding box' centre, and how far its sides carry them
+            const float4 norm = A.ecell_box[kk].norm;
+            const float n3[3] = {norm.x, norm.y, norm.z}, far = (float)A.cutneigh + norm.w + slack;
+            const float x = 0.5f * (blo[0] + bhi[0]) - ce.x, y = 0.5f * (blo[1] + bhi[1]) - ce.y,
+                        z = 0.5f * (blo[2] + bhi[2]) - ce.z;
+            const float hx = 0.5f * (bhi[0] - blo[0]), hy = 0.5f * (bhi[1] - blo[1]), hz = 0.5f * (bhi[2] - blo[2]);
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+              const float4 row = A.ecell_box[kk].row[r];
+              const float idx = row.x * x + row.y * y + row.z * z + row.w;
+              const float rho = far * n3[r] + 1e-4f + fabsf(row.x) * hx + fabsf(row.y) * hy + fabsf(row.z) * hz;
+              if (idx + rho < 0.0f || idx - rho > NC - 1) pass = false;
+            }
+          }
+        }
+        const unsigned acc = __ballot_sync(full, pass);
+        if (pass) {
+          const int at = m + __popc(acc & lanemask_lt());
+          st.centre[at] = ce;
+          st.kk[at] = kk;
+          st.w[at] = ow;
+        }
+        m += __popc(acc);
+        k0 += 32;
+        if (m > NEAR - 32 || (b + 32 >= cells && k0 >= total)) flush();
+      } while (k0 < total);
     }
   }
   return n;
@@ -1433,43 +1548,60 @@ __global__ void __launch_bounds__(32) k_build_atoms_sm(BuildArgs A, OneRep P, in
 // Phase A over every list slot: the element walk of each atom and Gauss
 // point; atoms with at least one item go on the work list of phase B (its
 // order does not matter: an atom's entries depend on that atom alone).
-template <int L, class RP>
-__device__ __forceinline__ void elem_items_slot(const BuildArgs &A, const RP &P, int2 *items, int *nitems, int icap,
-                                                int *work, int *nwork) {
-  const int t = (blockIdx.x * blockDim.x + threadIdx.x) / L;
-  if (t >= A.nsi) return;   // whole groups
+// The Gauss points go first, a warp for each element's eight (their walk is the
+// longest, and the atoms' fill in behind it), then the atoms, Q to a warp: 32
+// of the sorted ones, in a small system 8 (below EIGHT_QUERY_SITES a warp's
+// serial chain of loads is what the kernel takes: 6 k sites 20.5 us against
+// 22.9, while at 80 k to 88 k sites 32 are the faster by a fifth).
+// A query alone walked 27 cells, about 130 elements, in FP64, and its warp took
+// 6,700 instructions in one long chain.  Measured per build, before and after:
+// 1,554 queries 29 -> 16 us, 83,550 88 -> 31 us, 93,000 (FIRE) 145 -> 40 us,
+// 313,120 142 -> 53 us, 4.98 M 1024 -> 571 us, 64 replicas with 1.72 M
+// 828 -> 343 us.  Groups of queries within one cell, half of one or a quarter
+// instead of two: 5 M queries 1074, 1692 and 2662 us against 858 (each group
+// walks the cells again).  Registers: 8 blocks an SM at Q = 32 (96 -> 64
+// registers; 694 -> 571 us at 5 M), 5 at Q = 8, where more only spills.
+constexpr int EIGHT_QUERY_SITES = 30000;
+template <int Q, class RP>
+__device__ __forceinline__ void elem_items_queries(const BuildArgs &A, const RP &P, int first, int end, int2 *items,
+                                                   int *nitems, int icap, int *work, int *nwork, NearStage &st) {
+  constexpr int S = 32 / Q;
+  const int lane = threadIdx.x & 31, place = first + lane / S;
+  const bool live = place < end;
+  const int t = live ? place : end - 1;
+  const int i = t < A.na ? A.atom_of_slot[t] : t;
   Query q;
-  if (t < A.na) {
-    make_query(A, P, A.atom_of_slot[t], q);
-    q.slot = t;
-  } else {
-    make_query(A, P, t, q);
+  make_query(A, P, i, q);
+  q.slot = t;
+  int rep = 0;
+  if constexpr (RP::many) rep = P.site_rep[i];
+  const int n = element_items<Q>(A, q, rep, live, items + (size_t)t * icap, icap, st);
+  const bool one = live && lane % S == 0;
+  if (one) {
+    nitems[t] = n;
+    if (n > icap) {
+      atomicExch(&A.overflow[8], 1);
+      atomicMax(&A.overflow[9], n);
+    }
   }
-  const int n = element_items<L>(A, q, items + (size_t)t * icap, icap);
-  if (threadIdx.x % L) return;
-  nitems[t] = n;
-  if (n > icap) {
-    atomicExch(&A.overflow[8], 1);
-    atomicMax(&A.overflow[9], n);
-  }
-  if (t < A.na && n > 0) work[atomicAdd(nwork, 1)] = t;
+  const bool listed = one && t < A.na && n > 0;
+  const unsigned m = __ballot_sync(0xffffffffu, listed);
+  int at = 0;
+  if (m && lane == 0) at = atomicAdd(nwork, __popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (listed) work[at + __popc(m & lanemask_lt())] = t;
 }
 
-// One lane per query in the single-system form as the compiler allocates it;
-// the batch form capped at 64 registers (from 70) for 8 resident blocks per
-// SM: 4 % faster on a 64-replica batch, where the same cap slowed the
-// single-system form.  Below EIGHT_LANE_QUERIES a query's serial chain of cell
-// and element loads is what the kernel takes, and eight lanes share it.
-constexpr int EIGHT_LANE_QUERIES = 30000;
-template <int L>
-__global__ void __launch_bounds__(128) k_elem_items(BuildArgs A, OneRep P, int2 *items, int *nitems, int icap,
-                                                    int *work, int *nwork) {
-  elem_items_slot<L>(A, P, items, nitems, icap, work, nwork);
-}
-template <int L>
-__global__ void __launch_bounds__(128, 8) k_elem_items(BuildArgs A, ManyRep P, int2 *items, int *nitems, int icap,
-                                                       int *work, int *nwork) {
-  elem_items_slot<L>(A, P, items, nitems, icap, work, nwork);
+template <int Q, class RP>
+__global__ void __launch_bounds__(128, Q == 32 ? 8 : 5) k_elem_items(BuildArgs A, RP P, int2 *items, int *nitems, int icap, int *work,
+                                                    int *nwork) {
+  __shared__ NearStage stage[4];
+  NearStage &st = stage[threadIdx.x >> 5];
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w < A.ne)
+    elem_items_queries<8>(A, P, A.na + NG * w, A.nsi, items, nitems, icap, work, nwork, st);
+  else if (Q * (w - A.ne) < A.na)   // whole warps
+    elem_items_queries<Q>(A, P, Q * (w - A.ne), A.na, items, nitems, icap, work, nwork, st);
 }
 
 // Phase B for atoms: one warp per listed atom, its element sites appended
@@ -1893,7 +2025,7 @@ void neigh_plan(Ctx &c, bool want_half) {
   c.ecell_near.reserve(c.egrid.ncell + 1);
   c.acell_near.reserve(c.agrid.ncell + 1);
   c.ecell_elems.reserve(std::max(c.ne, 1));
-  c.ecell_sphere.reserve(std::max(c.ne, 1));
+  c.ecell_box.reserve(sizeof(ElemBox) * std::max(c.ne, 1));
   size_t slots = (size_t)c.cap * std::max(nsi, 1);
   c.raw_sites.reserve(slots);
   c.num_full.reserve(std::max(nsi, 1));
@@ -2002,7 +2134,7 @@ void neigh_build_async(Ctx &c, bool want_half) {
       if (n)
         k_place<<<nblk(n, 256), 256, 0, c.stream>>>(B, P, c.xs.p, c.acell_pos.p, c.acell_fix.p, c.slot_atom.p,
                                                     c.atom_slot.p, c.acell_of.p, c.ecenter.p, c.eframe.p,
-                                                    c.ecell_elems.p, c.ecell_sphere.p);
+                                                    c.ecell_elems.p, (ElemBox *)c.ecell_box.p);
     }
     BuildArgs A;
     A.xs = c.xs.p;
@@ -2019,7 +2151,7 @@ void neigh_build_async(Ctx &c, bool want_half) {
     A.ecell_near = (c.nrep == 1 && c.ne) ? c.ecell_near.p : nullptr;
     A.acell_near = (c.nrep == 1 && c.na && c.ne) ? c.acell_near.p : nullptr;
     A.ecell_elems = c.ecell_elems.p;
-    A.ecell_sphere = c.ecell_sphere.p;
+    A.ecell_box = (const ElemBox *)c.ecell_box.p;
     A.atom_of_slot = c.slot_atom.p;
     A.site_flag = c.site_flag.p;
     if (c.ne) CACB200_CUDA(cudaMemsetAsync(c.site_flag.p, 0, (size_t)c.ne * MARKS, c.stream));
@@ -2055,12 +2187,12 @@ void neigh_build_async(Ctx &c, bool want_half) {
     if (c.ne) {
       {
         KernelTimer t(c, "build_items");
-        if (nsi < EIGHT_LANE_QUERIES)
-          k_elem_items<8><<<nblk(8L * nsi, 128), 128, 0, es>>>(A, P, c.items.p, c.nitems.p, c.item_cap,
-                                                               c.atom_work.p, c.atom_nwork.p);
+        if (nsi < EIGHT_QUERY_SITES)
+          k_elem_items<8><<<nblk(32L * (c.ne + nblk(c.na, 8)), 128), 128, 0, es>>>(
+              A, P, c.items.p, c.nitems.p, c.item_cap, c.atom_work.p, c.atom_nwork.p);
         else
-          k_elem_items<1><<<nblk(nsi, 128), 128, 0, es>>>(A, P, c.items.p, c.nitems.p, c.item_cap, c.atom_work.p,
-                                                          c.atom_nwork.p);
+          k_elem_items<32><<<nblk(32L * (c.ne + nblk(c.na, 32)), 128), 128, 0, es>>>(
+              A, P, c.items.p, c.nitems.p, c.item_cap, c.atom_work.p, c.atom_nwork.p);
       }
       if (split) CACB200_CUDA(cudaEventRecord(c.items_ev, c.side));
       {

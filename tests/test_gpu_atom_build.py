@@ -48,7 +48,7 @@ def test_lists_equal_the_restatement(shape, oracle_mod):
 def test_element_walk_with_crowded_cells(copies, na, oracle_mod):
     """Elements lying over one another, so that an element cell holds more than
     32 of them (36 with six copies), for both forms of the element walk (eight
-    lanes a query below 30,000 queries)."""
+    atoms to a warp below 30,000 queries)."""
     from cac_b200.api import Engine
     s = gen.build_slab(3, 1, 1, 3, temperature=300.0, seed=4)
     rng = np.random.default_rng(9)

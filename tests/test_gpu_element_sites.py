@@ -40,3 +40,27 @@ def test_element_sites_equal_the_restatement(case, oracle_mod):
     if half:
         assert np.array_equal(e.neighbor_list(half=True), oracle_mod.build_list(st, cut + 0.5, True).canonical(s.natoms))
     e.close()
+
+
+@pytest.mark.parametrize("na,ne,scale", [(9, 12, 1.0), (0, 1, 2.5), (700, 3, 3.0), (31000, 2, 2.0), (31003, 12, 1.5)])
+def test_scattered_queries_equal_the_restatement(na, ne, scale, oracle_mod):
+    """Atoms and elements far apart, so that the queries of a warp stand in
+    many places (eight or 32 of them to a warp, below and above 30,000)."""
+    from cac_b200.api import Engine
+    s = gen.build_slab(3, 1, 1, 3, temperature=300.0, seed=8)
+    rng = np.random.default_rng(23)
+    s.boxhi = s.boxlo + scale * (s.boxhi - s.boxlo)
+    s.nodex = s.nodex[:ne] - s.nodex[:ne].mean(axis=1, keepdims=True) + rng.uniform(s.boxlo, s.boxhi, (ne, 1, 3))
+    s.nodev = s.nodev[:ne].copy()
+    s.x = rng.uniform(s.boxlo, s.boxhi, (na, 3))
+    s.v = np.zeros_like(s.x)
+    gen.wrap_into_box(s)
+    cut = 2.5 if na < 31000 else 0.8
+    st = oracle_mod.OracleState(s)
+    e = Engine(0)
+    e.upload(s)
+    e.pair_lj(0.4093, 2.338, cut)
+    e.neighbor(0.5, 10)
+    e.build_lists()
+    assert np.array_equal(e.neighbor_list(), oracle_mod.build_list(st, cut + 0.5, False).canonical(s.natoms))
+    e.close()
