@@ -364,9 +364,10 @@ void fetch_ev(Ctx &c) {
   c.ev_pending = false;
 }
 
+// (the pair table is filled by the force evaluation that follows: filled here
+// as well it cost a launch per rebuild, 8 us at 6 k sites, 21 us at 0.9 M)
 void build(Ctx &c, bool want_half) {
   neigh_build(c, want_half);
-  interpolate_sites(c);
   c.last_build_step = c.step;
 }
 
@@ -1039,6 +1040,7 @@ int cacb200_set_neighbor_modify(cacb200_ctx *ctx, int delay, int check) {
 int cacb200_build_lists(cacb200_ctx *ctx, int want_half) {
   API_BEGIN
   build(c, want_half != 0);
+  interpolate_sites(c);
   API_END
 }
 
