@@ -437,6 +437,32 @@ inline void note_build_box(Ctx &c) {
     }
 }
 
+// Launches a kernel of the chain of a step so that its blocks are set up while
+// the kernel before it in the stream still runs (programmatic dependent
+// launch); the kernel waits for that one itself (behind_previous, device.cuh).
+// A step of a small system is a chain of kernels of a few us each, which plain
+// launches put about 1 us apart: 6 k sites 31.7 -> 29.5 us a step with its share
+// of the rebuilds, 84 k sites in the mixed form 1.87 -> 1.66 ms for 25 steps, FIRE
+// at 93 k sites 9.88 -> 9.12 ms for 50 iterations.  Above
+// BEHIND_SITES the gaps are nothing and blocks that wait only take room from
+// those at work (1.21 M sites, 20 steps: 27.04 ms plainly, 26.86 ms so; 1.7 M
+// 29.65 and 29.72; 5 M 59.1 and 59.6).
+constexpr long BEHIND_SITES = 1500000;
+template <class... P, class... T>
+void launch_behind(const Ctx &c, int blocks, int threads, size_t smem, void (*kernel)(P...), T &&...args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c.stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = c.nsite_i() < BEHIND_SITES ? 1 : 0;
+  CACB200_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 // stages implemented in the .cu files
 void neigh_build(Ctx &c, bool want_half);
 void neigh_plan(Ctx &c, bool want_half);

@@ -95,6 +95,21 @@ __device__ __forceinline__ void ldg256(const float4 *p, float4 &a, float4 &b) {
       : "l"(p));
 }
 
+// The same where an earlier kernel has just written the data (launch_behind;
+// volatile, so that it stays behind behind_previous).
+__device__ __forceinline__ double4 ld256(const double4 *p) {
+  double4 r;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+
+// First statement of every kernel that launch_behind (ctx.cuh) starts: waits
+// for the kernel before to end (its writes are then visible) and lets the one
+// behind start.  What follows reads with plain loads, or constants.
+__device__ __forceinline__ void behind_previous() {
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;

@@ -33,6 +33,7 @@ constexpr int NP = 6;
 
 __global__ void k_fire_dots(const double *v, const double *f, int na, const double *nodev,
                             const double *nodef, int nn, double *partial) {
+  behind_previous();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   double vf = 0, vv = 0, ff = 0, vmax = 0, fmx = 0, fi2 = 0;
   const double *vp = nullptr, *fp = nullptr;
@@ -91,6 +92,7 @@ __global__ void k_fire_dots(const double *v, const double *f, int na, const doub
 // coefficients of the update kernel.
 __global__ void k_fire_control(const double *partial, int nb, const double *ev_out, FireState *S,
                                FireParams P) {
+  behind_previous();
   __shared__ double red[6][8];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   double a[6] = {0, 0, 0, 0, 0, 0};
@@ -193,6 +195,7 @@ __global__ void k_fire_update(double4 *xs, double *v, const double *f, int na, d
                               double *nodev, const double *nodef, int nn3, const FireState *S,
                               double mass, const double4 *xb, const double *nxb, int *inner_ok, double lim2,
                               double limc, const int *site_rep, const int *elem_rep) {
+  behind_previous();
   if (!S->apply) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   const double dtv = S->dtv, dtfm = dtv * FTM2V / mass, hb = S->halfback;
@@ -284,20 +287,20 @@ void fire_step(Ctx &c) {
   c.fire.mass = c.mass;
   {
     KernelTimer t(c, "fire_dots");
-    k_fire_dots<<<nb, 256, 0, c.stream>>>(c.v.p, c.f.p, c.na, c.nodev.p, c.nodef.p, 8 * c.ne,
-                                          c.fire_partial.p);
+    launch_behind(c, nb, 256, 0, k_fire_dots, c.v.p, c.f.p, c.na, c.nodev.p, c.nodef.p, 8 * c.ne,
+                  c.fire_partial.p);
   }
   {
     KernelTimer t(c, "fire_control");
-    k_fire_control<<<1, 256, 0, c.stream>>>(c.fire_partial.p, nb, c.ev_out.p, c.fire_state.p, c.fire);
+    launch_behind(c, 1, 256, 0, k_fire_control, c.fire_partial.p, nb, c.ev_out.p, c.fire_state.p, c.fire);
   }
   int n = c.na + 24 * c.ne;
   if (n) {
     KernelTimer t(c, "fire_update");
     const bool check = c.lists_valid && c.inner_ok.p && c.xbuild.p && inner_limit(c) > 0.0;
     const double lim = inner_limit(c);
-    k_fire_update<<<nblk(n, 256), 256, 0, c.stream>>>(
-        c.xs.p, c.v.p, c.f.p, c.na, c.nodex.p, c.nodev.p, c.nodef.p, 24 * c.ne, c.fire_state.p, c.mass,
+    launch_behind(
+        c, nblk(n, 256), 256, 0, k_fire_update, c.xs.p, c.v.p, c.f.p, c.na, c.nodex.p, c.nodev.p, c.nodef.p, 24 * c.ne, c.fire_state.p, c.mass,
         check ? c.xbuild.p : nullptr, check ? c.nodex_build.p : nullptr, c.inner_ok.p, lim * lim,
         lim / 1.7320508075688772, c.nrep > 1 ? c.site_rep.p : nullptr, c.nrep > 1 ? c.elem_rep.p : nullptr);
   }

@@ -16,6 +16,7 @@ inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 // (written by the last rebuild), so a fixed grid strides over the table.
 __global__ void k_pair_table(const double4 *xs, double4 *xss, const int *slot_atom, const double *nodex, int na,
                              int ne, const int *act_gid, const int *nact_dev) {
+  behind_previous();
   const int ngp = NG * ne;
   const int n = na + ngp + *nact_dev;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -82,6 +83,7 @@ __device__ __forceinline__ void node_force(const double *gf, int a, double acc[3
 // One thread per (element, node): the element's 8 threads read its 24
 // Gauss-point components together and each writes its node's force.
 __global__ void k_assemble(const double *gaussf, double *nodef, int ne) {
+  behind_previous();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int e = (int)(t >> 3), a = (int)(t & 7);
   if (e >= ne) return;
@@ -108,6 +110,7 @@ __global__ void k_nve_initial(double4 *xs, double *v, const double *f, int na, i
                               double *nodev, const double *nodef, const double *gaussf, int nnode, double dtfm,
                               double dtv, int prekick, const double4 *xb, const double *nxb, float *disp, float *edisp, unsigned *dmax,
                               const int *site_rep, const int *elem_rep) {
+  behind_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   float d = 0.0f;
   int rep = 0;
@@ -207,6 +210,7 @@ __global__ void k_nve_initial(double4 *xs, double *v, const double *f, int na, i
 // FixNVE::final_integrate (fix_nve.cpp:148-219)
 __global__ void k_nve_final(double *v, const double *f, int n3, double *nodev, const double *nodef,
                             int nn3, double dtfm) {
+  behind_previous();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n3) {
     v[t] = __dadd_rn(v[t], __dmul_rn(dtfm, f[t]));
@@ -227,14 +231,15 @@ void interpolate_sites(Ctx &c) {
     return;
   }
   // 64 blocks per SM, as the mixed form's pair table
-  k_pair_table<<<std::min(nblk((long)c.na + (long)NG * c.ne + (long)c.ne * NU, 256), 148 * 64), 256, 0, c.stream>>>(
+  launch_behind(
+      c, std::min(nblk((long)c.na + (long)NG * c.ne + (long)c.ne * NU, 256), 148 * 64), 256, 0, k_pair_table,
       c.xs.p, c.xss.p, c.slot_atom.p, c.nodex.p, c.na, c.ne, c.act_gid.p, c.dev_nact.p);
 }
 
 void assemble_nodef(Ctx &c) {
   if (c.ne == 0) return;
   KernelTimer t(c, "assemble");
-  k_assemble<<<nblk(8L * c.ne, 128), 128, 0, c.stream>>>(c.gaussf.p, c.nodef.p, c.ne);
+  launch_behind(c, nblk(8L * c.ne, 128), 128, 0, k_assemble, c.gaussf.p, c.nodef.p, c.ne);
 }
 
 void nve_initial(Ctx &c, double dt, bool prekick, bool assembling) {
@@ -247,7 +252,8 @@ void nve_initial(Ctx &c, double dt, bool prekick, bool assembling) {
   const int napad = (c.na + 31) & ~31;
   const long n = (long)napad + 8L * c.ne;
   const bool many = c.nrep > 1;
-  k_nve_initial<<<nblk(n, 256), 256, 0, c.stream>>>(
+  launch_behind(
+      c, nblk(n, 256), 256, 0, k_nve_initial,
       c.xs.p, c.v.p, c.f.p, c.na, napad, c.nodex.p, c.nodev.p, c.nodef.p,
       assembling ? c.gaussf.p : nullptr, 8 * c.ne, dtfm, dt, prekick ? 1 : 0,
       check ? c.xbuild.p : nullptr, check ? c.nodex_build.p : nullptr, c.disp.p, c.edisp.p,
@@ -316,8 +322,8 @@ void nve_final(Ctx &c, double dt) {
   int n = 3 * c.na + 24 * c.ne;
   if (n == 0) return;
   KernelTimer t(c, "nve_final");
-  k_nve_final<<<nblk(n, 256), 256, 0, c.stream>>>(c.v.p, c.f.p, 3 * c.na, c.nodev.p, c.nodef.p,
-                                                  24 * c.ne, dtfm);
+  launch_behind(c, nblk(n, 256), 256, 0, k_nve_final, c.v.p, c.f.p, 3 * c.na, c.nodev.p, c.nodef.p, 24 * c.ne,
+                dtfm);
 }
 
 }  // namespace cacb200

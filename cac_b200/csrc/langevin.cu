@@ -167,6 +167,7 @@ __device__ __forceinline__ double target_sqrt(const LgvArgs &A) {
 }
 
 __global__ void __launch_bounds__(32 * WARPS) k_langevin(LgvArgs A) {
+  behind_previous();
   __shared__ unsigned sb[WARPS][EXT];
   __shared__ unsigned sp[WARPS][WIN];
   __shared__ unsigned seq[WARPS][WIN + CHUNK];   // seq[rho] = Y_{B-96+jC+rho}
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_langevin(LgvArgs A) {
 __global__ void k_langevin_advance(unsigned *base, const unsigned *next, unsigned long long *m, long long *ctl,
                                    const int4 *meta, const int2 *rchunk, const double *partial, double *mean,
                                    int nrep) {
+  behind_previous();
   const int r = blockIdx.x;
   const int lane = threadIdx.x;
   if (r >= nrep) return;
@@ -290,6 +292,7 @@ __global__ void k_langevin_advance(unsigned *base, const unsigned *next, unsigne
 // zero yes: subtract each replica's mean random force from its atoms and nodes
 __global__ void k_langevin_zero(double *f, double *nodef, const double *mean, const int *site_rep,
                                 const int *elem_rep, int na, int ne) {
+  behind_previous();
   const long long n = 3LL * na + 24LL * ne;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
     if (q < 3LL * na) {
@@ -426,13 +429,12 @@ void langevin_post_force(Ctx &c, double dt) {
   {
     KernelTimer t(c, "langevin");
     if (c.lgv_nchunks > 0)
-      k_langevin<<<(c.lgv_nchunks + WARPS - 1) / WARPS, 32 * WARPS, 0, c.stream>>>(A);
-    k_langevin_advance<<<c.nrep, 32, 0, c.stream>>>(c.lgv_base.p, c.lgv_next.p, c.lgv_m.p, c.lgv_ctl.p,
-                                                     c.lgv_meta.p, c.lgv_rchunk.p, c.lgv_part.p,
-                                                     c.lgv.zero ? c.lgv_mean.p : nullptr, c.nrep);
+      launch_behind(c, (c.lgv_nchunks + WARPS - 1) / WARPS, 32 * WARPS, 0, k_langevin, A);
+    launch_behind(c, c.nrep, 32, 0, k_langevin_advance, c.lgv_base.p, c.lgv_next.p, c.lgv_m.p, c.lgv_ctl.p,
+                  c.lgv_meta.p, c.lgv_rchunk.p, c.lgv_part.p, c.lgv.zero ? c.lgv_mean.p : nullptr, c.nrep);
     if (c.lgv.zero)
-      k_langevin_zero<<<stride_grid(3L * c.na + 24L * c.ne, 256), 256, 0, c.stream>>>(
-          c.f.p, c.nodef.p, c.lgv_mean.p, c.nrep > 1 ? c.site_rep.p : nullptr, c.nrep > 1 ? c.elem_rep.p : nullptr,
+      launch_behind(
+          c, stride_grid(3L * c.na + 24L * c.ne, 256), 256, 0, k_langevin_zero, c.f.p, c.nodef.p, c.lgv_mean.p, c.nrep > 1 ? c.site_rep.p : nullptr, c.nrep > 1 ? c.elem_rep.p : nullptr,
           c.na, c.ne);
   }
   CACB200_CUDA(cudaGetLastError());

@@ -110,6 +110,7 @@ struct BuildStart {
 // which a small system would wait for one by one).
 template <class RP>
 __global__ void k_pbc_atoms(double4 *xs, int na, RP P, BuildStart S) {
+  behind_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (S.xbuild) {
     if (i < S.nrep) {
@@ -167,6 +168,7 @@ template <class RP>
 __global__ void k_elem_geom(double *nodex, int ne, RP P, double4 *ecenter, double *eframe,
                             unsigned long long *reach_bits, int *grew, double *nodex_build, float *edisp, int *key,
                             int *place, int *count) {
+  behind_previous();
   int e = blockIdx.x * blockDim.x + threadIdx.x;
   double reach = 0.0;
   if (e < ne) {
@@ -288,6 +290,7 @@ __global__ void k_elem_geom(double *nodex, int ne, RP P, double4 *ecenter, doubl
 // with its total behind (one block; larger grids use CUB).
 constexpr int SCAN_CELLS = 16384;
 __global__ void __launch_bounds__(1024) k_scan_cells(const int *count, int na_cell, int ne_cell, int *astart, int *estart) {
+  behind_previous();
   __shared__ int warp_sum[32];
   __shared__ int carry, atoms;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = na_cell + ne_cell;
@@ -361,6 +364,7 @@ struct BinArgs {
 
 // Atoms and elements to their cells; the cells' near flags.
 __global__ void k_scatter(BinArgs B) {
+  behind_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < B.na) {
     B.aorder[B.astart[B.akey[i]] + B.aplace[i]] = i;
@@ -415,6 +419,7 @@ struct ElemBox {
 template <class RP>
 __global__ void k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *fixed, int *slot_atom, int *atom_slot,
                         int *slot_cell, const double4 *ecenter, const double *eframe, int *elems, ElemBox *boxes) {
+  behind_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < B.na) {
     const int cell = B.akey[i], k = cell_place(B.astart, B.aorder, cell, i);
@@ -2092,6 +2097,7 @@ void neigh_build_async(Ctx &c, bool want_half) {
     throw Error(CACB200_ESTATE, "rebuild without a capacity plan");
   const int nsi = c.nsite_i();
   with_reps(c, [&](auto P) {
+    using RP = decltype(P);
     {
       KernelTimer t(c, "pbc_geom");
       // the positions these lists are built from are kept for the displacement
@@ -2108,15 +2114,15 @@ void neigh_build_async(Ctx &c, bool want_half) {
       const int n = std::max(std::max(c.na, c.nrep), c.num_sms);
       k_pbc_atoms<<<nblk(n, 256), 256, 0, c.stream>>>(c.xs.p, c.na, P, S);
       if (c.ne)
-        k_elem_geom<<<nblk(c.ne, 64), 64, 0, c.stream>>>(c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
-                                                         c.reach_bits.p, c.overflow.p + 3, c.nodex_build.p,
-                                                         c.edisp.p, c.elem_key.p, c.elem_place.p, ecount);
+        launch_behind(c, nblk(c.ne, 64), 64, 0, k_elem_geom<RP>, c.nodex.p, c.ne, P, c.ecenter.p, c.eframe.p,
+                      c.reach_bits.p, c.overflow.p + 3, c.nodex_build.p, c.edisp.p, c.elem_key.p, c.elem_place.p,
+                      ecount);
     }
     {
       KernelTimer t(c, "bin");
       const int nac = c.agrid.ncell, nec = c.ne ? c.egrid.ncell : 0;
       if (nac + nec <= SCAN_CELLS) {
-        k_scan_cells<<<1, 1024, 0, c.stream>>>(c.cell_count.p, nac, nec, c.acell_start.p, c.ecell_start.p);
+        launch_behind(c, 1, 1024, 0, k_scan_cells, c.cell_count.p, nac, nec, c.acell_start.p, c.ecell_start.p);
       } else {
         size_t bytes = c.cub_bytes;
         CACB200_CUDA(cub::DeviceScan::ExclusiveSum(c.cub_tmp.p, bytes, c.cell_count.p, c.acell_start.p, nac + 1, c.stream));
@@ -2130,11 +2136,11 @@ void neigh_build_async(Ctx &c, bool want_half) {
                       near ? c.acell_near.p : nullptr, near ? c.ecell_near.p : nullptr,
                       c.rep_h[0].ag, c.rep_h[0].eg};
       const long n = (long)c.na + c.ne, cells = near ? (long)c.rep_h[0].ag.ncell + c.rep_h[0].eg.ncell : 0;
-      if (n + cells) k_scatter<<<nblk(n + cells, 256), 256, 0, c.stream>>>(B);
+      if (n + cells) launch_behind(c, nblk(n + cells, 256), 256, 0, k_scatter, B);
       if (n)
-        k_place<<<nblk(n, 256), 256, 0, c.stream>>>(B, P, c.xs.p, c.acell_pos.p, c.acell_fix.p, c.slot_atom.p,
-                                                    c.atom_slot.p, c.acell_of.p, c.ecenter.p, c.eframe.p,
-                                                    c.ecell_elems.p, (ElemBox *)c.ecell_box.p);
+        launch_behind(c, nblk(n, 256), 256, 0, k_place<RP>, B, P, c.xs.p, c.acell_pos.p, c.acell_fix.p, c.slot_atom.p,
+                      c.atom_slot.p, c.acell_of.p, c.ecenter.p, c.eframe.p, c.ecell_elems.p,
+                      (ElemBox *)c.ecell_box.p);
     }
     BuildArgs A;
     A.xs = c.xs.p;
@@ -2243,6 +2249,8 @@ void neigh_build_async(Ctx &c, bool want_half) {
       k_act_table<<<nblk(c.ne, 8), 256, 0, c.stream>>>(c.site_flag.p, c.ne, nsi, c.site_words.p, c.act_gid.p,
                                                        c.dev_nact.p, c.overflow.p + 7);
       const int grid = (int)std::min<long>(nblk((long)NG * c.ne + c.na, 32), (long)8 * c.num_sms);
+      // (a plain launch: blocks that wait for k_act_table's to end keep its
+      // last ones out; 12 replicas 3.09 ms a run plainly, 3.17 ms so)
       k_remap_sites<<<grid, 256, 0, c.stream>>>(c.raw_sites.p, c.items.p, c.item_cap, c.num_full.p, c.num_in.p,
                                                 c.site_from.p, nsi, c.cap, c.site_words.p, c.na, c.ne,
                                                 c.atom_work.p, c.atom_nwork.p, c.nbr_full.p);

@@ -81,7 +81,7 @@ __device__ __forceinline__ void walk(const PairArgs &A, int t, int i, const int 
   for (; left > 0; left -= 4) {
     double4 o[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) o[u] = ldg256(A.xs + (v[u] >> IMG_BITS));
+    for (int u = 0; u < 4; u++) o[u] = ld256(A.xs + (v[u] >> IMG_BITS));
     if (((v[0] ^ IMG_ZERO) | (v[1] ^ IMG_ZERO) | (v[2] ^ IMG_ZERO) | (v[3] ^ IMG_ZERO)) & ((1 << IMG_BITS) - 1)) {
       // images: an entry's image (0, 0, 0) leaves its position as it is
       const double *L = A.site_rep ? A.reps[A.site_rep[i]].b.L : A.L;
@@ -199,6 +199,7 @@ struct LjParams {
 
 template <int G, bool EV>
 __global__ void __launch_bounds__(128, EV ? 4 : 6) k_lj(PairArgs A, LjParams P) {
+  behind_previous();
   double red[7] = {0, 0, 0, 0, 0, 0, 0};
   for_each_slot<G>(A.nsi, [&](int t, bool valid) {
     const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
@@ -324,6 +325,7 @@ __device__ __forceinline__ void rho_slot(const PairArgs &A, const EamTables &T, 
 template <int TB, int G>
 __global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho(PairArgs A, EamTables T, double *rho_out,
                                                        double *phi_site) {
+  behind_previous();
   for_each_slot<G>(A.nsi, [&](int t, bool valid) { rho_slot<G>(A, T, t, valid, rho_out, phi_site); });
 }
 
@@ -342,6 +344,7 @@ __global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho(PairArgs A, EamTables
 template <int TB, int G>
 __global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho_sm(PairArgs A, EamTables T, double *rho_out,
                                                           double *phi_site, int *cnt, int nsm) {
+  behind_previous();
   __shared__ int v;
   if (threadIdx.x == 0) v = sm_id() % nsm;
   const int nrun = (A.nsi + TB / G - 1) / (TB / G);
@@ -357,6 +360,7 @@ __global__ void __launch_bounds__(TB, 1024 / TB) k_eam_rho_sm(PairArgs A, EamTab
 // (pair_eam.cpp:957-969)
 __global__ void k_eam_site_fp(double4 *xs, const int *act_gid, const int *nact_dev, int base, int na,
                               const double *rho, EamTables T) {
+  behind_previous();
   const int nact = *nact_dev;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nact; k += gridDim.x * blockDim.x) {
     int gid = act_gid[k];
@@ -408,6 +412,7 @@ __device__ __forceinline__ void force_slot(const PairArgs &A, const EamTables &T
 template <int TB, int G, bool EV>
 __global__ void __launch_bounds__(TB, (EV ? 512 : 768) / TB) k_eam_force(PairArgs A, EamTables T,
                                                                        const double *phi_site) {
+  behind_previous();
   double red[7] = {0, 0, 0, 0, 0, 0, 0};
   for_each_slot<G>(A.nsi, [&](int t, bool valid) { force_slot<G, EV>(A, T, t, valid, phi_site, red); });
   if (EV) block_reduce_store<7>(red, A.partial);
@@ -416,6 +421,7 @@ __global__ void __launch_bounds__(TB, (EV ? 512 : 768) / TB) k_eam_force(PairArg
 template <int TB, int G>
 __global__ void __launch_bounds__(TB, 640 / TB) k_eam_force_sm(PairArgs A, EamTables T, const double *phi_site,
                                                            int *cnt, int nsm) {
+  behind_previous();
   __shared__ int v;
   if (threadIdx.x == 0) v = sm_id() % nsm;
   const int nrun = (A.nsi + TB / G - 1) / (TB / G);
@@ -520,18 +526,18 @@ constexpr int TWO_LANE_SITES = 100000;
 // the trial launches change nothing).  Not during stream capture: there the
 // default stays.
 template <int G>
-void launch_rho(int tb, int nsi, cudaStream_t st, const PairArgs &A, const EamTables &T, double *rho, double *phi) {
+void launch_rho(const Ctx &c, int tb, int nsi, const PairArgs &A, const EamTables &T, double *rho, double *phi) {
   const int nb = std::max(nblk((long)nsi * G, tb), 1);
-  if (tb == 64) k_eam_rho<64, G><<<nb, 64, 0, st>>>(A, T, rho, phi);
-  else if (tb == 256) k_eam_rho<256, G><<<nb, 256, 0, st>>>(A, T, rho, phi);
-  else k_eam_rho<128, G><<<nb, 128, 0, st>>>(A, T, rho, phi);
+  const auto kernel = tb == 64 ? k_eam_rho<64, G> : tb == 256 ? k_eam_rho<256, G> : k_eam_rho<128, G>;
+  launch_behind(c, nb, tb, 0, kernel, A, T, rho, phi);
 }
 template <int G>
-void launch_force(int tb, int nsi, cudaStream_t st, const PairArgs &A, const EamTables &T, const double *phi) {
+void launch_force(const Ctx &c, int tb, int nsi, const PairArgs &A, const EamTables &T, const double *phi) {
   const int nb = std::max(nblk((long)nsi * G, tb), 1);
-  if (tb == 64) k_eam_force<64, G, false><<<nb, 64, 0, st>>>(A, T, phi);
-  else if (tb == 256) k_eam_force<256, G, false><<<nb, 256, 0, st>>>(A, T, phi);
-  else k_eam_force<128, G, false><<<nb, 128, 0, st>>>(A, T, phi);
+  const auto kernel = tb == 64    ? k_eam_force<64, G, false>
+                      : tb == 256 ? k_eam_force<256, G, false>
+                                  : k_eam_force<128, G, false>;
+  launch_behind(c, nb, tb, 0, kernel, A, T, phi);
 }
 
 template <class F>
@@ -621,8 +627,8 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
     KernelTimer t(c, "pair_lj");
     by_lanes([&](auto g) {
       constexpr int G = decltype(g)::value;
-      if (eflag || vflag) k_lj<G, true><<<nb_ev, T, 0, c.stream>>>(A, P);
-      else k_lj<G, false><<<nb, T, 0, c.stream>>>(A, P);
+      if (eflag || vflag) launch_behind(c, nb_ev, T, 0, k_lj<G, true>, A, P);
+      else launch_behind(c, nb, T, 0, k_lj<G, false>, A, P);
     });
   } else if (c.pp.style == CACB200_PAIR_EAM) {
     EamTables Tb;
@@ -640,14 +646,14 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
     const bool many = c.nrep > 1;
     auto site_fp = [&] {
       if (c.ne)
-        k_eam_site_fp<<<stride_grid((long)c.ne * NU, 256), 256, 0, c.stream>>>(
-            c.xss.p, c.act_gid.p, c.dev_nact.p, c.na + NG * c.ne, c.na, c.rho.p, Tb);
+        launch_behind(
+            c, stride_grid((long)c.ne * NU, 256), 256, 0, k_eam_site_fp, c.xss.p, c.act_gid.p, c.dev_nact.p, c.na + NG * c.ne, c.na, c.rho.p, Tb);
     };
     auto rho = [&](int tb) {
-      by_lanes([&](auto g) { launch_rho<decltype(g)::value>(tb, nsi, c.stream, A, Tb, c.rho.p, c.phi_site.p); });
+      by_lanes([&](auto g) { launch_rho<decltype(g)::value>(c, tb, nsi, A, Tb, c.rho.p, c.phi_site.p); });
     };
     auto force = [&](int tb) {
-      by_lanes([&](auto g) { launch_force<decltype(g)::value>(tb, nsi, c.stream, A, Tb, c.phi_site.p); });
+      by_lanes([&](auto g) { launch_force<decltype(g)::value>(c, tb, nsi, A, Tb, c.phi_site.p); });
     };
     // single systems of more than a wave of blocks: the force-only passes
     // over SM-local runs
@@ -702,7 +708,7 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
       KernelTimer t(c, "eam_force");
       if (eflag || vflag) {
         by_lanes([&](auto g) {
-          k_eam_force<128, decltype(g)::value, true><<<nb_ev, T, 0, c.stream>>>(A, Tb, c.phi_site.p);
+          launch_behind(c, nb_ev, T, 0, k_eam_force<128, decltype(g)::value, true>, A, Tb, c.phi_site.p);
         });
       } else if (smq) {
         force_s();

@@ -83,6 +83,7 @@ __device__ __forceinline__ void pack_pos(double px, double py, double pz, int k,
 // as fixed-point records, with no FP64 copy in between.
 __global__ void k_pair_table32(const double4 *xs, const int *slot_atom, const double *nodex, int na, int ne,
                                const int *act_gid, const int *nact_dev, FixGrid G, int4 *pos, int *bad) {
+  behind_previous();
   const int ngp = NG * ne;
   const int n = na + ngp + *nact_dev;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -157,7 +158,7 @@ __device__ __forceinline__ void walk32(const Args32 &A, int t, int i, const int4
   for (; left > 0; left -= 4) {
     int4 o[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) o[u] = __ldg(A.pos + (v[u] >> IMG_BITS));
+    for (int u = 0; u < 4; u++) o[u] = A.pos[v[u] >> IMG_BITS];
     // images: shift the neighbour by s L, s in {-1, 0, 1}, modulo 2^32
     if (((v[0] ^ IMG_ZERO) | (v[1] ^ IMG_ZERO) | (v[2] ^ IMG_ZERO) | (v[3] ^ IMG_ZERO)) & ((1 << IMG_BITS) - 1)) {
       const int *Lq = A.G.reps ? A.G.reps[A.G.site_rep[i]].Lq : A.G.Lq;
@@ -270,12 +271,13 @@ struct Lj32 {
 
 template <int G, bool EV>
 __global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj32(Args32 A, Lj32 P) {
+  behind_previous();
   double red[7] = {0, 0, 0, 0, 0, 0, 0};
   for_each_slot<G>(A.nsi, [&](int t, bool valid) {
     const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
     ForceSums<G, EV> S;
     if (valid) {
-      const int4 oi = __ldg(A.pos + t);
+      const int4 oi = A.pos[t];
       for_each32<G>(A, t, i, oi, [&](int part, float dx, float dy, float dz, float rsq, float) {
         if (rsq < P.cutsq) {
           const float r2inv = 1.0f / (rsq * (QUANTUM * QUANTUM));
@@ -389,13 +391,14 @@ template <int G, bool FAST>
 __global__ void __launch_bounds__(512, 2) k_eam_rho32(Args32 A, Eam32 T, double *rho_out, double *phi_site,
                                                       int4 *pos_w) {
   extern __shared__ float4 tab[];
-  if (FAST) load_fast(T, T.fast, 1, tab);
+  if (FAST) load_fast(T, T.fast, 1, tab);   // (constants: loaded while the kernel before ends)
+  behind_previous();
   const float4 *mine = tab + threadIdx.x % T.copies;
   for_each_slot<G>(A.nsi, [&](int t, bool valid) {
     const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
     Sum4<float, G> sum;
     if (valid) {
-      const int4 oi = __ldg(A.pos + t);
+      const int4 oi = A.pos[t];
       for_each32<G>(A, t, i, oi, [&](int part, float, float, float, float rsq, float) {
         float p, v = 0.0f;
         bool spline = rsq < T.cutforcesq;
@@ -428,6 +431,7 @@ __global__ void __launch_bounds__(512, 2) k_eam_rho32(Args32 A, Eam32 T, double 
 
 __global__ void k_eam_site_fp32(int4 *pos, const int *act_gid, const int *nact_dev, int base, int na,
                                 const double *rho, Eam32 T) {
+  behind_previous();
   const int nact = *nact_dev;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nact; k += gridDim.x * blockDim.x) {
     int gid = act_gid[k];
@@ -445,6 +449,7 @@ template <int G, bool FAST, bool EV>
 __global__ void __launch_bounds__(512, EV ? 1 : 2) k_eam_force32(Args32 A, Eam32 T, const double *phi_site) {
   extern __shared__ float4 tab[];
   if (FAST) load_fast(T, T.fast + T.cnt + 1, 2, tab);
+  behind_previous();
   const float4 *mine = tab + threadIdx.x % T.copies;
   const int second = (T.cnt + 1) * T.copies;
   double red[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -452,7 +457,7 @@ __global__ void __launch_bounds__(512, EV ? 1 : 2) k_eam_force32(Args32 A, Eam32
     const int i = valid ? site_of_slot(A, t) : 0;           // site-table index
     ForceSums<G, EV> S;
     if (valid) {
-      const int4 oi = __ldg(A.pos + t);
+      const int4 oi = A.pos[t];
       const float fpi = __int_as_float(oi.w);
       for_each32<G>(A, t, i, oi, [&](int part, float dx, float dy, float dz, float rsq, float fpj) {
         float p, g = 0.0f, h = 0.0f, phi = 0.0f;
@@ -650,9 +655,8 @@ void pair_table_mixed(Ctx &c) {
   FixGrid G = make_fix_grid(c);
   // 64 blocks per SM: the item loop's loads are in flight across more
   // threads than stride_grid's 16 blocks give (0.193 -> 0.181 ms on config 3)
-  k_pair_table32<<<std::min(nblk(ns, 256), 148 * 64), 256, 0, c.stream>>>(c.xs.p, c.slot_atom.p, c.nodex.p, c.na, c.ne,
-                                                             c.act_gid.p, c.dev_nact.p, G, c.pos32.p,
-                                                             c.overflow.p + 6);
+  launch_behind(c, std::min(nblk(ns, 256), 148 * 64), 256, 0, k_pair_table32, c.xs.p, c.slot_atom.p, c.nodex.p,
+                c.na, c.ne, c.act_gid.p, c.dev_nact.p, G, c.pos32.p, c.overflow.p + 6);
 }
 
 void mixed_tables(Ctx &c) {
@@ -727,8 +731,8 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
     grid_ev = std::min(need, c.num_sms * 8);
     by_lanes([&](auto g) {
       constexpr int GL = decltype(g)::value;
-      if (ev) k_lj32<GL, true><<<grid_ev, 128, 0, c.stream>>>(A, P);
-      else k_lj32<GL, false><<<need, 128, 0, c.stream>>>(A, P);
+      if (ev) launch_behind(c, grid_ev, 128, 0, k_lj32<GL, true>, A, P);
+      else launch_behind(c, need, 128, 0, k_lj32<GL, false>, A, P);
     });
   } else {
     if (!c.have_mixed_tables) {
@@ -768,7 +772,7 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
     auto go = [&](auto kernel, int blocks, size_t bytes, auto... args) {
       if (bytes > 48 * 1024)
         CACB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-      kernel<<<blocks, tb, bytes, c.stream>>>(A, Tb, args...);
+      launch_behind(c, blocks, tb, bytes, kernel, A, Tb, args...);
     };
     {
       KernelTimer t(c, "eam_rho32");
@@ -780,8 +784,8 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
     }
     if (c.ne) {
       KernelTimer t(c, "eam_site_fp32");
-      k_eam_site_fp32<<<stride_grid((long)c.ne * NU, 256), 256, 0, c.stream>>>(
-          c.pos32.p, c.act_gid.p, c.dev_nact.p, c.na + NG * c.ne, c.na, c.rho.p, Tb);
+      launch_behind(
+          c, stride_grid((long)c.ne * NU, 256), 256, 0, k_eam_site_fp32, c.pos32.p, c.act_gid.p, c.dev_nact.p, c.na + NG * c.ne, c.na, c.rho.p, Tb);
     }
     {
       KernelTimer t(c, "eam_force32");
