@@ -312,8 +312,9 @@ class Engine:
         return r.value, f.value
 
     def work_queue(self, enable=None):
-        """Batches (mixed form): turn the persistent work-queue launches on or
-        off (None: unchanged); returns the tiles chosen per size class."""
+        """Turn the persistent launches of the EAM passes and the atom build on
+        or off (None: unchanged); returns the slots per block of a batch's mixed
+        passes for each size class (0: not run yet)."""
         t = (C.c_int * 3)()
         self._check(self.lib.cacb200_work_queue(self.h, -1 if enable is None else int(bool(enable)), t),
                     "work_queue")

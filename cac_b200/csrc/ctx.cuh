@@ -442,8 +442,8 @@ inline void note_build_box(Ctx &c) {
 // launch); the kernel waits for that one itself (behind_previous, device.cuh).
 // A step of a small system is a chain of kernels of a few us each, which plain
 // launches put about 1 us apart: 6 k sites 31.7 -> 29.5 us a step with its share
-// of the rebuilds, 84 k sites in the mixed form 1.87 -> 1.66 ms for 25 steps, FIRE
-// at 93 k sites 9.88 -> 9.12 ms for 50 iterations.  Above
+// of the rebuilds, 25 mixed LJ steps of 84 k sites 1.87 -> 1.66 ms (with the LJ
+// pass of that time), FIRE at 93 k sites 9.88 -> 9.12 ms for 50 iterations.  Above
 // BEHIND_SITES the gaps are nothing and blocks that wait only take room from
 // those at work (1.21 M sites, 20 steps: 27.04 ms plainly, 26.86 ms so; 1.7 M
 // 29.65 and 29.72; 5 M 59.1 and 59.6).
