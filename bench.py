@@ -954,8 +954,8 @@ def main():
                     help="steps per trajectory from the seeded initial state (the reference's CAC "
                          "dynamics heat up unboundedly after ~100 steps, so long runs restart)")
     ap.add_argument("--work-queue", default="on", choices=["on", "off"],
-                    help="mixed EAM passes as persistent launches (batches: work items per replica; "
-                         "single systems: SM-local runs of list slots) or one grid launch per pass")
+                    help="mixed EAM passes as resident blocks, and a single system's atom build and FP64 passes "
+                         "over SM-local runs, or one grid launch per pass")
     ap.add_argument("--prefix-margin", type=float, default=None,
                     help="margin of the lists' inner prefix in A (default: the library's, 0.5 x skin; 0: off)")
     args = ap.parse_args()

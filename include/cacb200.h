@@ -421,27 +421,23 @@ int cacb200_set_graphs(cacb200_ctx *ctx, int enable);
 /* graph launches made so far by this context */
 int cacb200_graph_launches(cacb200_ctx *ctx, long long *count);
 /* Block sizes (threads) of the force-only EAM passes of the current precision
- * form: chosen per context by timing 64, 128 and 256 threads on the
- * context's own lists the first time they run (results do not depend on the
- * choice); 128 before that.  No reference counterpart. */
+ * form.  FP64 batches: chosen per context by timing 64, 128 and 256 threads on
+ * the context's own lists the first time they run (results do not depend on the
+ * choice); otherwise 128.  Mixed form: 128 in small systems, else 512, after the
+ * first evaluation.  No reference counterpart. */
 int cacb200_pair_blocks(cacb200_ctx *ctx, int *rho_threads, int *force_threads);
-/* Batches in the mixed form run the EAM passes as persistent work-queue
- * launches: resident blocks take items (a run of consecutive list slots of
- * one replica, the largest replicas first) from a counter, so one launch
- * serves replicas of every size without idle tails.  The run length (tile:
- * 128, 512 or 2048 slots) is chosen per replica size class (i-sites below
- * 8,192, below 32,768, larger) by timing the force pass when the capacity
- * plan changes; results do not depend on it (each slot's arithmetic is that
- * of the grid launch).  Single systems run the atom-list build, and in the
- * FP64 form the force-only EAM passes, over SM-local runs instead: the
- * sorted atoms or list slots are cut into runs (32 atoms; 128 slots) and each
+/* Persistent launches.  The EAM passes of the mixed form (small systems aside)
+ * run as resident blocks of 512 threads that stride over the list slots.
+ * Single systems run the atom-list build, and in the FP64 form the force-only
+ * EAM passes of systems from 100,000 i-sites up, over SM-local runs: the sorted
+ * atoms or list slots are cut into runs (32 atoms; 64 slots) and each
  * multiprocessor owns a contiguous range of runs, so the blocks resident on
  * one multiprocessor share their neighbours' data in its L1; a block whose
  * own range is exhausted takes runs from another range (same lists and
  * results as the grid launches, bit for bit).  enable: 1 on (default), 0 off
- * (one grid launch per pass), -1 unchanged; tiles [3] gets the chosen tiles
- * of batches (0: not chosen yet).  No reference counterpart (the reference
- * runs one system per process). */
+ * (one grid launch per pass), -1 unchanged; tiles [3] gets 512 for batches
+ * after their first mixed EAM evaluation (0 before).  No reference counterpart
+ * (the reference runs one system per process). */
 int cacb200_work_queue(cacb200_ctx *ctx, int enable, int tiles[3]);
 
 /* Kernel timing: when enabled, every launch is bracketed by CUDA events and
