@@ -115,7 +115,8 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Pair passes.  A site's sums are kept in four partial sums: entry k of a
+// Pair passes (but the mixed LJ one, pair32.cu, which keeps one running sum).
+// A site's sums are kept in four partial sums: entry k of a
 // walk goes to partial k mod 4, and the partials are added as (0 + 1) + (2 +
 // 3).  G lanes share a site (G = 1, 2 or 4; lane g walks entries g, g + G,
 // ...) and each holds 4 / G of the partials, so a site's result is the same

@@ -24,9 +24,9 @@
 // pair-table index (atoms by list slot) with its image; a site's entries
 // inside the inner radius at build time fill its list from row 0 up, the
 // others from row cap-1 down, so no pass reorders them.  Element-site entries
-// are first written as lattice-site ids (the pair-table index of a lattice
-// site is known only once every list has marked the sites it uses) and
-// converted by k_remap_sites.  Half lists (read only by the list download)
+// are first written as (item, lattice site) along their query's own row (the
+// pair-table index of a lattice site is known only once every list has marked
+// the sites it uses) and converted by k_remap_sites.  Half lists (read only by the list download)
 // are written as raw entries and compacted by k_remap.
 //
 // Storage rules (the reference's, restated):
