@@ -395,11 +395,18 @@ __device__ __forceinline__ int cell_place(const int *start, const int *order, in
 }
 
 // Fixed-point copy of a wrapped atom position for the screen of the atom build: quanta of
-// 2^-20 A from the box corner, modulo 2^32 (4096 A), so that the differences
-// of near positions are exact integers whatever the size of the box.  An atom
+// 2^-20 A from the box corner, modulo 2^32 (4096 A).  The differences of
+// positions less than 2048 A apart are exact integers whatever the size of the
+// box; the build takes no positions together that could be further apart
+// (PART_SPAN; WIDE_CELL where the cells themselves are that large).  An atom
 // that is not in or near the box (a run that has blown up) gets FAR_ATOM and
 // is nobody's neighbour.
 constexpr int FAR_ATOM = 0x80000000;
+// A chunk's atoms are taken together over at most PART_SPAN A of their row of
+// cells.  With the cells to either side, each up to WIDE_CELL A wide, a
+// position lies within 1000 + 3 x 256 A of the part's first cell and of every
+// other one of the part: well inside 2048.
+constexpr double PART_SPAN = 1000.0, WIDE_CELL = 256.0;
 constexpr float QUANTUM = 1.0f / 1048576.0f;
 __device__ __forceinline__ int fix20(double x) { return (int)(unsigned)(unsigned long long)__double2ll_rn(x * 1048576.0); }
 
@@ -487,6 +494,7 @@ struct BuildArgs {
   double cutneigh, cutneighsq;
   double cutforcesq;          // pairs inside the inner radius (force cutoff + margin) at build time go first
   int want_half;
+  int wide;                   // cells wider than WIDE_CELL: no fixed-point screen of atoms
   int *nbr_full;              // final full-list entries (atoms; element sites after k_remap_sites)
   int *num_in;                // per slot: entries in the front segment
   int2 *site_from;            // per slot: front / back rows before the element-site entries
@@ -1218,8 +1226,9 @@ __device__ __forceinline__ unsigned f2_signs(unsigned mask, F2 v) {
 // Atoms, atom neighbours: one block per chunk of 32 consecutive sorted atoms
 // (list slots), the atoms as lanes.  Cells (>= cutneigh) are sorted x
 // fastest, so a chunk lies in one row of cells, or in two at a row's end
-// (then the warps take the two parts in turn).  For each of the 9 rows around
-// the part's row the candidates are the cells from one left of the part's
+// (then the warps take the two parts in turn); where atoms are so few that a
+// chunk spans more than PART_SPAN of its row, in as many parts as that takes.
+// For each of the 9 rows around the part's row the candidates are the cells from one left of the part's
 // first cell to one right of its last, as at most three runs of consecutive
 // cells under one image (the left and right wraps and the middle).  A lane
 // meets the cells of its own 27-cell block in the order a walk of that block
@@ -1279,7 +1288,9 @@ __device__ __forceinline__ void build_atoms_chunk(const BuildArgs &A, const RP &
     const int nc0 = R.ag.nc[0], nc1 = R.ag.nc[1], nc2 = R.ag.nc[2];
     const int row = (lkey - R.abase) / nc0;   // cz * nc1 + cy of the part
     const int hx = key - R.abase - row * nc0;
-    const bool active = mine && ((todo >> lane) & 1u) && hx >= 0 && hx < nc0;
+    // no further along the row than PART_SPAN from its first atom's cell
+    const int hx0 = lkey - R.abase - row * nc0;
+    const bool active = mine && ((todo >> lane) & 1u) && hx >= 0 && hx < nc0 && (hx - hx0) <= PART_SPAN * R.ag.inv[0];
     todo &= ~__ballot_sync(0xffffffffu, active);
     const int hy = row % nc1, hz = row / nc1;
     // unwrapped x range of the candidate cells
@@ -1359,7 +1370,7 @@ __device__ __forceinline__ void build_atoms_chunk(const BuildArgs &A, const RP &
       z = (float)(int)(uz - oz) * QUANTUM;
       const float dx = fmaxf(fmaxf(bx0 - x, x - bx1), 0.0f), dy = fmaxf(fmaxf(by0 - y, y - by1), 0.0f),
                   dz = fmaxf(fmaxf(bz0 - z, z - bz1), 0.0f);
-      return c.x != FAR_ATOM && dx * dx + dy * dy + dz * dz <= reach2;
+      return c.x != FAR_ATOM && (A.wide || dx * dx + dy * dy + dz * dz <= reach2);
     };
     auto keep = [&](unsigned m, int at, int k, int code, float x, float y, float z) {
       at += __popc(m & lanemask_lt());
@@ -1452,10 +1463,11 @@ __device__ __forceinline__ void build_atoms_chunk(const BuildArgs &A, const RP &
         if (unwrapped && self >= 0 && (self >> 5) == w) valid &= ~(0x80000000u >> (self & 31));
         mp &= valid;
         unsigned acc = ms & mp, in = mi & acc, band = mp & ~acc;
-        if (A.want_half || !unwrapped) {
+        if (A.want_half || A.wide || !unwrapped) {
           // half lists, and atoms outside the box, take every candidate
-          // through the exact test, in order
-          band = mp;
+          // through the exact test, in order (in wide cells even those that
+          // the screen drops)
+          band = A.wide ? valid : mp;
           acc = in = 0;
         }
         while (band) {
@@ -2170,6 +2182,10 @@ void neigh_build_async(Ctx &c, bool want_half) {
     A.cutneighsq = c.cutneighsq;
     A.cutforcesq = (c.pp.cut + c.inner_margin) * (c.pp.cut + c.inner_margin);
     A.want_half = want_half ? 1 : 0;
+    A.wide = 0;
+    for (const Rep &R : c.rep_h)
+      for (int d = 0; d < 3; d++)
+        if (R.ag.inv[d] * WIDE_CELL < 1.0) A.wide = 1;
     A.nbr_full = c.nbr_full.p;
     A.num_in = c.num_in.p;
     A.site_from = c.site_from.p;
