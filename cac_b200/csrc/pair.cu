@@ -241,18 +241,20 @@ struct EamTables {
 // Distance and its reciprocal from the square: rsqrt carries at most one ulp,
 // as the reciprocal of a rounded square root does, and one step of Newton's
 // method takes r = rsq / sqrt(rsq) to within rounding of the square root.
+// Sites on one another (the square's high word is 0 below 2e-314) are 0 apart
+// (0 x inf would be no number), with an infinite reciprocal.
 __device__ __forceinline__ double distance(double rsq, double &recip) {
   recip = rsqrt(rsq);
   const double r = rmul(rsq, recip);
-  return fma(fma(-r, r, rsq), rmul(0.5, recip), r);
+  return __double2hiint(rsq) ? fma(fma(-r, r, rsq), rmul(0.5, recip), r) : 0.0;
 }
 
 // The knot of distance r and the place p in its interval, as the reference's
-// m = int(r / dr + 1), limited to nr - 1, and p = min(r / dr + 1 - m, 1): the
+// m = int(r / dr + 1), limited to 1 .. nr - 1, and p = min(r / dr + 1 - m, 1): the
 // truncation is a fused operation rounded down at 2^52.
 __device__ __forceinline__ int r_knot(const EamTables &T, double r, double &p) {
   const double x = __fma_rd(r, T.rdr, 4503599627370497.0);   // 2^52 + 1
-  int m = __double2loint(x);
+  int m = max(__double2loint(x), 1);
   p = fma(r, T.rdr, rsub(4503599627370497.0, x));
   if (m >= T.nr) {
     m = T.nr - 1;
