@@ -378,6 +378,8 @@ __global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj32(Args32 A, Lj32 P) {
 // spline record from global memory as many, from eight copies in shared memory
 // four; with four copies the force pass is 17 % slower).  4.98 M sites: density
 // 1.047 -> 0.73 ms, force 1.170 -> 0.88 ms; 313 k: 91 -> 60 and 96 -> 70 us.
+constexpr int FAST_INTERVALS[] = {192, 256, 384, 512}, FAST_COPIES = 8;
+constexpr size_t FAST_BYTES = sizeof(float4) * (512 + 1) * FAST_COPIES;   // the most that one function takes
 struct Eam32 {
   const float4 *rz, *frho_val, *frho_der;
   float rdr, rdrho, rhomax, cutforcesq;      // cutforcesq in square quanta
@@ -688,7 +690,7 @@ void eam_fast_tables(Ctx &c, const std::vector<double4> &rz) {
   c.fast_cnt = 0;
   const HostSpline rho{rz, 0, c.pp.nr, c.pp.rdr}, z{rz, 1, c.pp.nr, c.pp.rdr};
   std::vector<float4> rec[3];
-  for (int n : {192, 256, 384, 512})
+  for (int n : FAST_INTERVALS)
     for (double top : {c.pp.cut, c.pp.cut - 4.0 * c.pp.dr}) {
       if (!(top > 0.5 * c.pp.cut)) continue;
       float inv_ds;
@@ -706,6 +708,19 @@ void eam_fast_tables(Ctx &c, const std::vector<double4> &rz) {
       stream_copy(c, c.fast32.p, out.data(), sizeof(float4) * out.size(), cudaMemcpyHostToDevice);
       return;
     }
+}
+
+// The limit on a kernel's shared memory belongs to the kernel on the device,
+// which every context of the process launches: it is the most that any table
+// can need, so no context lowers what another is about to launch with.
+void allow_fast_records() {
+  auto one = [](auto kernel, size_t bytes) {
+    CACB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  };
+  auto allow = [&](size_t bytes, auto... kernels) { (one(kernels, bytes), ...); };
+  allow(FAST_BYTES, k_eam_rho32<1, true>, k_eam_rho32<2, true>, k_eam_rho32<4, true>);
+  allow(2 * FAST_BYTES, k_eam_force32<1, true, false>, k_eam_force32<2, true, false>, k_eam_force32<4, true, false>,
+        k_eam_force32<1, true, true>, k_eam_force32<2, true, true>, k_eam_force32<4, true, true>);
 }
 
 }  // namespace
@@ -732,6 +747,7 @@ void mixed_tables(Ctx &c) {
     return h;
   };
   eam_fast_tables(c, conv(c.rz, c.rz32, 2 * c.pp.nr + 1));
+  if (c.fast_cnt) allow_fast_records();
   conv(c.frho_val, c.frho_val32, c.pp.nrho);
   conv(c.frho_der, c.frho_der32, c.pp.nrho);
 }
@@ -817,7 +833,7 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
     const long threads = (long)nsi * lanes;
     const bool small = threads < (long)c.num_sms * 512;
     const int tb = small ? 128 : 512;
-    Tb.copies = small ? 1 : 8;
+    Tb.copies = small ? 1 : FAST_COPIES;
     const int need = std::max(nblk(threads, tb), 1);
     const int grid = c.work_queue && !small ? std::min(need, 2 * c.num_sms) : need;
     grid_ev = std::min(need, small ? c.num_sms * 8 : c.num_sms);
@@ -827,8 +843,6 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
     const bool fast = c.fast_cnt > 0;
     const size_t rec = fast ? sizeof(float4) * (size_t)(c.fast_cnt + 1) * Tb.copies : 0;
     auto go = [&](auto kernel, int blocks, size_t bytes, auto... args) {
-      if (bytes > 48 * 1024)
-        CACB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
       launch_behind(c, blocks, tb, bytes, kernel, A, Tb, args...);
     };
     {
