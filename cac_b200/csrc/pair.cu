@@ -661,23 +661,20 @@ void pair_compute(Ctx &c, int eflag, int vflag) {
     // over SM-local runs
     const bool smq = !many && c.work_queue && lanes == 2;
     c.sm_counter.reserve(2 * c.num_sms);
-    auto sm_grid = [&](auto kernel, int &cache) {
-      if (!cache) {
-        int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 128, 0);
-        cache = (b > 0 ? b : 1) * c.num_sms;
-      }
-      return cache;
+    auto resident = [](auto kernel) {
+      int b = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 128, 0);
+      return b > 0 ? b : 1;
     };
-    static int grid_rho_sm = 0, grid_force_sm = 0;
+    static const int per_sm_rho = resident(k_eam_rho_sm<128, 2>), per_sm_force = resident(k_eam_force_sm<128, 2>);
     auto rho_s = [&] {
       CACB200_CUDA(cudaMemsetAsync(c.sm_counter.p, 0, sizeof(int) * c.num_sms, c.stream));
-      k_eam_rho_sm<128, 2><<<sm_grid(k_eam_rho_sm<128, 2>, grid_rho_sm), 128, 0, c.stream>>>(
+      k_eam_rho_sm<128, 2><<<per_sm_rho * c.num_sms, 128, 0, c.stream>>>(
           A, Tb, c.rho.p, c.phi_site.p, c.sm_counter.p, c.num_sms);
     };
     auto force_s = [&] {
       CACB200_CUDA(cudaMemsetAsync(c.sm_counter.p + c.num_sms, 0, sizeof(int) * c.num_sms, c.stream));
-      k_eam_force_sm<128, 2><<<sm_grid(k_eam_force_sm<128, 2>, grid_force_sm), 128, 0, c.stream>>>(
+      k_eam_force_sm<128, 2><<<per_sm_force * c.num_sms, 128, 0, c.stream>>>(
           A, Tb, c.phi_site.p, c.sm_counter.p + c.num_sms, c.num_sms);
     };
     if (many && c.tune_gen != c.gen && !eflag && !vflag && !capturing(c.stream)) {
