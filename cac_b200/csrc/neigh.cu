@@ -93,6 +93,19 @@ __device__ __forceinline__ int grid_cell(const Grid &g, const BoxD &b, const dou
   return (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
 }
 
+__device__ __forceinline__ void wrap_cell(int v, int nc, int &cell, int &W) {
+  W = 0;
+  while (v < 0) {
+    v += nc;
+    W--;
+  }
+  while (v >= nc) {
+    v -= nc;
+    W++;
+  }
+  cell = v;
+}
+
 // What a rebuild starts from, cleared by its first kernel.
 struct BuildStart {
   double4 *xbuild;      // the wrapped positions the lists are built from (null: only wrap)
@@ -360,6 +373,8 @@ struct BinArgs {
   int na, ne;
   unsigned char *anear, *enear;     // single systems with elements (else null)
   Grid ag, eg;
+  float reach;                      // cutneigh
+  int *bad_image;                   // flag (null while half lists are built)
 };
 
 // Atoms and elements to their cells; the cells' near flags.
@@ -399,8 +414,8 @@ __device__ __forceinline__ int cell_place(const int *start, const int *order, in
 // positions less than 2048 A apart are exact integers whatever the size of the
 // box; the build takes no positions together that could be further apart
 // (PART_SPAN; WIDE_CELL where the cells themselves are that large).  An atom
-// that is not in or near the box (a run that has blown up) gets FAR_ATOM and
-// is nobody's neighbour.
+// further than WIDE_CELL (or a box length) outside the box gets FAR_ATOM and is
+// nobody's neighbour (but see refuse_far_images).
 constexpr int FAR_ATOM = 0x80000000;
 // A chunk's atoms are taken together over at most PART_SPAN A of their row of
 // cells.  With the cells to either side, each up to WIDE_CELL A wide, a
@@ -420,12 +435,54 @@ struct ElemBox {
   float4 centre, row[3], norm;
 };
 
+// An atom that is outside the box after the wrap (positions given boxes away,
+// or a run that has blown up): is another one within reach under an image that
+// no list entry can hold?  Then the build is refused.  The screen of the atom
+// build knows the images of atoms inside the box only.
+template <class RP>
+__device__ void refuse_far_images(const BinArgs &B, const RP &P, const double4 *xs, int i) {
+  const Rep r = P.site(i);
+  const double4 p = xs[i];
+  const double px[3] = {p.x, p.y, p.z};
+  int c = B.akey[i] - r.abase, at[3], t[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    at[d] = c % r.ag.nc[d];
+    c /= r.ag.nc[d];
+    t[d] = -(int)floor((px[d] - r.b.lo[d]) / r.b.L[d]);
+  }
+#pragma unroll 1
+  for (int k = 0; k < 27; k++) {
+    const int o[3] = {k % 3 - 1, k / 3 % 3 - 1, k / 9 - 1};
+    int cell[3], W[3];
+    float q[3];
+    bool held = true;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      wrap_cell(at[d] + o[d], r.ag.nc[d], cell[d], W[d]);
+      held = held && abs(W[d] - t[d]) <= 1;
+    }
+    if (held) continue;
+    const int m = r.abase + (cell[2] * r.ag.nc[1] + cell[1]) * r.ag.nc[0] + cell[0];
+#pragma unroll 1
+    for (int u = B.astart[m]; u < B.astart[m + 1]; u++) {
+      if (*(volatile int *)B.bad_image) return;
+      const double4 x = xs[B.aorder[u]];
+      q[0] = (float)(px[0] - (x.x + W[0] * r.b.L[0]));
+      q[1] = (float)(px[1] - (x.y + W[1] * r.b.L[1]));
+      q[2] = (float)(px[2] - (x.z + W[2] * r.b.L[2]));
+      if (B.aorder[u] != i && q[0] * q[0] + q[1] * q[1] + q[2] * q[2] <= B.reach * B.reach) *B.bad_image = 1;
+    }
+  }
+}
+
 // The sorted atoms: positions (w = atom index), the fixed-point copies of the
 // screen (x, y, z parts na apart), slots and cells; and the sorted elements
 // with their boxes.
 template <class RP>
-__global__ void k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *fixed, int *slot_atom, int *atom_slot,
-                        int *slot_cell, const double4 *ecenter, const double *eframe, int *elems, ElemBox *boxes) {
+__global__ void __launch_bounds__(256, RP::many ? 6 : 8)
+    k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *fixed, int *slot_atom, int *atom_slot, int *slot_cell,
+            const double4 *ecenter, const double *eframe, int *elems, ElemBox *boxes) {
   behind_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < B.na) {
@@ -437,10 +494,12 @@ __global__ void k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *f
     const BoxD b = P.site(i).b;
     const double q[3] = {p.x, p.y, p.z};
     int f[3];
-    bool near = true;
+    bool near = true, in = true;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      near = near && q[d] >= b.lo[d] - b.L[d] && q[d] <= b.hi[d] + b.L[d];
+      in = in && q[d] >= b.lo[d] && q[d] < b.hi[d];
+      const double m = fmin(b.L[d], WIDE_CELL);
+      near = near && q[d] >= b.lo[d] - m && q[d] <= b.hi[d] + m;
       f[d] = fix20(q[d] - b.lo[d]);
     }
     if (f[0] == FAR_ATOM) f[0]++;
@@ -449,6 +508,7 @@ __global__ void k_place(BinArgs B, RP P, const double4 *xs, double4 *out, int *f
     fixed[k + 2 * (size_t)B.na] = f[2];
     p.w = __longlong_as_double((long long)i);
     out[k] = p;
+    if (!in && B.bad_image) refuse_far_images(B, P, xs, i);
     return;
   }
   i -= B.na;
@@ -631,19 +691,6 @@ __device__ __forceinline__ void try_atom(const BuildArgs &A, const Query &q, int
     bool keep = ord > 0 || (ord == 0 && (zero ? (j > q.i) : above_right(qq, q.xi)));
     if (keep) emit(A, q.slot, nh, A.raw_half, A.img_half, j, code);
   }
-}
-
-__device__ __forceinline__ void wrap_cell(int v, int nc, int &cell, int &W) {
-  W = 0;
-  while (v < 0) {
-    v += nc;
-    W--;
-  }
-  while (v >= nc) {
-    v -= nc;
-    W++;
-  }
-  cell = v;
 }
 
 // Element lattice sites are found in two phases.  Phase A (one thread per
@@ -2146,7 +2193,7 @@ void neigh_build_async(Ctx &c, bool want_half) {
       const BinArgs B{c.atom_key.p,  c.atom_place.p, c.acell_start.p, c.elem_key.p, c.elem_place.p,
                       c.ecell_start.p, c.atom_order.p, c.elem_order.p, c.na,         c.ne,
                       near ? c.acell_near.p : nullptr, near ? c.ecell_near.p : nullptr,
-                      c.rep_h[0].ag, c.rep_h[0].eg};
+                      c.rep_h[0].ag, c.rep_h[0].eg, (float)c.cutneigh, want_half ? nullptr : c.overflow.p + 2};
       const long n = (long)c.na + c.ne, cells = near ? (long)c.rep_h[0].ag.ncell + c.rep_h[0].eg.ncell : 0;
       if (n + cells) launch_behind(c, nblk(n + cells, 256), 256, 0, k_scatter, B);
       if (n)

@@ -65,3 +65,23 @@ def test_cells_wider_than_the_fixed_point_screen_covers(oracle_mod):
     assert np.array_equal(e.neighbor_list(), oracle_mod.build_list(st, 720.0, False).canonical(s.natoms))
     assert np.array_equal(e.neighbor_list(half=True), oracle_mod.build_list(st, 720.0, True).canonical(s.natoms))
     e.close()
+
+
+@pytest.mark.parametrize("boxes", [3, 4, -3])
+@pytest.mark.parametrize("axes", [(2,), (0, 1, 2)])
+def test_positions_boxes_away_are_refused(boxes, axes):
+    """Atoms without elements whose positions are given several box lengths
+    away, where one wrap leaves them outside: their neighbours stand under
+    images that list entries cannot hold, and the build says so."""
+    from cac_b200.api import CacB200Error, Engine
+    s = gen.build_slab(3, 1, 1, 6, temperature=10.0, seed=1)
+    s.nodex, s.nodev = s.nodex[:0], s.nodev[:0]
+    for d in axes:
+        s.x[:, d] += boxes * (s.boxhi - s.boxlo)[d]
+    e = Engine(0)
+    e.upload(s)
+    e.pair_lj(0.4093, 2.338, 5.5)
+    e.neighbor(1.0, 10)
+    with pytest.raises(CacB200Error, match="image"):
+        e.build_lists()
+    e.close()
