@@ -364,9 +364,9 @@ __global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj32(Args32 A, Lj32 P) {
 //
 // Beside them the smooth part of the same splines as functions of s = r^2,
 // which a pair needs no square root for: the density rho, and the two terms
-// of the force over r, rho'/r and phi'/r, each a cubic in s on intervals of
-// equal width (eam_fast_tables: fitted to the splines to 2e-8 of their local
-// size, a third of an FP32 rounding, or not used).  Their records, 16 bytes
+// of the force over r, rho'/r and phi'/r, and for tallies phi, each a cubic in s
+// on intervals of equal width (eam_fast_tables: fitted to the splines to 2e-8 of
+// their local size, a third of an FP32 rounding, and phi to 4e-8, or not used).  Their records, 16 bytes
 // per function, cover the intervals [lo, lo + cnt) and are few enough to be
 // held in shared memory `copies` times over, lane l reading copy l % copies:
 // with eight copies a warp's gather has no bank conflict, and L1 keeps the
@@ -378,13 +378,15 @@ __global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj32(Args32 A, Lj32 P) {
 // spline record from global memory as many, from eight copies in shared memory
 // four; with four copies the force pass is 17 % slower).  4.98 M sites: density
 // 1.047 -> 0.73 ms, force 1.170 -> 0.88 ms; 313 k: 91 -> 60 and 96 -> 70 us.
+// With tallies: 313 k sites 123 -> 96 us, 1.21 M 417 -> 310 us (133 and 489 us
+// where phi was read from the splines beside the records).
 constexpr int FAST_INTERVALS[] = {192, 256, 384, 512}, FAST_COPIES = 8;
 constexpr size_t FAST_BYTES = sizeof(float4) * (512 + 1) * FAST_COPIES;   // the most that one function takes
 struct Eam32 {
   const float4 *rz, *frho_val, *frho_der;
   float rdr, rdrho, rhomax, cutforcesq;      // cutforcesq in square quanta
   int nr, nrho;
-  const float4 *fast;                        // [3][cnt + 1]: rho, rho'/r, phi'/r
+  const float4 *fast;                        // [4][cnt + 1]: rho, rho'/r, phi'/r, phi
   float inv_ds;                              // intervals per square quantum
   int base, cnt, copies;                     // base: bits of 2^23 + the first interval
 };
@@ -512,7 +514,7 @@ __global__ void k_eam_site_fp32(int4 *pos, const int *act_gid, const int *nact_d
 template <int G, bool FAST, bool EV>
 __global__ void __launch_bounds__(512, EV ? 1 : 2) k_eam_force32(Args32 A, Eam32 T, const double *phi_site) {
   extern __shared__ float4 tab[];
-  if (FAST) load_fast(T, T.fast + T.cnt + 1, 2, tab);
+  if (FAST) load_fast(T, T.fast + T.cnt + 1, EV ? 3 : 2, tab);
   behind_previous();
   const float4 *mine = tab + threadIdx.x % T.copies;
   const int second = (T.cnt + 1) * T.copies;
@@ -525,20 +527,15 @@ __global__ void __launch_bounds__(512, EV ? 1 : 2) k_eam_force32(Args32 A, Eam32
       const float fpi = __int_as_float(oi.w);
       for_each32<G>(A, t, i, oi, [&](int part, float dx, float dy, float dz, float rsq, float fpj) {
         float p, g = 0.0f, h = 0.0f, phi = 0.0f;
-        const bool inside = rsq < T.cutforcesq;
-        bool spline = inside;
+        bool spline = rsq < T.cutforcesq;
         if (FAST) {
           const unsigned m = fast_interval(T, rsq, p);
           g = cubic(mine[m * T.copies], p);
           h = cubic(mine[m * T.copies + second], p);
-          spline = inside && m == T.cnt;
+          if (EV) phi = cubic(mine[m * T.copies + 2 * second], p);
+          spline = spline && m == T.cnt;
         }
-        if (spline) {
-          spline_force(T, rsq, g, h, phi);
-        } else if (EV && inside) {
-          float g2, h2;
-          spline_force(T, rsq, g2, h2, phi);
-        }
+        if (spline) spline_force(T, rsq, g, h, phi);
         const float pull = __fmaf_rn(__fadd_rn(fpi, fpj), g, h);
         S.add(part, dx, dy, dz, pull);
         if (EV) S.add_ev(part, dx, dy, dz, pull, phi);
@@ -606,23 +603,25 @@ struct HostSpline {
 // 29 / 19 / 15, 84 k 33 / 33 / 31, 313 k 91 / 83 / 88, 1.21 M 268 / 275 / 311.
 constexpr int ONE_LANE_SITES = 600000, TWO_LANE_SITES = 100000;
 
-// The three functions of s = r^2 that the passes need, as cubics on n equal
-// intervals of [0, top^2], each the interpolant at the interval's four
-// Chebyshev nodes.  An interval is good when every function's cubic stays
-// within 2e-8 of the spline, relative to its largest value within 0.5 A.
-// Returns the first interval from which all are good (n: none).
-int fit_fast(const HostSpline &rho, const HostSpline &z, double top, int n, float &inv_ds, std::vector<float4> rec[3]) {
+// The functions of s = r^2 that the passes need (three for the forces, and
+// phi for tallies), as cubics on n equal intervals of [0, top^2], each the
+// interpolant at the interval's four Chebyshev nodes.  An interval is good when
+// every function's cubic stays within 2e-8 (phi: 4e-8) of the spline, relative
+// to its largest value within 0.5 A.  Returns the first interval from which all
+// are good (n: none).
+int fit_fast(const HostSpline &rho, const HostSpline &z, double top, int n, float &inv_ds, std::vector<float4> rec[4]) {
   // pairs at the top or beyond fall past the last interval
   inv_ds = (float)((double)n / (double)(float)(top * top));
   while ((double)inv_ds * (double)(float)(top * top) < n) inv_ds = std::nextafter(inv_ds, 1e30f);
   const double ds = 1.0 / (double)inv_ds;
-  auto eval = [&](double s, double out[3]) {
+  auto eval = [&](double s, double out[4]) {
     const double r = std::sqrt(s);
     double dr, zv, dz;
     rho.at(r, out[0], dr);
     z.at(r, zv, dz);
     out[1] = dr / r;
     out[2] = (dz - zv / r) / s;
+    out[3] = zv / r;
   };
   double node[4], inv[4][4];
   for (int k = 0; k < 4; k++) node[k] = 0.5 - 0.5 * std::cos((2 * k + 1) * 3.14159265358979323846 / 8.0);
@@ -644,40 +643,40 @@ int fit_fast(const HostSpline &rho, const HostSpline &z, double top, int n, floa
     std::copy(c, c + 4, inv[k]);
   }
   constexpr int TEST = 12;
-  std::vector<double> err[3], val[3], mid(n);
-  for (int q = 0; q < 3; q++) {
+  std::vector<double> err[4], val[4], mid(n);
+  for (int q = 0; q < 4; q++) {
     rec[q].resize(n);
     err[q].assign(n, 0.0);
     val[q].assign(n, 0.0);
   }
   for (int m = 0; m < n; m++) {
     mid[m] = std::sqrt((m + 0.5) * ds);
-    double c[3][4] = {};
+    double c[4][4] = {};
     for (int k = 0; k < 4; k++) {
-      double v[3];
+      double v[4];
       eval((m + node[k]) * ds, v);
-      for (int q = 0; q < 3; q++)
+      for (int q = 0; q < 4; q++)
         for (int d = 0; d < 4; d++) c[q][d] += v[q] * inv[k][d];
     }
     for (int u = 0; u <= TEST; u++) {
       const double p = (double)u / TEST;
-      double v[3];
+      double v[4];
       eval(std::max((m + p) * ds, 1e-6 * ds), v);
-      for (int q = 0; q < 3; q++) {
+      for (int q = 0; q < 4; q++) {
         const double a = ((c[q][3] * p + c[q][2]) * p + c[q][1]) * p + c[q][0];
         err[q][m] = std::max(err[q][m], std::fabs(a - v[q]));
         val[q][m] = std::max(val[q][m], std::fabs(v[q]));
       }
     }
-    for (int q = 0; q < 3; q++)
+    for (int q = 0; q < 4; q++)
       rec[q][m] = make_float4((float)c[q][3], (float)c[q][2], (float)c[q][1], (float)c[q][0]);
   }
   for (int m = n - 1; m >= 0; m--)
-    for (int q = 0; q < 3; q++) {
+    for (int q = 0; q < 4; q++) {
       double size = 0.0;
       for (int j = m; j >= 0 && mid[m] - mid[j] <= 0.5; j--) size = std::max(size, val[q][j]);
       for (int j = m; j < n && mid[j] - mid[m] <= 0.5; j++) size = std::max(size, val[q][j]);
-      if (!(err[q][m] <= 2e-8 * size)) return m + 1;
+      if (!(err[q][m] <= (q < 3 ? 2e-8 : 4e-8) * size)) return m + 1;
     }
   return 0;
 }
@@ -689,7 +688,7 @@ int fit_fast(const HostSpline &rho, const HostSpline &z, double top, int n, floa
 void eam_fast_tables(Ctx &c, const std::vector<double4> &rz) {
   c.fast_cnt = 0;
   const HostSpline rho{rz, 0, c.pp.nr, c.pp.rdr}, z{rz, 1, c.pp.nr, c.pp.rdr};
-  std::vector<float4> rec[3];
+  std::vector<float4> rec[4];
   for (int n : FAST_INTERVALS)
     for (double top : {c.pp.cut, c.pp.cut - 4.0 * c.pp.dr}) {
       if (!(top > 0.5 * c.pp.cut)) continue;
@@ -700,7 +699,7 @@ void eam_fast_tables(Ctx &c, const std::vector<double4> &rz) {
       c.fast_cnt = n - lo;
       c.fast_inv_ds = inv_ds;
       std::vector<float4> out;
-      for (int q = 0; q < 3; q++) {
+      for (int q = 0; q < 4; q++) {
         out.insert(out.end(), rec[q].begin() + lo, rec[q].end());
         out.push_back(make_float4(0.0f, 0.0f, 0.0f, 0.0f));
       }
@@ -719,8 +718,8 @@ void allow_fast_records() {
   };
   auto allow = [&](size_t bytes, auto... kernels) { (one(kernels, bytes), ...); };
   allow(FAST_BYTES, k_eam_rho32<1, true>, k_eam_rho32<2, true>, k_eam_rho32<4, true>);
-  allow(2 * FAST_BYTES, k_eam_force32<1, true, false>, k_eam_force32<2, true, false>, k_eam_force32<4, true, false>,
-        k_eam_force32<1, true, true>, k_eam_force32<2, true, true>, k_eam_force32<4, true, true>);
+  allow(2 * FAST_BYTES, k_eam_force32<1, true, false>, k_eam_force32<2, true, false>, k_eam_force32<4, true, false>);
+  allow(3 * FAST_BYTES, k_eam_force32<1, true, true>, k_eam_force32<2, true, true>, k_eam_force32<4, true, true>);
 }
 
 }  // namespace
@@ -862,7 +861,7 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
       KernelTimer t(c, "eam_force32");
       by_lanes([&](auto g) {
         constexpr int GL = decltype(g)::value;
-        if (ev && fast) go(k_eam_force32<GL, true, true>, grid_ev, 2 * rec, c.phi_site.p);
+        if (ev && fast) go(k_eam_force32<GL, true, true>, grid_ev, 3 * rec, c.phi_site.p);
         else if (ev) go(k_eam_force32<GL, false, true>, grid_ev, 0, c.phi_site.p);
         else if (fast) go(k_eam_force32<GL, true, false>, grid, 2 * rec, c.phi_site.p);
         else go(k_eam_force32<GL, false, false>, grid, 0, c.phi_site.p);
