@@ -1039,8 +1039,14 @@ __device__ void items_warp(const BuildArgs &A, const Query &q, const int2 *items
       // times as much
       const float reach = (float)(A.cutneigh + 2.0 * (A.ecenter[e].w + A.eframe[(size_t)e * EFR + 12]));
       const float pre = (float)A.cutneigh + 2e-5f * reach, sure = (float)A.cutneigh - 2e-5f * reach;
-      st.lim[lane][0] = pre * pre;
-      st.lim[lane][1] = sure > 0.0f ? sure * sure : 0.0f;
+      // In an element large against the cutoff that margin no longer covers the
+      // rounding of the rows' discriminants (some 1e-6 reach^2 against 4e-5
+      // cutneigh reach, in units of the squared step), nor, from 250 A on, the
+      // prefix rule's allowance of 1e-3 A that of the segments (4e-6 reach):
+      // there no row is cut short, and every site near enough is decided exactly.
+      const bool long_rows = reach > 40.0f * (float)A.cutneigh;
+      st.lim[lane][0] = long_rows ? 3e38f : pre * pre;
+      st.lim[lane][1] = sure > 0.0f && !long_rows && reach <= 250.0f ? sure * sure : 0.0f;
     }
     __syncwarp();
     // the maps, four items at a time: lane 8 i + p takes the node at corner p =
@@ -1160,7 +1166,7 @@ __device__ void items_warp(const BuildArgs &A, const Query &q, const int2 *items
         float low[3], up[3];
         row_map(m, a, bb, low, up);
         // |low + cc up|^2 <= lim: the exact neighbours lie well inside (lim
-        // holds the margin), so rounding here loses none
+        // holds the margin, or is without bound), so rounding here loses none
         const float A2 = up[0] * up[0] + up[1] * up[1] + up[2] * up[2];
         const float B = low[0] * up[0] + low[1] * up[1] + low[2] * up[2];
         const float C = low[0] * low[0] + low[1] * low[1] + low[2] * low[2] - st.lim[m][0];
