@@ -446,7 +446,9 @@ inline void note_build_box(Ctx &c) {
 // pass of that time), FIRE at 93 k sites 9.88 -> 9.12 ms for 50 iterations.  Above
 // BEHIND_SITES the gaps are nothing and blocks that wait only take room from
 // those at work (1.21 M sites, 20 steps: 27.04 ms plainly, 26.86 ms so; 1.7 M
-// 29.65 and 29.72; 5 M 59.1 and 59.6).
+// 29.65 and 29.72; 5 M 59.1 and 59.6).  While kernels are timed they are
+// launched plainly, one by one (also those that share a timer), so that a timed
+// run is a check on the waits of the others.
 constexpr long BEHIND_SITES = 1500000;
 template <class... P, class... T>
 void launch_behind(const Ctx &c, int blocks, int threads, size_t smem, void (*kernel)(P...), T &&...args) {
@@ -459,7 +461,7 @@ void launch_behind(const Ctx &c, int blocks, int threads, size_t smem, void (*ke
   cfg.dynamicSmemBytes = smem;
   cfg.stream = c.stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = c.nsite_i() < BEHIND_SITES ? 1 : 0;
+  cfg.numAttrs = c.nsite_i() < BEHIND_SITES && !c.prof.enabled ? 1 : 0;
   CACB200_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
 }
 
