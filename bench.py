@@ -715,8 +715,7 @@ def b200_arm(args, rank, local, ws, dist):
                     "d2h_bytes_per_step": bytes_state, "steps": k_e2e},
             "gpu_launches": int(round(launches_per_step * args.steps)),
             "tuned_blocks": dict(zip(("rho", "force"), tuned)),
-            "work_queue_tiles": (dict(zip(("below_8192_sites", "below_32768_sites", "larger"), work_tiles))
-                                 if work_tiles else None),
+            "resident_block_threads": work_tiles[0] if work_tiles else None,
             "thermo_readout_ms": thermo_ms,
             "clocks": clocks,
         }

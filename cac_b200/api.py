@@ -313,8 +313,8 @@ class Engine:
 
     def work_queue(self, enable=None):
         """Turn the persistent launches of the EAM passes and the atom build on
-        or off (None: unchanged); returns the slots per block of a batch's mixed
-        passes for each size class (0: not run yet)."""
+        or off (None: unchanged); returns the threads of a resident block of a
+        batch's mixed EAM passes, three times (0: none, or not run yet)."""
         t = (C.c_int * 3)()
         self._check(self.lib.cacb200_work_queue(self.h, -1 if enable is None else int(bool(enable)), t),
                     "work_queue")

@@ -88,8 +88,7 @@ struct Rep {
   Grid ag, eg;
   int abase, ebase;
   double reach_budget;
-  double qscale[3];   // mixed form: fixed-point scale 2^k per dimension ...
-  float qinv[3];      // ... and 2^-k
+  double qscale[3];   // mixed form: fixed-point scale 2^k per dimension
   int Lq[3];          // rint(L 2^k)
 };
 
@@ -229,7 +228,6 @@ struct Ctx {
   // atom cell grid (candidate search)
   Grid agrid{}, egrid{};
   DBuf<int> acell_start;         // [ncell+1]
-  DBuf<int> acell_atoms;         // [na] atom ids sorted by cell
   DBuf<double4> acell_pos;       // [na] wrapped positions sorted by cell, w = bitcast(id)
   DBuf<int> acell_fix;           // [3][na] the same in fixed point (the atom build's screen, neigh.cu)
   DBuf<int> acell_of;            // [na] cell of each sorted atom
@@ -300,11 +298,11 @@ struct Ctx {
   int build_count = 0;
 
   PairParams pp;
-  DBuf<double4> rhor_val, rhor_der, z2r_val, z2r_der, frho_val, frho_der;
+  DBuf<double4> frho_val, frho_der;
   // per r-knot m: [2m] rhor value coefficients, [2m+1] z2r value coefficients
   // (one 64-byte record read by a pair; derivatives follow from them)
   DBuf<double4> rz;
-  // mixed precision: FP32 tables, per-site FP32 offsets and packed anchor cells
+  // mixed precision: FP32 tables
   DBuf<float4> frho_val32, frho_der32;
   DBuf<float4> rz32;              // the same r-knot records in FP32 (32 bytes)
   bool have_mixed_tables = false;
@@ -336,7 +334,7 @@ struct Ctx {
   // persistent forms of the pair passes and the atom build
   bool work_queue = true;
   DBuf<int> sm_counter;   // single systems: run counters of the SM-local ranges (rho, force)
-  int work_tile[3] = {0, 0, 0};    // batches, mixed form: list slots a resident block takes at a time
+  int work_tile[3] = {0, 0, 0};    // batches, mixed form: threads of a resident block (0: none yet)
   double escale_node_last = 0.0;   // node energy scale of the last evaluation
   DBuf<int> rep_meta;              // [4][nrep] aoff, na, eoff, ne (per-replica energy)
   DBuf<double> rep_energy;         // [nrep]

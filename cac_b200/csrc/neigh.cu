@@ -1830,21 +1830,17 @@ __device__ __forceinline__ int site_index(int e, int u, const uint2 *words, int 
   return na + NG * ne + (int)w.y + __popc(w.x & ((1u << (u & 31)) - 1u));
 }
 
-// Packs each entry as (pair-table index << 5 | image code): atoms by their
-// list slot (the pair table holds atoms in cell-sorted order), element sites
-// after them as in the site table.  Entries inside the inner radius (the
-// force cutoff plus a margin) at build time go first, each group in build
-// order, and their number is kept (num_in): while no site has moved half the
-// margin since the build, every pair inside the cutoff lies in that prefix,
-// in the same order, so the pair loops may stop there with identical sums.
+// Packs each entry of a half list as (pair-table index << 5 | image code): atoms
+// by their list slot (the pair table holds atoms in cell-sorted order), element
+// sites after them as in the site table.  Entries inside the inner radius (the
+// force cutoff plus a margin) at build time go first, each group in build order.
 __global__ void k_remap(const int *raw, const unsigned char *img, const int *num, int nsi, int cap,
-                        const uint2 *words, const int *atom_slot, int na, int ne, int *out, int *num_in) {
+                        const uint2 *words, const int *atom_slot, int na, int ne, int *out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nsi) return;
   int n = min(num[i], cap);
   int nin = 0;
   for (int k = 0; k < n; k++) nin += (img[(size_t)k * nsi + i] & IN_CUT) != 0;
-  if (num_in) num_in[i] = nin;
   int a = 0, b = nin;   // next in-cutoff and next other position
   for (int k = 0; k < n; k++) {
     size_t o = (size_t)k * nsi + i;
@@ -2053,7 +2049,6 @@ void neigh_plan(Ctx &c, bool want_half) {
     // quanta modulo 2^32 (pair separations are taken modulo 2^32 as well)
     for (int d = 0; d < 3; d++) {
       R.qscale[d] = std::ldexp(1.0, 26);
-      R.qinv[d] = std::ldexp(1.0f, -26);
       R.Lq[d] = (int)(uint32_t)(uint64_t)std::llrint(R.b.L[d] * R.qscale[d]);
     }
     R.abase = abase;
@@ -2326,7 +2321,7 @@ void neigh_build_async(Ctx &c, bool want_half) {
     }
     if (want_half)
       k_remap<<<nblk(nsi, 256), 256, 0, c.stream>>>(c.raw_half.p, c.img_half.p, c.num_half.p, nsi, c.cap,
-                                                     c.site_words.p, c.atom_slot.p, c.na, c.ne, c.nbr_half.p, nullptr);
+                                                     c.site_words.p, c.atom_slot.p, c.na, c.ne, c.nbr_half.p);
   }
   c.have_half = want_half;
   c.lists_valid = true;

@@ -498,14 +498,12 @@ void eam_tables(Ctx &c, const double *frho, const double *rhor, const double *z2
   spline7(p.nrho, p.drho, a, sp);
   upload_split(c, sp, p.nrho, c.frho_val, c.frho_der);
   spline7(p.nr, p.dr, b, sp);
-  upload_split(c, sp, p.nr, c.rhor_val, c.rhor_der);
   std::vector<double4> rz((size_t)2 * (p.nr + 1));
   for (int m = 0; m <= p.nr; m++) {
     const double *r = &sp[(size_t)m * 7];
     rz[2 * m] = make_double4(r[3], r[4], r[5], r[6]);
   }
   spline7(p.nr, p.dr, z, sp);
-  upload_split(c, sp, p.nr, c.z2r_val, c.z2r_der);
   for (int m = 0; m <= p.nr; m++) {
     const double *r = &sp[(size_t)m * 7];
     rz[2 * m + 1] = make_double4(r[3], r[4], r[5], r[6]);

@@ -15,8 +15,9 @@
 // What stays FP64 (as the mixed form specifies): positions and velocities and
 // their integration, element interpolation, nodal assembly over Gauss points,
 // and the global energy/virial reductions (per-block partials in FP64).
-// Per-site sums of pair terms are FP32; EAM spline coefficients are FP32
-// copies of the FP64 splines.
+// Per-site sums of pair terms are FP32.  EAM terms are cubics in r^2 fitted to
+// the FP64 splines where these are smooth (Eam32), else FP32 copies of the
+// splines' coefficients.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -837,8 +838,8 @@ void pair_compute_mixed(Ctx &c, int eflag, int vflag) {
     const int grid = c.work_queue && !small ? std::min(need, 2 * c.num_sms) : need;
     grid_ev = std::min(need, small ? c.num_sms * 8 : c.num_sms);
     c.tb_rho32 = c.tb_force32 = tb;
-    if (c.nrep > 1 && c.work_queue)
-      for (int &k : c.work_tile) k = 512;
+    if (c.nrep > 1)
+      for (int &k : c.work_tile) k = c.work_queue && !small ? tb : 0;
     const bool fast = c.fast_cnt > 0;
     const size_t rec = fast ? sizeof(float4) * (size_t)(c.fast_cnt + 1) * Tb.copies : 0;
     auto go = [&](auto kernel, int blocks, size_t bytes, auto... args) {

@@ -435,9 +435,10 @@ int cacb200_pair_blocks(cacb200_ctx *ctx, int *rho_threads, int *force_threads);
  * one multiprocessor share their neighbours' data in its L1; a block whose
  * own range is exhausted takes runs from another range (same lists and
  * results as the grid launches, bit for bit).  enable: 1 on (default), 0 off
- * (one grid launch per pass), -1 unchanged; tiles [3] gets 512 for batches
- * after their first mixed EAM evaluation (0 before).  No reference counterpart
- * (the reference runs one system per process). */
+ * (one grid launch per pass), -1 unchanged; tiles [3] gets the threads of a
+ * resident block of a batch's mixed EAM passes, three times the same (0: none,
+ * or not evaluated yet).  No reference counterpart (the reference runs one
+ * system per process). */
 int cacb200_work_queue(cacb200_ctx *ctx, int enable, int tiles[3]);
 
 /* Kernel timing: when enabled, every launch is bracketed by CUDA events and
