@@ -379,6 +379,9 @@ __global__ void __launch_bounds__(128, EV ? 4 : 8) k_lj32(Args32 A, Lj32 P) {
 // spline record from global memory as many, from eight copies in shared memory
 // four; with four copies the force pass is 17 % slower).  4.98 M sites: density
 // 1.047 -> 0.73 ms, force 1.170 -> 0.88 ms; 313 k: 91 -> 60 and 96 -> 70 us.
+// Other tables, 1.21 M sites: 7 A cutoff (482 records) density 647 -> 434 us, force
+// 723 -> 603; without a fit (1,000 knots, 5.5 A; this launch shape with the
+// splines from memory) 335 -> 286 and 376 -> 351.
 // With tallies: 313 k sites 123 -> 96 us, 1.21 M 417 -> 310 us (133 and 489 us
 // where phi was read from the splines beside the records).
 constexpr int FAST_INTERVALS[] = {192, 256, 384, 512}, FAST_COPIES = 8;
