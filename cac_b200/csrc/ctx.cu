@@ -665,6 +665,7 @@ void minimize_fire(Ctx &c, double etol, double ftol, int maxiter, double dt, int
             wrapped = true;
           }
         }
+        c.tally_step_e = c.step;   // nothing has moved since the last evaluation: its energy is this step's
         break;
       }
     }
