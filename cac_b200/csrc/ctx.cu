@@ -156,6 +156,8 @@ void upload_system(Ctx &c, int nrep, const int *rna, const int *rne, const doubl
       c.rep_h[r].b.L[d] = hi[3 * r + d] - lo[3 * r + d];
     }
   }
+  // a snapshot and per-site values are laid out for the sizes they were made of
+  if (c.na != na || c.ne != ne) c.have_snapshot = c.have_peratom_e = c.have_peratom_v = false;
   c.na = na;
   c.ne = ne;
   c.mass = mass;
