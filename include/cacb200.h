@@ -379,7 +379,7 @@ int cacb200_minimize_fire(cacb200_ctx *ctx, double etol, double ftol, int maxite
 /* Device-side copy of the state (x, v, nodex, nodev) and its restoration;
  * restoring invalidates the lists (call cacb200_setup before stepping).
  * Serves restarts of short trajectories and job preemption without host
- * traffic. */
+ * traffic.  An upload of other sizes forgets the snapshot. */
 int cacb200_snapshot(cacb200_ctx *ctx);
 int cacb200_restore(cacb200_ctx *ctx);
 
